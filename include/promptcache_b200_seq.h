@@ -149,8 +149,9 @@ typedef struct pcs_attn_params {
   const int32_t* seq_len;
   const int32_t* seq_off;
   int32_t n_tokens, n_seqs, max_len, dtype;   /* max_len: host upper bound of the new tokens of one entry */
-  int32_t impl;             /* 0 = automatic, 1 = the plain kernel */
-  int32_t max_keys;         /* host upper bound of the keys one token sees (sizes the split of the keys); 0: one split */
+  int32_t impl;             /* 0 = automatic, 1 = the plain kernel, 2 = the plain kernels with the split of the keys, 3 = automatic without the tcgen05
+                               prompt kernel */
+  int32_t max_keys;         /* host upper bound of the keys one token sees (sizes the split of the keys); 0: one split (prompts: cap) */
   float* workspace;         /* fp32 scratch of pcs_attn_workspace_floats() elements, or NULL (one split) */
   int64_t workspace_floats;
   float softcap;            /* > 0: score = softcap * tanh(score / softcap), after the scale and before the bias */
@@ -180,6 +181,8 @@ typedef struct pcs_attn_params {
 /* scratch the key split of pcs_attn needs for n_tokens tokens */
 int64_t pcs_attn_workspace_floats(int n_tokens, int n_heads, int vdim);
 int pcs_attn(const pcs_attn_params* p, void* stream);
+/* blocks of the tcgen05 prompt kernel that gave up a wait after two seconds, since the library was loaded (0 in a working system); synchronises */
+int pcs_attn_timeouts(void);
 
 /* ig = cap * tanh((w_i h + b_i) / cap);  fg = logsigmoid(cap * tanh((w_f h + b_f) / cap))    (fp32 [n_tokens, heads]) */
 int pcs_mlstm_gates(const void* h, int64_t h_stride, const void* w_i, const void* w_f, const float* b_i, const float* b_f,

@@ -17,7 +17,7 @@ from ._native import NativeError, note_replayed_launches  # noqa: F401  (one err
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libpromptcache_b200_seq.so")
 PCS_BF16, PCS_F32 = 0, 1
-EXPORTS = ("pcs_version", "pcs_last_error", "pcs_launch_count", "pcs_attn_workspace_floats", "pcs_embed", "pcs_rmsnorm", "pcs_gate_norm_add", "pcs_xielu", "pcs_linear_rows",
+EXPORTS = ("pcs_version", "pcs_last_error", "pcs_launch_count", "pcs_attn_workspace_floats", "pcs_attn_timeouts", "pcs_embed", "pcs_rmsnorm", "pcs_gate_norm_add", "pcs_xielu", "pcs_linear_rows",
            "pcs_qk_prep", "pcs_attn", "pcs_mlstm_gates", "pcs_mlstm_scan", "pcs_embed_bigram", "pcs_norm_conv", "pcs_rope_kv_prep", "pcs_moe_route",
            "pcs_moe_rows_up", "pcs_moe_rows_down", "pcs_moe_plan", "pcs_moe_gather", "pcs_moe_gemm", "pcs_moe_combine", "pcs_silu_mul", "pcs_glu_mul",
            "pcs_depth_mix", "pcs_latent_prep", "pcs_latent_q", "pcs_latent_gather", "pcs_latent_expand", "pcs_head_gate", "pcs_gla_decay", "pcs_gla_scan", "pcs_gla_chunk_prep", "pcs_gla_chunk_scan", "pcs_gla_chunk_out",
@@ -356,6 +356,7 @@ class Batch:
         self.wants_all = False  # the logits of every token are asked for, in order
         self.prev_ids = None  # int64 [T] on the device: every token's predecessor in its sequence, -1 for a first token
         self.n_tokens, self.n_seqs, self.max_len = T, B, max(lens) if lens else 0
+        self.max_keys = max((p0 + n for p0, n in zip(pos0, lens)), default=0)
         self.offsets, self.lens, self.pos0, self.slots = offs, list(lens), list(pos0), list(slots)
 
 
@@ -518,6 +519,8 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: 
         if workspace.dtype != torch.float32 or not workspace.is_cuda or not workspace.is_contiguous():
             raise NativeError("attention: the workspace must be a contiguous CUDA float32 tensor")
         p.max_keys, p.workspace, p.workspace_floats = int(max_keys), workspace.data_ptr(), workspace.numel()
+    else:
+        p.max_keys = batch.max_keys   # what a launch over a prompt sizes its split by
     _check(load().pcs_attn(C.byref(p), _stream()), "pcs_attn")
 
 

@@ -497,6 +497,7 @@ PCS_API int pcs_qk_prep(const pcs_qkprep_params* p, void* stream) {
 
 namespace pcs {
 int launch_attn_tc(const pcs_attn_params& p, cudaStream_t st, bool* handled);
+int launch_attn_tc5(const pcs_attn_params& p, cudaStream_t st, bool* handled);
 int launch_attn_latent(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
 int launch_attn_talk(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
 }
@@ -530,8 +531,11 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
     }
     return PCS_OK;
   }
-  if (p->impl == 0) {  // (impl 2: the plain kernels with the split of the keys, never a tensor-core kernel)
+  if (p->impl == 0 || p->impl == 3) {  // (impl 2: the plain kernels with the split of the keys, never a tensor-core kernel; 3: not the tcgen05 prompt kernel)
     bool handled = false;
+    if (p->impl == 0)
+      if (int rc = pcs::launch_attn_tc5(*p, st, &handled)) return rc;
+    if (handled) return PCS_OK;
     if (int rc = pcs::launch_attn_tc(*p, st, &handled)) return rc;
     if (handled) return PCS_OK;
     int latent_splits = 0;   // few tokens over rows that all heads share: the tensor-core kernel, then the merge of its partial results
