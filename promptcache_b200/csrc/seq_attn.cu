@@ -9,7 +9,7 @@
 //               and the running sum at 1 instead of (-inf, 0).  A score may be capped (cap * tanh(score / cap)), and the keys may
 //               be limited to a sliding window plus the first keys of the sequence: a query then walks a dense list of its
 //               visible keys, so its work is bounded by window + keep_first whatever the sequence's length.
-#include "seq_common.cuh"
+#include "seq_attn.cuh"
 
 namespace pcs {
 
@@ -175,30 +175,6 @@ __global__ void __launch_bounds__(256) qk_prep_vec_kernel(const pcs_qkprep_param
 
 constexpr int kAttnThreads = 128;
 constexpr int kAttnMaxVPT = 4;  // value columns per thread: vdim <= 512
-
-// The keys a query at position `pos` sees, as one dense index range: with a window, the kept first keys [0, n_first) and
-// then the window [lo, pos]; without one (or when the two touch), all of [0, pos].  With chunks, the keys of the query's own chunk.
-struct VisibleKeys {
-  int n_first, lo, count;
-  __device__ __forceinline__ VisibleKeys(int pos, int window, int keep_first, int chunk) {
-    lo = window > 0 ? max(0, pos - window + 1) : (chunk > 0 ? pos / chunk * chunk : 0);
-    n_first = chunk > 0 ? 0 : min(max(keep_first, 0), lo);
-    count = n_first + (pos + 1 - lo);
-  }
-  __device__ __forceinline__ int key(int v) const { return v < n_first ? v : lo + (v - n_first); }
-};
-
-// where head h of token t is written, and what its normalised result is multiplied by: the constant and the head's gate
-template <typename T>
-__device__ __forceinline__ T* out_row(const pcs_attn_params& p, int t, int h) {
-  return static_cast<T*>(p.out) + static_cast<long long>(t) * (p.out_stride > 0 ? p.out_stride : static_cast<long long>(p.n_heads) * p.vdim) + h * p.vdim;
-}
-template <typename T>
-__device__ __forceinline__ float out_factor(const pcs_attn_params& p, int t, int h) {
-  float f = p.out_scale != 0.f ? p.out_scale : 1.f;
-  if (p.head_gate) f *= sigmoidf_(ldf(static_cast<const T*>(p.head_gate) + static_cast<long long>(t) * p.head_gate_stride + h));
-  return f;
-}
 
 template <typename T>
 __global__ void __launch_bounds__(kAttnThreads) attn_plain_kernel(const pcs_attn_params p) {
@@ -422,8 +398,6 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(const pcs_att
   }
 }
 
-constexpr int kAttnMaxSplits = 64;
-
 // Merge of the splits' partial results.  The splits' maxima and sums are read by one thread each, the common maximum, the total
 // and every split's factor exp(m_s - M) are formed once in shared memory, and the columns then need independent loads only.
 template <typename T>
@@ -498,6 +472,7 @@ PCS_API int pcs_qk_prep(const pcs_qkprep_params* p, void* stream) {
 namespace pcs {
 int launch_attn_tc(const pcs_attn_params& p, cudaStream_t st, bool* handled);
 int launch_attn_tc5(const pcs_attn_params& p, cudaStream_t st, bool* handled);
+int launch_attn_group_decode(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
 int launch_attn_latent(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
 int launch_attn_talk(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
 }
@@ -533,9 +508,10 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
   }
   if (p->impl == 0 || p->impl == 3) {  // (impl 2: the plain kernels with the split of the keys, never a tensor-core kernel; 3: not the tcgen05 prompt kernel)
     bool handled = false;
-    if (p->impl == 0)
+    if (p->impl == 0) {
       if (int rc = pcs::launch_attn_tc5(*p, st, &handled)) return rc;
-    if (handled) return PCS_OK;
+      if (handled) return PCS_OK;
+    }
     if (int rc = pcs::launch_attn_tc(*p, st, &handled)) return rc;
     if (handled) return PCS_OK;
     int latent_splits = 0;   // few tokens over rows that all heads share: the tensor-core kernel, then the merge of its partial results
@@ -556,6 +532,16 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
   const bool decode = (p->impl == 0 || p->impl == 2) && p->workspace != nullptr && p->dim % piece == 0 && p->vdim % piece == 0 &&
                       p->vdim / piece <= pcs::kAttnThreads && p->v_row_stride % piece == 0;
   int splits = 1;
+  if (decode && p->impl == 0) {
+    if (int rc = pcs::launch_attn_group_decode(*p, st, &splits)) return rc;
+    if (splits > 1) {
+      PCS_DISPATCH(p->dtype, pcs::attn_combine_kernel<T><<<dim3(p->n_tokens, p->n_heads, (p->vdim + pcs::kAttnThreads - 1) / pcs::kAttnThreads), pcs::kAttnThreads, 0, st>>>(*p, splits));
+      PCS_CHECK_CUDA(cudaGetLastError());
+      pcs::count_launch();
+    }
+    if (splits > 0) return PCS_OK;
+    splits = 1;
+  }
   if (p->workspace != nullptr && p->max_keys > 512) {
     const long long blocks = static_cast<long long>(p->n_tokens) * p->n_heads;
     const int want = static_cast<int>((2 * 148 + blocks - 1) / blocks);
