@@ -472,6 +472,7 @@ PCS_API int pcs_qk_prep(const pcs_qkprep_params* p, void* stream) {
 namespace pcs {
 int launch_attn_tc(const pcs_attn_params& p, cudaStream_t st, bool* handled);
 int launch_attn_tc5(const pcs_attn_params& p, cudaStream_t st, bool* handled);
+int launch_attn_f32(const pcs_attn_params& p, cudaStream_t st, bool* handled);
 int launch_attn_group_decode(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
 int launch_attn_latent(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
 int launch_attn_talk(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
@@ -510,6 +511,8 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
     bool handled = false;
     if (p->impl == 0) {
       if (int rc = pcs::launch_attn_tc5(*p, st, &handled)) return rc;
+      if (handled) return PCS_OK;
+      if (int rc = pcs::launch_attn_f32(*p, st, &handled)) return rc;
       if (handled) return PCS_OK;
     }
     if (int rc = pcs::launch_attn_tc(*p, st, &handled)) return rc;

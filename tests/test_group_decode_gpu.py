@@ -1,4 +1,4 @@
-"""Decoding attention of a group of heads over the rows they share against float64: group sizes off the padded ones, row
+"""Decoding attention of a group of heads over the rows they share, and 32-bit prompt attention, against float64: group sizes off the padded ones, row
 widths at and off the lanes that read a row, splits as clusters and through the workspace, sequences of one key, every option."""
 import math
 
@@ -64,3 +64,17 @@ def test_group_decode(nsq, shape, name):  # noqa: F811
 def test_several_tokens_of_a_sequence(nsq):  # noqa: F811
     check(nsq, "bias", 8, 2, 128, 128, (3, 1, 5), (200, 0, 1000), BF16, True, 5)
 
+
+PROMPT32 = [
+    (4, 2, 128, 128, (31, 32, 33, 65), (0, 63, 1, 64)),
+    (3, 1, 68, 36, (130,), (0,)),
+    (2, 2, 192, 64, (20, 1), (1900, 7)),    # a walk shared by a cluster
+    (1, 1, 256, 128, (300,), (0,)),
+]
+
+
+@pytest.mark.parametrize("shape", PROMPT32)
+@pytest.mark.parametrize("name", OPTIONS)
+def test_prompt_attention_in_32_bits(nsq, shape, name):  # noqa: F811
+    H, G, D, V, lens, pos0 = shape
+    check(nsq, name, H, G, D, V, lens, pos0, F32, False, D + len(name))
