@@ -66,7 +66,7 @@
 extern "C" {
 #endif
 
-#define PCS_ABI_VERSION 6
+#define PCS_ABI_VERSION 7
 #define PCS_BF16 0
 #define PCS_F32 1
 
@@ -214,11 +214,15 @@ typedef struct pcs_mlstm_params {
   int32_t n_seqs, dtype;
   int32_t max_len;          /* host upper bound of the new tokens of one entry */
   int32_t impl;             /* 0 = automatic, 1 = token by token with the state in shared memory, 2 = token by token (registers
-                               where the sizes allow): never the chunkwise tensor-core kernel */
+                               where the sizes allow): never the chunkwise tensor-core kernels, 3 = automatic with the chunks one after the other */
   float* o_raw;             /* fp32 scratch of n_tokens*heads*vdim + n_seqs*heads*(dim+1) elements: the recurrence's result before
                                the per-head norm, and the new n / m of every entry until they are committed */
   int32_t n_tokens, reserved;
+  float* chunk_scratch;     /* fp32 scratch of pcs_mlstm_scratch_floats() elements, 16-byte aligned, or NULL: with it the chunks of a prompt
+                               run side by side (vdim <= 512), without it one after the other */
+  int64_t chunk_floats;
 } pcs_mlstm_params;
+int64_t pcs_mlstm_scratch_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim);
 int pcs_mlstm_scan(const pcs_mlstm_params* p, void* stream);
 
 /* out[t, :] = table[ids[t], :] * scale + pair[r, :], r = (prev_ids[t] * mul_prev + ids[t] * mul_cur) mod buckets, or r = buckets (the

@@ -18,7 +18,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libpromptcache_b200_seq.so")
 PCS_BF16, PCS_F32 = 0, 1
 EXPORTS = ("pcs_version", "pcs_last_error", "pcs_launch_count", "pcs_attn_workspace_floats", "pcs_attn_timeouts", "pcs_embed", "pcs_rmsnorm", "pcs_gate_norm_add", "pcs_xielu", "pcs_linear_rows",
-           "pcs_qk_prep", "pcs_attn", "pcs_mlstm_gates", "pcs_mlstm_scan", "pcs_embed_bigram", "pcs_norm_conv", "pcs_rope_kv_prep", "pcs_moe_route",
+           "pcs_qk_prep", "pcs_attn", "pcs_mlstm_gates", "pcs_mlstm_scan", "pcs_mlstm_scratch_floats", "pcs_embed_bigram", "pcs_norm_conv", "pcs_rope_kv_prep", "pcs_moe_route",
            "pcs_moe_rows_up", "pcs_moe_rows_down", "pcs_moe_plan", "pcs_moe_gather", "pcs_moe_gemm", "pcs_moe_combine", "pcs_silu_mul", "pcs_glu_mul",
            "pcs_depth_mix", "pcs_latent_prep", "pcs_latent_q", "pcs_latent_gather", "pcs_latent_expand", "pcs_head_gate", "pcs_gla_decay", "pcs_gla_scan", "pcs_gla_chunk_prep", "pcs_gla_chunk_scan", "pcs_gla_chunk_out",
            "pcs_add_layer_norm", "pcs_gru_scan", "pcs_group_norm_conv", "pcs_soft_cap", "pcs_short_conv", "pcs_delta_inputs", "pcs_delta_scan", "pcs_delta_chunk_prep", "pcs_delta_chunk_scan",
@@ -210,7 +210,7 @@ class pcs_mlstm_params(C.Structure):
                 ("heads", C.c_int32), ("dim", C.c_int32), ("vdim", C.c_int32), ("q_scale", C.c_float), ("eps", C.c_float),
                 ("seq_slot", C.c_void_p), ("seq_pos0", C.c_void_p), ("seq_len", C.c_void_p), ("seq_off", C.c_void_p),
                 ("n_seqs", C.c_int32), ("dtype", C.c_int32), ("max_len", C.c_int32), ("impl", C.c_int32),
-                ("o_raw", C.c_void_p), ("n_tokens", C.c_int32), ("reserved", C.c_int32)]
+                ("o_raw", C.c_void_p), ("n_tokens", C.c_int32), ("reserved", C.c_int32), ("chunk_scratch", C.c_void_p), ("chunk_floats", C.c_int64)]
 
 
 _lib: Optional[C.CDLL] = None
@@ -232,6 +232,7 @@ def load() -> C.CDLL:
     lib.pcs_version.restype = C.c_int
     lib.pcs_last_error.restype = C.c_char_p
     lib.pcs_launch_count.restype = C.c_int64
+    lib.pcs_mlstm_scratch_floats.restype = C.c_int64
     lib.pcs_embed.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_float, C.c_int, C.c_void_p]
     lib.pcs_rmsnorm.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_float, C.c_int, C.c_void_p]
     lib.pcs_gate_norm_add.argtypes = [C.POINTER(pcs_gna_params), C.c_void_p]
@@ -540,6 +541,9 @@ def mlstm_gates(h: torch.Tensor, w_i: torch.Tensor, w_f: torch.Tensor, b_i: torc
                                   dtype_code(w_i.dtype), _stream()), "pcs_mlstm_gates")
 
 
+MLSTM_SCRATCH_MAX = 1 << 28   # floats
+
+
 def mlstm_scan(proj: torch.Tensor, offs, ig: torch.Tensor, fg: torch.Tensor, norm_w: torch.Tensor, out: torch.Tensor,
                s_pool: torch.Tensor, n_pool: torch.Tensor, m_pool: torch.Tensor, eps: float, batch: Batch, impl: int = 0) -> None:
     """proj [T, *] with q / k / v / output-gate columns at `offs`; state pools float32 [slots, H, dim, vdim], [slots, H, dim],
@@ -560,6 +564,12 @@ def mlstm_scan(proj: torch.Tensor, offs, ig: torch.Tensor, fg: torch.Tensor, nor
     p.seq_slot, p.seq_pos0, p.seq_len, p.seq_off = (batch.seq_slot.data_ptr(), batch.seq_pos0.data_ptr(), batch.seq_len.data_ptr(),
                                                     batch.seq_off.data_ptr())
     p.n_seqs, p.dtype, p.max_len, p.impl = batch.n_seqs, dtype_code(dt), batch.max_len, impl
+    # prompts in bfloat16: the chunks side by side, as long as their states take at most a gigabyte (beyond: one after the other)
+    if dt == torch.bfloat16 and impl == 0 and batch.max_len > 192:   # (fewer chunks never run side by side)
+        floats = int(load().pcs_mlstm_scratch_floats(batch.n_tokens, batch.n_seqs, p.heads, p.dim, p.vdim))
+        if floats <= MLSTM_SCRATCH_MAX:
+            scratch = torch.empty(floats, dtype=torch.float32, device=proj.device)
+            p.chunk_scratch, p.chunk_floats = scratch.data_ptr(), floats
     # scratch: the recurrence's raw result per token, and the new n / m per entry until the commit launch stores them
     o_raw = torch.empty(batch.n_tokens * p.heads * p.vdim + batch.n_seqs * p.heads * (p.dim + 1), dtype=torch.float32, device=proj.device)
     p.o_raw, p.n_tokens = o_raw.data_ptr(), batch.n_tokens
