@@ -787,6 +787,9 @@ typedef struct pcs_gla_chunk_params {
   void* out;
 } pcs_gla_chunk_params;
 int pcs_gla_chunk_prep(const pcs_gla_chunk_params* p, void* stream);
+/* u[c, h] = kd[c, h]^T vf[c, h] on the tensor cores, v from the projections (bfloat16 runs, chunks of 64, dim a multiple of 16 up to 256, 16-byte pieces;
+ * otherwise PCS_ERR_UNSUPPORTED) */
+int pcs_gla_chunk_sums(const pcs_gla_chunk_params* p, void* stream);
 int pcs_gla_chunk_scan(const pcs_gla_chunk_params* p, void* stream);
 int pcs_gla_chunk_out(const pcs_gla_chunk_params* p, void* stream);
 

@@ -20,7 +20,7 @@ PCS_BF16, PCS_F32 = 0, 1
 EXPORTS = ("pcs_version", "pcs_last_error", "pcs_launch_count", "pcs_attn_workspace_floats", "pcs_attn_timeouts", "pcs_embed", "pcs_rmsnorm", "pcs_gate_norm_add", "pcs_xielu", "pcs_linear_rows",
            "pcs_qk_prep", "pcs_attn", "pcs_mlstm_gates", "pcs_mlstm_scan", "pcs_mlstm_scratch_floats", "pcs_embed_bigram", "pcs_norm_conv", "pcs_rope_kv_prep", "pcs_moe_route",
            "pcs_moe_rows_up", "pcs_moe_rows_down", "pcs_moe_plan", "pcs_moe_gather", "pcs_moe_gemm", "pcs_moe_combine", "pcs_silu_mul", "pcs_glu_mul",
-           "pcs_depth_mix", "pcs_latent_prep", "pcs_latent_q", "pcs_latent_gather", "pcs_latent_expand", "pcs_head_gate", "pcs_gla_decay", "pcs_gla_scan", "pcs_gla_chunk_prep", "pcs_gla_chunk_scan", "pcs_gla_chunk_out",
+           "pcs_depth_mix", "pcs_latent_prep", "pcs_latent_q", "pcs_latent_gather", "pcs_latent_expand", "pcs_head_gate", "pcs_gla_decay", "pcs_gla_scan", "pcs_gla_chunk_prep", "pcs_gla_chunk_sums", "pcs_gla_chunk_scan", "pcs_gla_chunk_out",
            "pcs_add_layer_norm", "pcs_gru_scan", "pcs_group_norm_conv", "pcs_soft_cap", "pcs_short_conv", "pcs_delta_inputs", "pcs_delta_scan", "pcs_delta_chunk_prep", "pcs_delta_chunk_scan",
            "pcs_head_norm_gate", "pcs_delta_chunk_out", "pcs_side_gate", "pcs_side_boundary")
 GLU_SILU, GLU_CLAMPED_SWISH, GLU_GELU_TANH = 0, 1, 4
@@ -977,8 +977,9 @@ def _gla_chunk_plan(batch: Batch, chunk: int):
 def gla_scan_chunked(proj: torch.Tensor, offs, ld: torch.Tensor, norm_w: torch.Tensor, out: torch.Tensor, s_pool: torch.Tensor, eps: float, batch: Batch,
                      chunk: int = GLA_CHUNK) -> None:
     """The recurrence of `gla_scan` in chunks: the factors that carry decays are formed by `pcs_gla_chunk_prep` (32-bit, every
-    exponent <= 0), the sums over tokens and channels are three batched float32 matrix products, the chunks' start states come
-    from one pass over the chunks (`pcs_gla_chunk_scan`)."""
+    exponent <= 0), the chunks' start states come
+    from one pass over the chunks (`pcs_gla_chunk_scan`).  bfloat16 runs take the sums over a chunk's tokens on the tensor cores
+    (`pcs_gla_chunk_sums`) and the read-out of the delta rule's chunks; others batched float32 matrix products."""
     H, D, V = s_pool.shape[1:]
     dt, dev = proj.dtype, proj.device
     plan = _gla_chunk_plan(batch, chunk)
@@ -993,10 +994,27 @@ def gla_scan_chunked(proj: torch.Tensor, offs, ld: torch.Tensor, norm_w: torch.T
     p.chunk_first, p.chunk_len, p.n_chunks, p.n_tokens, p.dtype, p.n_seqs = plan["first"].data_ptr(), plan["len"].data_ptr(), nc, batch.n_tokens, dtype_code(dt), batch.n_seqs
     p.qd, p.kd, p.g, p.vf, p.a = qd.data_ptr(), kd.data_ptr(), g.data_ptr(), vf.data_ptr(), a.data_ptr()
     _check(load().pcs_gla_chunk_prep(C.byref(p), _stream()), "pcs_gla_chunk_prep")
-    u = torch.bmm(kd.transpose(1, 2), vf)                  # [chunks * H, dim, vdim]: every chunk's own sum of k v^T, decayed to its end
-    p.u, p.s_pool = u.data_ptr(), s_pool.data_ptr()
+    # u [chunks * H, dim, vdim]: every chunk's own sum of k v^T, decayed to its end
+    tensor_cores = dt == torch.bfloat16 and chunk == DELTA_CHUNK and D % 16 == 0 and D <= 256 and V % 8 == 0 and p.v_off % 8 == 0 and p.row_stride % 8 == 0 and p.proj % 16 == 0
+    if tensor_cores:
+        u = torch.empty(nc * H, D, V, **f32)
+        p.u = u.data_ptr()
+        _check(load().pcs_gla_chunk_sums(C.byref(p), _stream()), "pcs_gla_chunk_sums")
+    else:
+        u = torch.bmm(kd.transpose(1, 2), vf)
+        p.u = u.data_ptr()
+    p.s_pool = s_pool.data_ptr()
     p.seq_slot, p.seq_pos0, p.seq_chunk0, p.seq_chunks = batch.seq_slot.data_ptr(), batch.seq_pos0.data_ptr(), plan["seq0"].data_ptr(), plan["seqn"].data_ptr()
     _check(load().pcs_gla_chunk_scan(C.byref(p), _stream()), "pcs_gla_chunk_scan")   # u now holds the state every chunk starts from
+    if tensor_cores and V <= DELTA_OUT_MAX_VDIM:
+        # the read-out of chunks that the delta rule has too: o = qd S + a v with the head's norm and gate, in one launch
+        r, n = pcs_delta_chunk_params(), pcs_headnorm_params()
+        r.heads, r.kv_heads, r.dim, r.vdim, r.n_chunks, r.n_tokens, r.dtype, r.n_seqs = H, H, D, V, nc, batch.n_tokens, dtype_code(dt), batch.n_seqs
+        r.chunk_first, r.chunk_len, r.qd, r.u, r.a, r.s = p.chunk_first, p.chunk_len, qd.data_ptr(), vf.data_ptr(), a.data_ptr(), u.data_ptr()
+        n.w, n.g, n.g_stride, n.out, n.out_stride = norm_w.data_ptr(), proj.data_ptr() + offs[3] * proj.element_size(), proj.stride(0), out.data_ptr(), out.stride(0)
+        n.n_tokens, n.heads, n.vdim, n.eps, n.out_scale, n.dtype, n.silu = batch.n_tokens, H, V, float(eps), 1.0, dtype_code(dt), 1
+        _check(load().pcs_delta_chunk_out(C.byref(r), C.byref(n), _stream()), "pcs_delta_chunk_out")
+        return
     o = torch.baddbmm(torch.bmm(a, vf), qd, u)             # [chunks * H, chunk, vdim]
     p.o, p.tok_row, p.norm_w, p.out = o.data_ptr(), plan["tok_row"].data_ptr(), norm_w.data_ptr(), out.data_ptr()
     _check(load().pcs_gla_chunk_out(C.byref(p), _stream()), "pcs_gla_chunk_out")

@@ -356,13 +356,39 @@ constexpr int kPrepThreads = 1024;
 template <typename T>
 __global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep_kernel(const pcs_gla_chunk_params p) {
   extern __shared__ float sm[];
-  const int D = p.dim, V = p.vdim, H = p.heads, C = p.chunk, DP = D + 1;
+  // rows of whole 16-byte pieces where the channels allow it (a padding piece keeps eight neighbouring rows in different banks)
+  const int D = p.dim, V = p.vdim, H = p.heads, C = p.chunk, DP = D % 4 == 0 ? D + 4 : D + 1;
   float* qs = sm;              // [C][DP]
   float* ks = qs + C * DP;     // [C][DP]
   float* Bs = ks + C * DP;     // [C][DP]
   const int cn = blockIdx.x, head = blockIdx.y, tid = threadIdx.x;
   const int first = p.chunk_first[cn], n = p.chunk_len[cn];
   const T* proj = static_cast<const T*>(p.proj);
+  // rows in pieces of four channels, a warp per row, where the sizes allow it (bfloat16 runs)
+  const int warp = tid >> 5, lane = tid & 31;
+  auto al = [](const void* q, int b) { return (reinterpret_cast<uintptr_t>(q) & (b - 1)) == 0; };
+  const bool quads = sizeof(T) == 2 && D % 4 == 0 && V % 4 == 0 && p.q_off % 4 == 0 && p.k_off % 4 == 0 && p.v_off % 4 == 0 && p.row_stride % 4 == 0 && al(p.proj, 8) &&
+                     al(p.ld, 16) && al(p.qd, 16) && al(p.kd, 16) && al(p.vf, 16);
+  auto ld4 = [](const T* x) {
+    const uint2 u = *reinterpret_cast<const uint2*>(x);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+  };
+  if (quads) {
+    for (int i = warp; i < C; i += kPrepThreads / 32) {
+      const T* row = proj + static_cast<long long>(first + i) * p.row_stride;
+      for (int d = lane * 4; d < D; d += 128) {
+        float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv, lv = qv;
+        if (i < n) {
+          qv = ld4(row + p.q_off + head * D + d);
+          kv = ld4(row + p.k_off + head * D + d);
+          lv = *reinterpret_cast<const float4*>(p.ld + static_cast<long long>(first + i) * (H * D) + head * D + d);
+        }
+        *reinterpret_cast<float4*>(qs + i * DP + d) = make_float4(qv.x * p.q_scale, qv.y * p.q_scale, qv.z * p.q_scale, qv.w * p.q_scale);
+        *reinterpret_cast<float4*>(ks + i * DP + d) = kv;
+        *reinterpret_cast<float4*>(Bs + i * DP + d) = lv;
+      }
+    }
+  } else
   for (int e = tid; e < C * D; e += kPrepThreads) {
     const int i = e / D, d = e - i * D;
     float qv = 0.f, kv = 0.f, lv = 0.f;
@@ -389,6 +415,15 @@ __global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep_kernel(const pcs_
   float* qd = p.qd + base * C * D;
   float* kd = p.kd + base * C * D;
   const float* Be = Bs + (C - 1) * DP;
+  if (quads) {
+    for (int i = warp; i < C; i += kPrepThreads / 32)
+      for (int d = lane * 4; d < D; d += 128) {
+        const float4 b = *reinterpret_cast<const float4*>(Bs + i * DP + d), be = *reinterpret_cast<const float4*>(Be + d);
+        const float4 q = *reinterpret_cast<const float4*>(qs + i * DP + d), k = *reinterpret_cast<const float4*>(ks + i * DP + d);
+        *reinterpret_cast<float4*>(qd + i * D + d) = make_float4(q.x * expf(b.x), q.y * expf(b.y), q.z * expf(b.z), q.w * expf(b.w));
+        *reinterpret_cast<float4*>(kd + i * D + d) = make_float4(k.x * expf(be.x - b.x), k.y * expf(be.y - b.y), k.z * expf(be.z - b.z), k.w * expf(be.w - b.w));
+      }
+  } else
   for (int e = tid; e < C * D; e += kPrepThreads) {
     const int i = e / D, d = e - i * D;
     const float bi = Bs[i * DP + d];
@@ -397,6 +432,11 @@ __global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep_kernel(const pcs_
   }
   for (int d = tid; d < D; d += kPrepThreads) p.g[base * D + d] = expf(Be[d]);
   float* vf = p.vf + base * C * V;
+  if (quads) {
+    for (int i = warp; i < C; i += kPrepThreads / 32)
+      for (int c = lane * 4; c < V; c += 128)
+        *reinterpret_cast<float4*>(vf + i * V + c) = i < n ? ld4(proj + static_cast<long long>(first + i) * p.row_stride + p.v_off + head * V + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  } else
   for (int e = tid; e < C * V; e += kPrepThreads) {
     const int i = e / V, c = e - i * V;
     vf[e] = i < n ? ldf(proj + static_cast<long long>(first + i) * p.row_stride + p.v_off + head * V + c) : 0.f;
@@ -417,24 +457,136 @@ __global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep_kernel(const pcs_
     }
   }
   __syncthreads();
-  const int half = (C + 1) / 2;
-  for (int e = tid; e < half * (C + 1); e += kPrepThreads) {
+  const int half = (C + 1) / 2, places = half * (C + 1);
+  auto pair_at = [&](int e, int& i, int& s_) {
     const int r = e / (C + 1), j = e - r * (C + 1);
-    int i, s_;
     if (j <= r) { i = r; s_ = j; } else { i = C - 1 - r; s_ = j - r - 1; }
-    if (i >= n || s_ > i || (i == r && j > r)) continue;   // (an odd chunk's middle row is taken once)
+    return i < n && s_ <= i && !(i == r && j > r);   // (an odd chunk's middle row is taken once)
+  };
+  // bfloat16 runs: whole rounds of one pair per thread, and the pairs that are left one per warp (64 tokens: 2080 pairs are two rounds and 32 pairs)
+  const int whole = kFast ? places / kPrepThreads * kPrepThreads : places;
+  for (int e = whole + warp; e < places; e += kPrepThreads / 32) {
+    int i, s_;
+    if (!pair_at(e, i, s_)) continue;
+    float x = 0.f;
+    for (int d = lane; d < D; d += 32) x = fmaf(qs[i * DP + d] * ks[s_ * DP + d], ex2(Bs[i * DP + d] - Bs[s_ * DP + d]), x);
+    x = warp_sum(x);
+    if (lane == 0) a[i * C + s_] = x;
+  }
+  for (int e = tid; e < whole; e += kPrepThreads) {
+    int i, s_;
+    if (!pair_at(e, i, s_)) continue;
     const float* qi = qs + i * DP;
     const float* bi = Bs + i * DP;
     const float* kk = ks + s_ * DP;
     const float* bs = Bs + s_ * DP;
     float a0 = 0.f, a1 = 0.f;
     int d = 0;
+    if (kFast && D % 4 == 0) {   // four channels per read: the loop is bound by shared memory (with the loads in pieces and the pairs in whole rounds: 86 -> 56 us at 136 chunks of 256 channels)
+#pragma unroll 2
+      for (; d < D; d += 4) {
+        const float4 q4 = *reinterpret_cast<const float4*>(qi + d), k4 = *reinterpret_cast<const float4*>(kk + d);
+        const float4 b4 = *reinterpret_cast<const float4*>(bi + d), c4 = *reinterpret_cast<const float4*>(bs + d);
+        a0 = fmaf(q4.x * k4.x, ex2(b4.x - c4.x), a0);
+        a1 = fmaf(q4.y * k4.y, ex2(b4.y - c4.y), a1);
+        a0 = fmaf(q4.z * k4.z, ex2(b4.z - c4.z), a0);
+        a1 = fmaf(q4.w * k4.w, ex2(b4.w - c4.w), a1);
+      }
+    }
     for (; d + 1 < D; d += 2) {
       a0 = fmaf(qi[d] * kk[d], kFast ? ex2(bi[d] - bs[d]) : expf(bi[d] - bs[d]), a0);
       a1 = fmaf(qi[d + 1] * kk[d + 1], kFast ? ex2(bi[d + 1] - bs[d + 1]) : expf(bi[d + 1] - bs[d + 1]), a1);
     }
     if (d < D) a0 = fmaf(qi[d] * kk[d], kFast ? ex2(bi[d] - bs[d]) : expf(bi[d] - bs[d]), a0);
     a[i * C + s_] = a0 + a1;
+  }
+}
+
+// A chunk's own sum of k v^T, decayed to its end: u[c, h] = kd[c, h]^T v (bfloat16 runs, chunks of 64).  kd is 32-bit and enters the tensor cores as three
+// bfloat16 parts (all 24 bits of it), v is bfloat16 already, the sums are 32-bit: as exact as the library's 32-bit product this stands for, which runs on the
+// multiply-add units (59 us at 34 chunks x 4 heads of 256 x 512; this: 38 us).  Block = (chunk, head, 128 value columns), a warp = 32 channels x 64 columns
+// per turn; kd stays 32-bit in shared memory and is taken apart in registers (rows D + 4 numbers apart: a fragment's eight channels x four token pairs lie in
+// different banks).
+constexpr int kSumsThreads = 256, kSumsCols = 128, kSumsChunk = 64, kSumsRow = kSumsCols + 8;
+__global__ void __launch_bounds__(kSumsThreads, 2) gla_chunk_sums_kernel(const pcs_gla_chunk_params p) {
+  extern __shared__ __align__(16) float sm[];
+  const int D = p.dim, V = p.vdim, H = p.heads, LK = D + 4;
+  float* Ks = sm;                                                                  // [64][D + 4]
+  __nv_bfloat16* Vs = reinterpret_cast<__nv_bfloat16*>(Ks + kSumsChunk * LK);      // [64][136]
+  const int cn = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * kSumsCols, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = lane >> 2, qd = lane & 3;
+  const long long base = static_cast<long long>(cn) * H + head;
+  const int first = p.chunk_first[cn], n = p.chunk_len[cn], pieces = D / 4;
+  const float* kd = p.kd + base * kSumsChunk * D;
+  for (int e = tid; e < kSumsChunk * pieces; e += kSumsThreads) {
+    const int r = e / pieces, c = (e - r * pieces) * 4;
+    cp_async16(Ks + r * LK + c, kd + r * D + c);
+  }
+  const __nv_bfloat16* rows = static_cast<const __nv_bfloat16*>(p.proj) + static_cast<long long>(first) * p.row_stride + p.v_off + head * V + v0;
+#pragma unroll
+  for (int u = 0; u < kSumsChunk * kSumsCols / 8 / kSumsThreads; ++u) {
+    const int e = tid + u * kSumsThreads, r = e / (kSumsCols / 8), c = e % (kSumsCols / 8) * 8;
+    if (r < n && v0 + c < V) cp_async16(Vs + r * kSumsRow + c, rows + r * p.row_stride + c);
+    else *reinterpret_cast<uint4*>(Vs + r * kSumsRow + c) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const uint32_t v_base = static_cast<uint32_t>(__cvta_generic_to_shared(Vs)) + ((lane & 15) * kSumsRow + (lane >> 4) * 8) * 2;
+  float* U = p.u + base * D * V;
+  // a pair of neighbouring tokens at one channel as three packed parts
+  auto parts = [](float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+    h = pack_bf16(x0, x1);
+    x0 -= __uint_as_float(h << 16);
+    x1 -= __uint_as_float(h & 0xffff0000u);
+    m = split_pair(x0, x1, l);
+  };
+  for (int w = warp; w < (D + 31) / 32 * 2; w += kSumsThreads / 32) {
+    const int d0 = (w >> 1) * 32, c0 = (w & 1) * 64;
+    if (v0 + c0 >= V) continue;
+    float acc[2][8][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < kSumsChunk / 16; ++ks) {
+      uint32_t f[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) ldsm_x4_t(v_base + (ks * 16 * kSumsRow + c0 + u * 16) * 2, f[u][0], f[u][1], f[u][2], f[u][3]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        float step[8][4];   // sums of sixteen tokens join in rounded additions: the tensor core's own running sum cuts bits off (1.35e-7 -> 1.5e-7 of a state)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) step[j][0] = step[j][1] = step[j][2] = step[j][3] = 0.f;
+        uint32_t a[3][4];   // [part][fragment register]: channels grp, grp + 8; tokens 2 qd.., 2 qd + 8..
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int d = d0 + i * 16 + grp + (q & 1) * 8, s = ks * 16 + 2 * qd + (q >> 1) * 8;
+          const float* k = Ks + s * LK + min(d, D - 1);
+          parts(k[0], k[LK], a[0][q], a[1][q], a[2][q]);
+        }
+#pragma unroll
+        for (int x = 2; x >= 0; --x)   // the smallest part first
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            mma_bf16(step[2 * u], a[x][0], a[x][1], a[x][2], a[x][3], f[u][0], f[u][1]);
+            mma_bf16(step[2 * u + 1], a[x][0], a[x][1], a[x][2], a[x][3], f[u][2], f[u][3]);
+          }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc[i][j][q] += step[j][q];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int d = d0 + i * 16 + grp, col = v0 + c0 + j * 8 + qd * 2;
+        if (col >= V) continue;
+        if (d < D) *reinterpret_cast<float2*>(U + static_cast<long long>(d) * V + col) = make_float2(acc[i][j][0], acc[i][j][1]);
+        if (d + 8 < D) *reinterpret_cast<float2*>(U + static_cast<long long>(d + 8) * V + col) = make_float2(acc[i][j][2], acc[i][j][3]);
+      }
   }
 }
 
@@ -504,12 +656,30 @@ PCS_API int pcs_gla_chunk_prep(const pcs_gla_chunk_params* p, void* stream) {
   if (p->n_chunks == 0) return PCS_OK;
   PCS_REQUIRE(p->proj && p->ld && p->chunk_first && p->chunk_len && p->qd && p->kd && p->g && p->vf && p->a, "pcs_gla_chunk_prep: null tensor");
   PCS_REQUIRE(p->heads > 0 && p->heads <= 65535 && p->dim > 0 && p->vdim > 0 && p->chunk > 0, "pcs_gla_chunk_prep: bad sizes");
-  const size_t smem = static_cast<size_t>(3) * p->chunk * (p->dim + 1) * sizeof(float);
+  const size_t smem = static_cast<size_t>(3) * p->chunk * (p->dim % 4 == 0 ? p->dim + 4 : p->dim + 1) * sizeof(float);
   PCS_REQUIRE(smem <= 220 * 1024, "pcs_gla_chunk_prep: a chunk of %d tokens x %d channels exceeds shared memory", p->chunk, p->dim);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (smem > 48 * 1024)
     PCS_DISPATCH(p->dtype, PCS_CHECK_CUDA(cudaFuncSetAttribute(pcs::gla_chunk_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
   PCS_DISPATCH(p->dtype, pcs::gla_chunk_prep_kernel<T><<<dim3(p->n_chunks, p->heads), pcs::kPrepThreads, smem, st>>>(*p));
+  PCS_CHECK_CUDA(cudaGetLastError());
+  pcs::count_launch();
+  return PCS_OK;
+}
+
+// PCS_ERR_UNSUPPORTED: other types, chunks or sizes (the caller forms the product itself)
+PCS_API int pcs_gla_chunk_sums(const pcs_gla_chunk_params* p, void* stream) {
+  PCS_REQUIRE(p, "pcs_gla_chunk_sums: null params");
+  if (p->n_chunks == 0) return PCS_OK;
+  PCS_REQUIRE(p->proj && p->kd && p->u && p->chunk_first && p->chunk_len && p->heads > 0 && p->heads <= 65535 && p->dim > 0 && p->vdim > 0, "pcs_gla_chunk_sums: bad arguments");
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (p->dtype != PCS_BF16 || p->chunk != pcs::kSumsChunk || p->dim % 16 != 0 || p->dim > 256 || p->vdim % 8 != 0 || p->v_off % 8 != 0 || p->row_stride % 8 != 0 ||
+      !al16(p->proj) || !al16(p->kd) || !al16(p->u))
+    return pcs::set_error(PCS_ERR_UNSUPPORTED, "pcs_gla_chunk_sums: serves bfloat16 in 16-byte pieces, chunks of %d, dim a multiple of 16 up to 256", pcs::kSumsChunk);
+  auto smem = [](int D) { return static_cast<size_t>(pcs::kSumsChunk) * (D + 4) * sizeof(float) + static_cast<size_t>(pcs::kSumsChunk) * pcs::kSumsRow * 2; };
+  PCS_CHECK_CUDA(cudaFuncSetAttribute(pcs::gla_chunk_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem(256))));
+  pcs::gla_chunk_sums_kernel<<<dim3(p->n_chunks, p->heads, (p->vdim + pcs::kSumsCols - 1) / pcs::kSumsCols), pcs::kSumsThreads, smem(p->dim),
+                               static_cast<cudaStream_t>(stream)>>>(*p);
   PCS_CHECK_CUDA(cudaGetLastError());
   pcs::count_launch();
   return PCS_OK;
