@@ -17,8 +17,8 @@ from ._native import NativeError, note_replayed_launches  # noqa: F401  (one err
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libpromptcache_b200_seq.so")
 PCS_BF16, PCS_F32 = 0, 1
-EXPORTS = ("pcs_version", "pcs_last_error", "pcs_launch_count", "pcs_attn_workspace_floats", "pcs_attn_timeouts", "pcs_embed", "pcs_rmsnorm", "pcs_gate_norm_add", "pcs_xielu", "pcs_linear_rows",
-           "pcs_qk_prep", "pcs_attn", "pcs_mlstm_gates", "pcs_mlstm_scan", "pcs_mlstm_scratch_floats", "pcs_embed_bigram", "pcs_norm_conv", "pcs_rope_kv_prep", "pcs_moe_route",
+EXPORTS = ("pcs_version", "pcs_last_error", "pcs_launch_count", "pcs_attn_workspace_floats", "pcs_mlstm_scratch_floats", "pcs_attn_timeouts", "pcs_embed", "pcs_rmsnorm", "pcs_gate_norm_add", "pcs_xielu", "pcs_linear_rows",
+           "pcs_qk_prep", "pcs_attn", "pcs_mlstm_gates", "pcs_mlstm_scan", "pcs_embed_bigram", "pcs_norm_conv", "pcs_rope_kv_prep", "pcs_moe_route",
            "pcs_moe_rows_up", "pcs_moe_rows_down", "pcs_moe_plan", "pcs_moe_gather", "pcs_moe_gemm", "pcs_moe_combine", "pcs_silu_mul", "pcs_glu_mul",
            "pcs_depth_mix", "pcs_latent_prep", "pcs_latent_q", "pcs_latent_gather", "pcs_latent_expand", "pcs_head_gate", "pcs_gla_decay", "pcs_gla_scan", "pcs_gla_chunk_prep", "pcs_gla_chunk_sums", "pcs_gla_chunk_scan", "pcs_gla_chunk_out",
            "pcs_add_layer_norm", "pcs_gru_scan", "pcs_group_norm_conv", "pcs_soft_cap", "pcs_short_conv", "pcs_delta_inputs", "pcs_delta_scan", "pcs_delta_chunk_prep", "pcs_delta_chunk_scan",
@@ -232,6 +232,7 @@ def load() -> C.CDLL:
     lib.pcs_version.restype = C.c_int
     lib.pcs_last_error.restype = C.c_char_p
     lib.pcs_launch_count.restype = C.c_int64
+    lib.pcs_mlstm_scratch_floats.argtypes = [C.c_int] * 5
     lib.pcs_mlstm_scratch_floats.restype = C.c_int64
     lib.pcs_embed.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_float, C.c_int, C.c_void_p]
     lib.pcs_rmsnorm.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_float, C.c_int, C.c_void_p]
@@ -274,7 +275,7 @@ def load() -> C.CDLL:
     lib.pcs_gla_decay.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_float, C.c_void_p, C.c_int,
                                   C.c_int, C.c_int, C.c_void_p]
     lib.pcs_gla_scan.argtypes = [C.POINTER(pcs_gla_params), C.c_void_p]
-    for name in ("pcs_gla_chunk_prep", "pcs_gla_chunk_scan", "pcs_gla_chunk_out"):
+    for name in ("pcs_gla_chunk_prep", "pcs_gla_chunk_sums", "pcs_gla_chunk_scan", "pcs_gla_chunk_out"):
         getattr(lib, name).argtypes = [C.POINTER(pcs_gla_chunk_params), C.c_void_p]
     lib.pcs_add_layer_norm.argtypes = [C.POINTER(pcs_addln_params), C.c_void_p]
     lib.pcs_gru_scan.argtypes = [C.POINTER(pcs_gru_params), C.c_void_p]
@@ -289,7 +290,7 @@ def load() -> C.CDLL:
     lib.pcs_delta_chunk_out.argtypes = [C.POINTER(pcs_delta_chunk_params), C.POINTER(pcs_headnorm_params), C.c_void_p]
     lib.pcs_side_boundary.argtypes = [C.POINTER(pcs_side_params), C.c_void_p]
     lib.pcs_side_gate.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
-    for name in EXPORTS[4:]:
+    for name in EXPORTS[5:]:   # the first five: a version, a string and three 64-bit counts
         getattr(lib, name).restype = C.c_int
     _lib = lib
     return lib
