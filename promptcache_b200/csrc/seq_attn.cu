@@ -535,16 +535,6 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
   const bool decode = (p->impl == 0 || p->impl == 2) && p->workspace != nullptr && p->dim % piece == 0 && p->vdim % piece == 0 &&
                       p->vdim / piece <= pcs::kAttnThreads && p->v_row_stride % piece == 0;
   int splits = 1;
-  if (decode && p->impl == 0) {
-    if (int rc = pcs::launch_attn_group_decode(*p, st, &splits)) return rc;
-    if (splits > 1) {
-      PCS_DISPATCH(p->dtype, pcs::attn_combine_kernel<T><<<dim3(p->n_tokens, p->n_heads, (p->vdim + pcs::kAttnThreads - 1) / pcs::kAttnThreads), pcs::kAttnThreads, 0, st>>>(*p, splits));
-      PCS_CHECK_CUDA(cudaGetLastError());
-      pcs::count_launch();
-    }
-    if (splits > 0) return PCS_OK;
-    splits = 1;
-  }
   if (p->workspace != nullptr && p->max_keys > 512) {
     const long long blocks = static_cast<long long>(p->n_tokens) * p->n_heads;
     const int want = static_cast<int>((2 * 148 + blocks - 1) / blocks);
@@ -554,6 +544,16 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
     if (splits < 1) splits = 1;
     PCS_REQUIRE(splits == 1 || p->workspace_floats >= static_cast<long long>(p->n_tokens) * p->n_heads * splits * (p->vdim + 2),
                 "pcs_attn: workspace too small for %d splits", splits);
+  }
+  if (decode && p->impl == 0) {
+    int parts = 0;
+    if (int rc = pcs::launch_attn_group_decode(*p, st, &parts)) return rc;
+    if (parts > 1) {
+      PCS_DISPATCH(p->dtype, pcs::attn_combine_kernel<T><<<dim3(p->n_tokens, p->n_heads, (p->vdim + pcs::kAttnThreads - 1) / pcs::kAttnThreads), pcs::kAttnThreads, 0, st>>>(*p, parts));
+      PCS_CHECK_CUDA(cudaGetLastError());
+      pcs::count_launch();
+    }
+    if (parts > 0) return PCS_OK;
   }
   dim3 grid(p->n_tokens, p->n_heads, splits);
   if (decode) {

@@ -320,12 +320,16 @@ int launch(const pcs_attn_params& p, int* splits_io, int per_group, cudaStream_t
   int splits = *splits_io;
   bool cluster = true;
   if (splits > 2 * kMaxCluster && groups * kMaxCluster * 2 <= room[1]) {
-    cluster = false;
     const long long want = room[1] / groups;
-    if (splits > want) splits = static_cast<int>(want);
-    if (splits > kAttnMaxSplits) splits = kAttnMaxSplits;
-    PCS_REQUIRE(p.workspace_floats >= static_cast<long long>(p.n_tokens) * p.n_heads * splits * (p.vdim + 2), "pcs_attn: workspace too small for %d splits", splits);
-  } else {
+    int wide = splits > want ? static_cast<int>(want) : splits;
+    if (wide > kAttnMaxSplits) wide = kAttnMaxSplits;
+    // (a workspace that holds only the fewer splits that pcs_attn asks for: a cluster, which needs none)
+    if (p.workspace_floats >= static_cast<long long>(p.n_tokens) * p.n_heads * wide * (p.vdim + 2)) {
+      cluster = false;
+      splits = wide;
+    }
+  }
+  if (cluster) {
     if (splits > kMaxCluster) splits = kMaxCluster;
     while (splits > 1 && room[splits] < groups) --splits;
     if (splits < 1) splits = 1;

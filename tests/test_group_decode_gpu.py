@@ -25,7 +25,7 @@ def check(nsq, name, H, G, D, V, lens, pos0, dt, workspace, seed):
     out = torch.empty(T, H * V, device=DEV, dtype=dt)
     opt = {a: x for a, x in o.items() if a not in ("r1", "r2", "sink")}
     if workspace:
-        opt.update(workspace=nsq.attn_workspace(T, H, V, torch.device(DEV)), max_keys=cap)
+        opt.update(workspace=nsq.attn_workspace(T, H, V, torch.device(DEV))[:None if workspace is True else workspace], max_keys=cap)
     nsq.attention(q, k, v, out, H, D ** -0.5, o.get("r1"), o.get("r2"), o.get("sink", False), nsq.Batch(slots, pos0, lens, torch.device(DEV)), **opt)
     off = 0
     for b, (n, p) in enumerate(zip(lens, pos0)):
@@ -63,6 +63,14 @@ def test_group_decode(nsq, shape, name):  # noqa: F811
 
 def test_several_tokens_of_a_sequence(nsq):  # noqa: F811
     check(nsq, "bias", 8, 2, 128, 128, (3, 1, 5), (200, 0, 1000), BF16, True, 5)
+
+
+def test_workspace_of_fewer_splits(nsq):  # noqa: F811
+    """20 heads over 24 x 128 keys ask for 15 splits; a workspace that holds no more is enough, one float less is refused."""
+    floats = 20 * 15 * (256 + 2)
+    check(nsq, "plain", 20, 1, 256, 256, (1,), (3000,), BF16, floats, 3)
+    with pytest.raises(nsq.NativeError, match="workspace too small"):
+        check(nsq, "plain", 20, 1, 256, 256, (1,), (3000,), BF16, floats - 1, 3)
 
 
 PROMPT32 = [
