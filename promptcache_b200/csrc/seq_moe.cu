@@ -188,32 +188,35 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const pcs_route_params p
   route_select(p, t, lane, z, c, gs);
 }
 
-// The same with one WARP per token (many tokens): the eight warps of a block walk the router's rows together, so a row comes
-// from L2 once per eight tokens; each warp then selects for its own token.  Results equal the block-per-token kernel's.
-constexpr int kWarpRouteOutputs = 256;
+// The same for many tokens: two tokens per block, four warps per token.  Each warp takes every fourth router output (a row comes from L1 for the second
+// token), the first one then selects.  Bound by the latency of the dots' loads, so what counts is the warps in flight: with one warp per token (eight
+// tokens per block) 14 warps per SM walked all outputs, 38 us of a feed-forward of 197 us at 2048 tokens, 16 outputs, width 2048 (B200); now it is 188 us.  (Four
+// rows at a time in one warp: 43.8 us, its registers leave one block per SM.)  An output's sum is one warp's, so results equal the block-per-token kernel's.
+constexpr int kWarpRouteOutputs = 256, kRouteTokens = 2, kRouteWarps = 8 / kRouteTokens;
 template <typename T>
 __global__ void __launch_bounds__(256) moe_route_warp_kernel(const pcs_route_params p) {
-  __shared__ float buf[8][4 * kWarpRouteOutputs];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, E = p.n_outputs, K = p.width;
-  const int t = blockIdx.x * 8 + warp;
-  if (t >= p.n_tokens) return;
-  float* z = buf[warp];
+  __shared__ float buf[kRouteTokens][4 * kWarpRouteOutputs];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = warp % kRouteWarps, E = p.n_outputs, K = p.width;
+  const int t = blockIdx.x * kRouteTokens + warp / kRouteWarps;
+  float* z = buf[warp / kRouteWarps];
   float* c = z + kWarpRouteOutputs;
   float* gs = c + kWarpRouteOutputs;
-  const T* h = static_cast<const T*>(p.h) + static_cast<long long>(t) * p.h_stride;
-  const T* wr = static_cast<const T*>(p.w_router);
-  const bool vec = K % Vec<T>::n == 0 && aligned16(h) && aligned16(wr) && (p.h_stride * sizeof(T)) % 16 == 0;
-  for (int e = 0; e < E; ++e) {
-    const float d = warp_dot(h, wr + static_cast<long long>(e) * K, K, lane, vec);
-    if (lane == 0) z[e] = d;
+  if (t < p.n_tokens) {
+    const T* h = static_cast<const T*>(p.h) + static_cast<long long>(t) * p.h_stride;
+    const T* wr = static_cast<const T*>(p.w_router);
+    const bool vec = K % Vec<T>::n == 0 && aligned16(h) && aligned16(wr) && (p.h_stride * sizeof(T)) % 16 == 0;
+    for (int e = sub; e < E; e += kRouteWarps) {
+      const float d = warp_dot(h, wr + static_cast<long long>(e) * K, K, lane, vec);
+      if (lane == 0) z[e] = d;
+    }
+    if (p.w_sg && sub == kRouteWarps - 1) {
+      const T* ws = static_cast<const T*>(p.w_sg);
+      const float d = warp_dot(h, ws, K, lane, vec && aligned16(ws));
+      if (lane == 0) p.shared_gate[t] = sigmoidf_(d);
+    }
   }
-  if (p.w_sg) {
-    const T* ws = static_cast<const T*>(p.w_sg);
-    const float d = warp_dot(h, ws, K, lane, vec && aligned16(ws));
-    if (lane == 0) p.shared_gate[t] = sigmoidf_(d);
-  }
-  __syncwarp();
-  route_select(p, t, lane, z, c, gs);
+  __syncthreads();
+  if (t < p.n_tokens && sub == 0) route_select(p, t, lane, z, c, gs);
 }
 
 // block = (pair, 8 features); warp w owns features n0 + 2w, n0 + 2w + 1
@@ -357,7 +360,7 @@ PCS_API int pcs_moe_route(const pcs_route_params* p, void* stream) {
   PCS_REQUIRE(p->w_sg == nullptr || p->shared_gate != nullptr, "pcs_moe_route: the shared gate needs its output");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (p->n_tokens >= 64 && p->n_outputs <= pcs::kWarpRouteOutputs)
-    PCS_DISPATCH(p->dtype, pcs::moe_route_warp_kernel<T><<<(p->n_tokens + 7) / 8, 256, 0, st>>>(*p));
+    PCS_DISPATCH(p->dtype, pcs::moe_route_warp_kernel<T><<<(p->n_tokens + pcs::kRouteTokens - 1) / pcs::kRouteTokens, 256, 0, st>>>(*p));
   else
     PCS_DISPATCH(p->dtype, pcs::moe_route_kernel<T><<<p->n_tokens, 256, 0, st>>>(*p));
   PCS_CHECK_CUDA(cudaGetLastError());
