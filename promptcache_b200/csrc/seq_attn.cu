@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_plain_kernel(const pcs_attn
     const float tmax = block_max(s, red);
     const float m_new = fmaxf(m, tmax);
     const float f = (m == -INFINITY) ? 0.f : expf(m - m_new);
-    const float w = (j0 + tid < k_end) ? expf(s - m_new) : 0.f;
+    const float w = (j0 + tid < k_end) ? expf(s - (m_new == -INFINITY ? 0.f : m_new)) : 0.f;   // (a bias table may hide every key so far)
     ws[tid] = w;
     const float tsum = block_sum(w, red);  // its barriers also publish ws
     l = l * f + tsum;
@@ -343,10 +343,10 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_kernel(const pcs_att
     float tmax = red[0];
 #pragma unroll
     for (int i = 1; i < kAttnThreads / 32; ++i) tmax = fmaxf(tmax, red[i]);
-    const float m_new = fmaxf(m, tmax);  // finite: a tile has at least one key
+    const float m_new = fmaxf(m, tmax);  // minus infinity while the bias table hides every key so far
     const float f = (m == -INFINITY) ? 0.f : expf(m - m_new);
     m = m_new;
-    ws[tid] = (j0 + tid < k_end) ? expf(s - m_new) : 0.f;
+    ws[tid] = (j0 + tid < k_end) ? expf(s - (m_new == -INFINITY ? 0.f : m_new)) : 0.f;
     __syncthreads();
     if (active) {
       const int nt = min(kAttnThreads, k_end - j0);

@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kThreads) attn_group_decode_kernel(const pcs_a
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1)
       if (o < C::DUP || o >= C::DUP * GP) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    const float m_new = fmaxf(m, mx);   // finite: a tile has at least one key
+    const float m_new = fmaxf(m, mx);   // minus infinity while the bias table hides every key so far (a tile has as few as four)
     if (__any_sync(0xffffffffu, m_new != m)) {
       const float f = m == -INFINITY ? 0.f : expf(m - m_new);
       l *= f;
@@ -175,10 +175,11 @@ __global__ void __launch_bounds__(kThreads) attn_group_decode_kernel(const pcs_a
         for (int e = 0; e < N; ++e) acc[hh][e] *= fh;
       }
     }
+    const float sub = m == -INFINITY ? 0.f : m;   // hidden scores then give exp(-inf) = 0
     __syncwarp();   // the previous tile's weights have been read
 #pragma unroll
     for (int grp = 0; grp < kLoads / C::NG; ++grp) {
-      const float w = expf(s[grp] - m);
+      const float w = expf(s[grp] - sub);
       if (first_of_dups) {
         l += w;
         w_tile[((grp * C::NG + own_i) * C::RK + rk) * GP + own_h] = w;
