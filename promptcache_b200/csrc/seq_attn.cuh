@@ -30,4 +30,57 @@ __device__ __forceinline__ float out_factor(const pcs_attn_params& p, int t, int
   return f;
 }
 
+// Columns [c0, c0 + n) of the result of head h of token t (entry b, position pos), by one warp with multiply-adds over the visible keys alone; n <= 128,
+// rows in 16-byte pieces.  A matrix product over tiles of keys multiplies hidden keys by a weight of 0, and 0 * inf is not 0: a query whose result is not
+// finite there is formed again here, so that rows it does not see cannot reach it.
+template <typename T>
+__device__ __forceinline__ void attn_row_again(const pcs_attn_params& p, int b, int h, int t, int pos, int c0, int n) {
+  constexpr int N = Vec<T>::n;
+  const int lane = threadIdx.x & 31, D = p.dim, slot = p.pool_slot ? p.pool_slot[b] : p.seq_slot[b];
+  const long long VS = p.v_row_stride > 0 ? p.v_row_stride : p.vdim, plane = (static_cast<long long>(slot) * p.n_kv_heads + h / (p.n_heads / p.n_kv_heads)) * p.cap;
+  const T* q = static_cast<const T*>(p.q) + (static_cast<long long>(t) * p.n_heads + h) * D;
+  const T* K = static_cast<const T*>(p.k_pool) + plane * D;
+  const T* Vp = static_cast<const T*>(p.v_pool) + plane * VS + c0;
+  const float scale = p.scale * (p.head_scale ? p.head_scale[h] : 1.f), r1 = p.bias_r1 ? p.bias_r1[h] : 0.f, r2 = p.bias_r1 ? p.bias_r2[h] : 0.f;
+  const float* tab = p.bias_table ? p.bias_table + static_cast<long long>(h) * p.bias_len : nullptr;
+  const VisibleKeys vis(pos, p.window, p.keep_first, p.chunk);
+  float m = p.sink ? (p.sink_logit ? p.sink_logit[h] : 0.f) : -INFINITY, l = p.sink ? 1.f : 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int j0 = 0; j0 < vis.count; j0 += 32) {
+    const int nt = min(32, vis.count - j0);
+    float s = -INFINITY;
+    if (lane < nt) {
+      const int j = vis.key(j0 + lane);
+      float a = 0.f;
+      for (int d = 0; d < D; d += N) {
+        float x[N], y[N];
+        ld16(q + d, x);
+        ld16(K + static_cast<long long>(j) * D + d, y);
+#pragma unroll
+        for (int e = 0; e < N; ++e) a = fmaf(x[e], y[e], a);
+      }
+      s = a * scale;
+      if (p.softcap > 0.f) s = p.softcap * tanhf(s / p.softcap);
+      if (p.bias_r1) s -= r1 * log1pf(r2 * static_cast<float>(pos - j));
+      if (tab) s += tab[min(pos - j, p.bias_len - 1)];
+    }
+    const float mn = fmaxf(m, warp_max(s)), f = m == -INFINITY ? 0.f : expf(m - mn);
+    const float w = lane < nt ? expf(s - (mn == -INFINITY ? 0.f : mn)) : 0.f;
+    m = mn;
+    l = l * f + warp_sum(w);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[u] *= f;
+    for (int i = 0; i < nt; ++i) {
+      const float wi = __shfl_sync(0xffffffffu, w, i);
+      const T* v = Vp + static_cast<long long>(vis.key(j0 + i)) * VS;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (lane + 32 * u < n) acc[u] = fmaf(wi, ldf(v + lane + 32 * u), acc[u]);
+    }
+  }
+  const float inv = (l > 0.f ? 1.f / l : 0.f) * out_factor<T>(p, t, h);
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (lane + 32 * u < n) stf(out_row<T>(p, t, h) + c0 + lane + 32 * u, acc[u] * inv);
+}
+
 }  // namespace pcs

@@ -5,7 +5,8 @@
 // pieces along the summed index (rows padded by 16 bytes: eight lanes read eight rows without a bank conflict), 64 multiply-adds per 8 reads, two per
 // instruction.  K of the next tile travels (cp.async) while V is multiplied, V while the scores are formed.  Two blocks share an SM; the blocks
 // with the most keys come first and every second group of 148 runs backwards, so that a long block is paired with a short one.
-// Distance biases are evaluated once per distance and tile; expf, log1pf and tanhf as in the plain kernel.
+// Distance biases are evaluated once per distance and tile; expf, log1pf and tanhf as in the plain kernel.  A row whose result is not finite is formed again
+// from the keys it sees alone (attn_row_again).
 //
 // 8 heads of 128 (B200), against the plain kernel (one block per token and head, every row read again): 1024 tokens 818 -> 103 us (21 TFLOP/s), 2048: 2.92 -> 0.32
 // ms, 64 behind 400 stored 76 -> 21 us, 16 behind 4000 100 -> 69 us.  A cluster shares a walk where there are few blocks (choose_splits).
@@ -28,7 +29,7 @@ __device__ __forceinline__ void fma_x2(float2& d, float2 a, float2 b) {
 
 // VP: value columns padded to 64 or 128
 template <int VP>
-__global__ void __launch_bounds__(F_THREADS) attn_f32_kernel(const pcs_attn_params p, const int splits) {
+__global__ void __launch_bounds__(F_THREADS) attn_f32_kernel(const __grid_constant__ pcs_attn_params p, const int splits) {
   constexpr int VC = VP / 64;              // 4-column pieces of a thread's result row
   extern __shared__ __align__(16) float sm[];
   const int D = p.dim, V = p.vdim, LD = D + 4;
@@ -183,6 +184,12 @@ __global__ void __launch_bounds__(F_THREADS) attn_f32_kernel(const pcs_attn_para
     }
     __syncthreads();   // V, the weights and the biases may be written over
   }
+  unsigned again = 0u;   // rows whose result is not finite, as far as this thread has seen it
+  auto put = [&](int t, int row, int c, float4 x) {
+    *reinterpret_cast<float4*>(out_row<float>(p, t, h) + c) = x;
+    const float zero = fmaf(x.x, 0.f, x.y * 0.f) + fmaf(x.z, 0.f, x.w * 0.f);   // NaN where one of them is not finite
+    if (zero != 0.f) again |= 1u << row;
+  };
   if (splits > 1) {
     // A cluster shares the walk: block q owns the rows [q, q + 1) * 32 / splits, to which the others send their sums (over its V tile) and (m, l)
     const int mine = FM / splits;
@@ -220,23 +227,30 @@ __global__ void __launch_bounds__(F_THREADS) attn_f32_kernel(const pcs_attn_para
       }
       const int t = off + q0 + row;
       const float inv = (lt > 0.f ? 1.f / lt : 0.f) * out_factor<float>(p, t, h);
-      *reinterpret_cast<float4*>(out_row<float>(p, t, h) + c) = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
+      put(t, row, c, make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv));
     }
-    return;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int x = 8; x >= 1; x >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], x);
+      const int row = ty + 8 * i;
+      if (row >= rows) continue;
+      const int t = off + q0 + row;
+      const float inv = (l[i] > 0.f ? 1.f / l[i] : 0.f) * out_factor<float>(p, t, h);
+#pragma unroll
+      for (int c = 0; c < VC; ++c)
+        if (c * 64 + tx * 4 < V) put(t, row, c * 64 + tx * 4, make_float4(o[i][c][0].x * inv, o[i][c][0].y * inv, o[i][c][1].x * inv, o[i][c][1].y * inv));
+    }
   }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-#pragma unroll
-    for (int x = 8; x >= 1; x >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], x);
-    const int row = ty + 8 * i;
-    if (row >= rows) continue;
-    const int t = off + q0 + row;
-    const float inv = (l[i] > 0.f ? 1.f / l[i] : 0.f) * out_factor<float>(p, t, h);
-    float* out = out_row<float>(p, t, h);
-#pragma unroll
-    for (int c = 0; c < VC; ++c)
-      if (c * 64 + tx * 4 < V)
-        *reinterpret_cast<float4*>(out + c * 64 + tx * 4) = make_float4(o[i][c][0].x * inv, o[i][c][0].y * inv, o[i][c][1].x * inv, o[i][c][1].y * inv);
+  if (__syncthreads_or(again != 0u)) {
+    unsigned* rows_again = reinterpret_cast<unsigned*>(Ts);
+    if (tid == 0) *rows_again = 0u;
+    __syncthreads();
+    if (again) atomicOr(rows_again, again);
+    __syncthreads();
+    for (unsigned w = *rows_again, k = 0; w; w &= w - 1, ++k)
+      if ((k & 3) == tid >> 5) attn_row_again<float>(p, b, h, off + q0 + __ffs(w) - 1, first + __ffs(w) - 1, 0, V);
   }
 }
 
