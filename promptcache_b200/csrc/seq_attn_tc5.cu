@@ -9,7 +9,8 @@
 //
 // The 32-bit weights enter the tensor cores as P = hi + lo (hi = bf16(P), lo = bf16(P - hi)), so ~16 bits of each are kept: three 128 x 64 x 128
 // products per tile and half where a plain flash kernel has two.  TMEM: S 4 x 64 columns, O 2 x vdim columns.  The accumulator is rescaled only when
-// a row's maximum grew by more than 2^8 (P then stays below 2^8, exact in the same 16 bits).
+// a row's maximum grew by more than 2^8 (P then stays below 2^8, exact in the same 16 bits).  The products multiply hidden keys of a tile by 0: a row
+// whose result is not finite is formed again from the keys it sees (attn_row_again).
 //
 // Which two tiles a block takes: neighbours of one head (2m, 2m + 1), those with the most keys in the first blocks; or one from either end (m,
 // n - 1 - m), which gives every block of a sequence the same work.  Where that leaves SMs idle (few new tokens behind many stored ones) a cluster of 2,
@@ -19,6 +20,7 @@
 // rate; without any softmax arithmetic the walk takes 1.24 us.  Against the mma.sync kernel it replaces (seq_attn_tc.cu, which still serves wider heads):
 //   2048 new tokens                  120 ->  44 us        6144 and 2311 new tokens          836 -> 247 us (714 TFLOP/s of the two-product count)
 //   256 behind 4000 stored           167 ->  37 us        four continued prompts, window 1024, cap  172 -> 84 us
+#include "seq_attn.cuh"
 #include "seq_mma.cuh"
 #include "seq_tc5.cuh"
 
@@ -77,20 +79,12 @@ struct Range {
   __device__ __forceinline__ bool has(int k) const { return k < n_first || (k >= lo && k < hi); }
 };
 
-// where row t of head h is written, and what its sum of weighted values is multiplied by
-__device__ __forceinline__ __nv_bfloat16* out_row(const pcs_attn_params& p, long long t, int h) {
-  return static_cast<__nv_bfloat16*>(p.out) + t * (p.out_stride > 0 ? p.out_stride : static_cast<long long>(p.n_heads) * p.vdim) + h * p.vdim;
-}
-__device__ __forceinline__ float out_factor(const pcs_attn_params& p, float l, long long t, int h, bool live) {
-  float f = l > 0.f ? 1.f / l : 0.f;
-  if (p.out_scale != 0.f) f *= p.out_scale;
-  if (p.head_gate && live) f *= sigmoidf_(ldf(static_cast<const __nv_bfloat16*>(p.head_gate) + t * p.head_gate_stride + h));
-  return f;
-}
+// (a call: in line, it made a walk of 6144 keys 1 % slower; the 32-bit kernel is 1.5 % slower with a call)
+__device__ __noinline__ void row_again(const pcs_attn_params& p, int b, int h, int t, int pos, int c0, int n) { attn_row_again<__nv_bfloat16>(p, b, h, t, pos, c0, n); }
 
 template <int DP, int VP, bool BIAS, bool CAP>
 __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                                                               const __grid_constant__ CUtensorMap map_v, const pcs_attn_params p, const int ends,
+                                                               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ pcs_attn_params p, const int ends,
                                                                const int splits) {
   using C = Cfg<DP, VP>;
   constexpr int ST = C::kStages;
@@ -157,6 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
   auto tile_of = [&](int it) { return it0 + it < nf ? it0 + it : lo + it0 + it - nf; };
   float m = -INFINITY, l = 0.f;  // (softmax threads) the row's running maximum and sum
   int j = 0;                     // and its tiles so far
+  bool again = false;            // its result is not finite
 
   if (warp == 8 && lane == 0) {
     tma_prefetch_desc(&map_q);
@@ -350,7 +345,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
         const bool need_mask = k0 + BN > end_key || (lo_key > k0 && k0 + BN > keep);
         if (CAP) {  // cap tanh(s scale / cap) as 1 - 2 / (1 + e^(2x)), in the base-2 domain
           // Three uses of the exponential unit per score made a window of 1024 under a cap 96 us; four scores that share one reciprocal: 84 us.  e^(2x) is
-          // held below 2^30 (tanh is 1 there), so the product of four stays in range.
+          // held below 2^30 (tanh is 1 there), so the product of four stays in range.  (A hidden score that is no number spoils its three neighbours: such a
+          // row's sum is no number either, and the row is formed again at the end.)
 #pragma unroll
           for (int c = 0; c < BN; c += 4) {
             float d[4];
@@ -434,8 +430,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
       __syncwarp();
       tc_fence_after();
       if (splits == 1) {  // the result: O / l, times the constant and the head's gate
-        const float inv = out_factor(p, l, off + r.q0 + row, h, live);
-        __nv_bfloat16* out = out_row(p, off + r.q0 + row, h);
+        const int t = off + r.q0 + row;
+        const float inv = live ? (l > 0.f ? 1.f / l : 0.f) * out_factor<__nv_bfloat16>(p, t, h) : 0.f;
+        __nv_bfloat16* out = out_row<__nv_bfloat16>(p, t, h);
+        float zero[4] = {0.f, 0.f, 0.f, 0.f};   // stay 0 over finite numbers
 #pragma unroll
         for (int f = 0; f < VP / 32; ++f) {
           uint32_t o[32];
@@ -446,11 +444,16 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
             for (int v = 0; v < 4; ++v) {
               uint32_t w[4];
 #pragma unroll
-              for (int c = 0; c < 4; ++c) w[c] = pack_bf16(__uint_as_float(o[v * 8 + 2 * c]) * inv, __uint_as_float(o[v * 8 + 2 * c + 1]) * inv);
+              for (int c = 0; c < 4; ++c) {
+                const float x = __uint_as_float(o[v * 8 + 2 * c]) * inv, y = __uint_as_float(o[v * 8 + 2 * c + 1]) * inv;
+                zero[c] = fmaf(x, 0.f, fmaf(y, 0.f, zero[c]));
+                w[c] = pack_bf16(x, y);
+              }
               if (f * 32 + v * 8 < p.vdim) *reinterpret_cast<uint4*>(out + f * 32 + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
             }
           }
         }
+        again = (zero[0] + zero[1]) + (zero[2] + zero[3]) != 0.f;
       }
     }
   }
@@ -502,9 +505,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
         lt = fmaf(ls[q], ms[q], lt);
       }
       const bool live = row < r.rows;
-      const long long t = off + r.q0 + row;
-      const float inv = out_factor(p, lt, t, h, live);
-      __nv_bfloat16* out = out_row(p, t, h) + rank * vc;
+      const int t = off + r.q0 + row;
+      const float inv = live ? (lt > 0.f ? 1.f / lt : 0.f) * out_factor<__nv_bfloat16>(p, t, h) : 0.f;
+      __nv_bfloat16* out = out_row<__nv_bfloat16>(p, t, h) + rank * vc;
+      float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       for (int c0 = 0; c0 < vc; c0 += 8) {
         float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -514,14 +518,26 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
 #pragma unroll
             for (int c = 0; c < 8; ++c) a[c] = fmaf(src[c * BM], ms[q], a[c]);
           }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          a[c] *= inv;
+          zero[c] = fmaf(a[c], 0.f, zero[c]);
+        }
         if (live && rank * vc + c0 < p.vdim)
-          *reinterpret_cast<uint4*>(out + c0) = make_uint4(pack_bf16(a[0] * inv, a[1] * inv), pack_bf16(a[2] * inv, a[3] * inv),
-                                                           pack_bf16(a[4] * inv, a[5] * inv), pack_bf16(a[6] * inv, a[7] * inv));
+          *reinterpret_cast<uint4*>(out + c0) = make_uint4(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]), pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
       }
+      again = live && ((zero[0] + zero[1]) + (zero[2] + zero[3])) + ((zero[4] + zero[5]) + (zero[6] + zero[7])) != 0.f;
     }
   }
   tc_fence_before();
-  __syncthreads();
+  __syncthreads();   // TMEM has been read
+  if (warp < 8) {   // rows whose result is not finite: from the keys they see alone (this block's columns of them)
+    const int q0 = (warp >> 2) ? rg[1].q0 : rg[0].q0, cols = VP / splits, c0 = splits > 1 ? rank * cols : 0;
+    for (uint32_t w = __ballot_sync(0xffffffffu, again && c0 < p.vdim); w; w &= w - 1) {
+      const int row = q0 + (warp & 3) * 32 + __ffs(w) - 1;
+      row_again(p, b, h, off + row, pos0 + row, c0, min(cols, p.vdim - c0));
+    }
+  }
   if (warp == 9) {
     tc_fence_after();
     tmem_free<512>(tmem_base);

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 OPTS = {"plain": {}, "window": dict(softcap=20.0, window=70, keep_first=5), "chunk": dict(chunk=96), "cap": dict(softcap=30.0)}
 
 
-@pytest.mark.parametrize("dt", [F32])
+@pytest.mark.parametrize("dt", [BF16, F32])
 @pytest.mark.parametrize("name", OPTS)
 @pytest.mark.parametrize("bad", [(201, "k", math.nan), (202, "v", math.nan), (127, "v", math.inf), (200, "kv", math.nan)])
 @pytest.mark.parametrize("H,stored,new", [(1, 0, 300), (2, 100, 200), (1, 0, 2049), (40, 0, 600)])   # (clusters of several sizes; a launch of many tiles)
