@@ -349,15 +349,16 @@ __global__ void __launch_bounds__(kOutThreads) gla_out_kernel(const pcs_gla_para
 
 // ---- the chunkwise form (prompts) -------------------------------------------------------------------------------------
 // One block per (chunk, head).  q, k and the running sums of the log decays of the chunk sit in shared memory as 32-bit rows
-// of dim + 1 numbers (a row per token: threads that walk the tokens at a fixed channel touch different banks).  The scores
+// of DP numbers: dim + 1 where the pairs' loop reads single numbers (a row per token: threads that walk the tokens at a fixed channel touch different
+// banks), dim + 4 where it reads 16-byte pieces (eight neighbouring rows in different banks).  The scores
 // inside the chunk are formed pair by pair with the exact factor exp(B_i[d] - B_s[d]) <= 1 per channel, so no decay, however
 // strong, overflows a factor; everything that crosses chunks is left to matrix products on exp(B_i) and exp(B_e - B_i) <= 1.
 constexpr int kPrepThreads = 1024;
 template <typename T>
-__global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep_kernel(const pcs_gla_chunk_params p) {
+__global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep_kernel(const pcs_gla_chunk_params p, const int DP) {
   extern __shared__ float sm[];
-  // rows of whole 16-byte pieces where the channels allow it (a padding piece keeps eight neighbouring rows in different banks)
-  const int D = p.dim, V = p.vdim, H = p.heads, C = p.chunk, DP = D % 4 == 0 ? D + 4 : D + 1;
+  const int D = p.dim, V = p.vdim, H = p.heads, C = p.chunk;
+  const bool rows4 = DP == D + 4;   // rows of whole 16-byte pieces
   float* qs = sm;              // [C][DP]
   float* ks = qs + C * DP;     // [C][DP]
   float* Bs = ks + C * DP;     // [C][DP]
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep_kernel(const pcs_
   // rows in pieces of four channels, a warp per row, where the sizes allow it (bfloat16 runs)
   const int warp = tid >> 5, lane = tid & 31;
   auto al = [](const void* q, int b) { return (reinterpret_cast<uintptr_t>(q) & (b - 1)) == 0; };
-  const bool quads = sizeof(T) == 2 && D % 4 == 0 && V % 4 == 0 && p.q_off % 4 == 0 && p.k_off % 4 == 0 && p.v_off % 4 == 0 && p.row_stride % 4 == 0 && al(p.proj, 8) &&
+  const bool quads = sizeof(T) == 2 && rows4 && V % 4 == 0 && p.q_off % 4 == 0 && p.k_off % 4 == 0 && p.v_off % 4 == 0 && p.row_stride % 4 == 0 && al(p.proj, 8) &&
                      al(p.ld, 16) && al(p.qd, 16) && al(p.kd, 16) && al(p.vf, 16);
   auto ld4 = [](const T* x) {
     const uint2 u = *reinterpret_cast<const uint2*>(x);
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep_kernel(const pcs_
     const float* bs = Bs + s_ * DP;
     float a0 = 0.f, a1 = 0.f;
     int d = 0;
-    if (kFast && D % 4 == 0) {   // four channels per read: the loop is bound by shared memory (with the loads in pieces and the pairs in whole rounds: 86 -> 56 us at 136 chunks of 256 channels)
+    if (kFast && rows4) {   // four channels per read: the loop is bound by shared memory (with the loads in pieces and the pairs in whole rounds: 86 -> 56 us at 136 chunks of 256 channels)
 #pragma unroll 2
       for (; d < D; d += 4) {
         const float4 q4 = *reinterpret_cast<const float4*>(qi + d), k4 = *reinterpret_cast<const float4*>(kk + d);
@@ -656,12 +657,14 @@ PCS_API int pcs_gla_chunk_prep(const pcs_gla_chunk_params* p, void* stream) {
   if (p->n_chunks == 0) return PCS_OK;
   PCS_REQUIRE(p->proj && p->ld && p->chunk_first && p->chunk_len && p->qd && p->kd && p->g && p->vf && p->a, "pcs_gla_chunk_prep: null tensor");
   PCS_REQUIRE(p->heads > 0 && p->heads <= 65535 && p->dim > 0 && p->vdim > 0 && p->chunk > 0, "pcs_gla_chunk_prep: bad sizes");
-  const size_t smem = static_cast<size_t>(3) * p->chunk * (p->dim % 4 == 0 ? p->dim + 4 : p->dim + 1) * sizeof(float);
+  // (32-bit runs read single numbers: rows of dim + 4 would put four neighbouring rows into one bank)
+  const int row = p->dtype == PCS_BF16 && p->dim % 4 == 0 ? p->dim + 4 : p->dim + 1;
+  const size_t smem = static_cast<size_t>(3) * p->chunk * row * sizeof(float);
   PCS_REQUIRE(smem <= 220 * 1024, "pcs_gla_chunk_prep: a chunk of %d tokens x %d channels exceeds shared memory", p->chunk, p->dim);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (smem > 48 * 1024)
     PCS_DISPATCH(p->dtype, PCS_CHECK_CUDA(cudaFuncSetAttribute(pcs::gla_chunk_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
-  PCS_DISPATCH(p->dtype, pcs::gla_chunk_prep_kernel<T><<<dim3(p->n_chunks, p->heads), pcs::kPrepThreads, smem, st>>>(*p));
+  PCS_DISPATCH(p->dtype, pcs::gla_chunk_prep_kernel<T><<<dim3(p->n_chunks, p->heads), pcs::kPrepThreads, smem, st>>>(*p, row));
   PCS_CHECK_CUDA(cudaGetLastError());
   pcs::count_launch();
   return PCS_OK;
