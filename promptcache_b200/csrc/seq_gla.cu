@@ -658,12 +658,14 @@ PCS_API int pcs_gla_chunk_prep(const pcs_gla_chunk_params* p, void* stream) {
   PCS_REQUIRE(p->proj && p->ld && p->chunk_first && p->chunk_len && p->qd && p->kd && p->g && p->vf && p->a, "pcs_gla_chunk_prep: null tensor");
   PCS_REQUIRE(p->heads > 0 && p->heads <= 65535 && p->dim > 0 && p->vdim > 0 && p->chunk > 0, "pcs_gla_chunk_prep: bad sizes");
   // (32-bit runs read single numbers: rows of dim + 4 would put four neighbouring rows into one bank)
-  const int row = p->dtype == PCS_BF16 && p->dim % 4 == 0 ? p->dim + 4 : p->dim + 1;
-  const size_t smem = static_cast<size_t>(3) * p->chunk * row * sizeof(float);
-  PCS_REQUIRE(smem <= 220 * 1024, "pcs_gla_chunk_prep: a chunk of %d tokens x %d channels exceeds shared memory", p->chunk, p->dim);
+  constexpr size_t kLimit = 220 * 1024;
+  auto bytes = [&](int row) { return static_cast<size_t>(3) * p->chunk * row * sizeof(float); };
+  const int row = p->dtype == PCS_BF16 && p->dim % 4 == 0 && bytes(p->dim + 4) <= kLimit ? p->dim + 4 : p->dim + 1;
+  const size_t smem = bytes(row);
+  PCS_REQUIRE(smem <= kLimit, "pcs_gla_chunk_prep: a chunk of %d tokens x %d channels exceeds shared memory", p->chunk, p->dim);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (smem > 48 * 1024)
-    PCS_DISPATCH(p->dtype, PCS_CHECK_CUDA(cudaFuncSetAttribute(pcs::gla_chunk_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
+    PCS_DISPATCH(p->dtype, PCS_CHECK_CUDA(cudaFuncSetAttribute(pcs::gla_chunk_prep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLimit))));
   PCS_DISPATCH(p->dtype, pcs::gla_chunk_prep_kernel<T><<<dim3(p->n_chunks, p->heads), pcs::kPrepThreads, smem, st>>>(*p, row));
   PCS_CHECK_CUDA(cudaGetLastError());
   pcs::count_launch();

@@ -6,7 +6,7 @@ pytestmark = pytest.mark.gpu
 DEV, F64 = torch.device("cuda:0"), torch.float64
 
 
-@pytest.mark.parametrize("dt", [torch.float32])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("D", [260, 288, 289, 291, 292, 293, 296])
 def test_wide_heads(dt, D):
     from promptcache_b200 import _native_seq as nsq
