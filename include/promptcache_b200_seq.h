@@ -66,7 +66,7 @@
 extern "C" {
 #endif
 
-#define PCS_ABI_VERSION 7
+#define PCS_ABI_VERSION 8
 #define PCS_BF16 0
 #define PCS_F32 1
 
@@ -724,6 +724,8 @@ typedef struct pcs_delta_chunk_params {
   int64_t dec_stride;
   const float* dt_bias;        /* [heads] */
   const float* rate;           /* [heads] */
+  int32_t parts, reserved;     /* pcs_delta_chunk_out: bfloat16 parts in which qd, a, s and u enter: 0 or 2 (16 of their 24 bits), or 3 (all of them; u then holds
+                                  bfloat16 numbers) */
 } pcs_delta_chunk_params;
 int pcs_delta_chunk_prep(const pcs_delta_chunk_params* p, void* stream);
 int pcs_delta_chunk_scan(const pcs_delta_chunk_params* p, void* stream);

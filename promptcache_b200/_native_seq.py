@@ -193,7 +193,8 @@ class pcs_delta_chunk_params(C.Structure):
                 ("dim", C.c_int32), ("vdim", C.c_int32), ("chunk_first", C.c_void_p), ("chunk_len", C.c_void_p), ("n_chunks", C.c_int32), ("n_tokens", C.c_int32),
                 ("dtype", C.c_int32), ("n_seqs", C.c_int32), ("qd", C.c_void_p), ("kd", C.c_void_p), ("w", C.c_void_p), ("g", C.c_void_p), ("u", C.c_void_p),
                 ("a", C.c_void_p), ("s", C.c_void_p), ("s_pool", C.c_void_p), ("seq_slot", C.c_void_p), ("seq_pos0", C.c_void_p), ("seq_chunk0", C.c_void_p),
-                ("seq_chunks", C.c_void_p), ("dec_a", C.c_void_p), ("dec_stride", C.c_int64), ("dt_bias", C.c_void_p), ("rate", C.c_void_p)]
+                ("seq_chunks", C.c_void_p), ("dec_a", C.c_void_p), ("dec_stride", C.c_int64), ("dt_bias", C.c_void_p), ("rate", C.c_void_p),
+                ("parts", C.c_int32), ("reserved", C.c_int32)]
 
 
 class pcs_headnorm_params(C.Structure):
@@ -1008,10 +1009,11 @@ def gla_scan_chunked(proj: torch.Tensor, offs, ld: torch.Tensor, norm_w: torch.T
     p.seq_slot, p.seq_pos0, p.seq_chunk0, p.seq_chunks = batch.seq_slot.data_ptr(), batch.seq_pos0.data_ptr(), plan["seq0"].data_ptr(), plan["seqn"].data_ptr()
     _check(load().pcs_gla_chunk_scan(C.byref(p), _stream()), "pcs_gla_chunk_scan")   # u now holds the state every chunk starts from
     if tensor_cores and V <= DELTA_OUT_MAX_VDIM:
-        # the read-out of chunks that the delta rule has too: o = qd S + a v with the head's norm and gate, in one launch
+        # the read-out of chunks that the delta rule has too: o = qd S + a v with the head's norm and gate, in one launch; the 32-bit operands enter with
+        # all their bits
         r, n = pcs_delta_chunk_params(), pcs_headnorm_params()
         r.heads, r.kv_heads, r.dim, r.vdim, r.n_chunks, r.n_tokens, r.dtype, r.n_seqs = H, H, D, V, nc, batch.n_tokens, dtype_code(dt), batch.n_seqs
-        r.chunk_first, r.chunk_len, r.qd, r.u, r.a, r.s = p.chunk_first, p.chunk_len, qd.data_ptr(), vf.data_ptr(), a.data_ptr(), u.data_ptr()
+        r.chunk_first, r.chunk_len, r.qd, r.u, r.a, r.s, r.parts = p.chunk_first, p.chunk_len, qd.data_ptr(), vf.data_ptr(), a.data_ptr(), u.data_ptr(), 3
         n.w, n.g, n.g_stride, n.out, n.out_stride = norm_w.data_ptr(), proj.data_ptr() + offs[3] * proj.element_size(), proj.stride(0), out.data_ptr(), out.stride(0)
         n.n_tokens, n.heads, n.vdim, n.eps, n.out_scale, n.dtype, n.silu = batch.n_tokens, H, V, float(eps), 1.0, dtype_code(dt), 1
         _check(load().pcs_delta_chunk_out(C.byref(r), C.byref(n), _stream()), "pcs_delta_chunk_out")

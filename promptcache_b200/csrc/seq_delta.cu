@@ -1541,28 +1541,42 @@ static int launch_delta_chunk_scan(const pcs_delta_chunk_params& p, size_t smem,
 // Block = (chunk, head), a warp = 32 value columns: o = qd S + a u over dim + 64 terms, then the head's norm and gate on the accumulators, and the
 // result's rows.  The result leaves in bfloat16, so the operands enter as hi + lo bfloat16 pairs (hi hi + hi lo + lo hi in 32-bit accumulators,
 // about 2^-16 of a product); the state itself stays as it is.  [qd | a] is staged in shared memory as such pairs, S and u are read once, a step ahead.
+// Three parts (gated linear attention, whose read-out was a 32-bit product): all 24 bits of qd, a and S (u holds bfloat16 numbers there and is its own first
+// part), six products per step of sixteen terms, the smallest first, and the steps' sums join in rounded additions (the tensor core's running sum cuts
+// bits off).  That takes registers for half of the tokens only: a block of 32 tokens, S is read by two blocks.
 constexpr int kDoMaxWarps = 16;
 
+template <int PARTS>
 __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const pcs_delta_chunk_params p, const pcs_headnorm_params o) {
   extern __shared__ __align__(16) float sm[];
+  constexpr int MT = PARTS == 2 ? 4 : 2, R = 16 * MT;   // tiles of 16 tokens, tokens of a block
   const int D = p.dim, V = p.vdim, H = p.heads, D16 = (D + 15) & ~15, LD = D16 + kC + 8;   // (rows an odd number of 16-byte pieces apart)
-  __nv_bfloat16* Ah = reinterpret_cast<__nv_bfloat16*>(sm);   // [64][LD]
-  __nv_bfloat16* Al = Ah + kC * LD;                           // [64][LD]
-  float* red = reinterpret_cast<float*>(Al + kC * LD);        // [warps][64], then [64]
+  __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(sm);          // [parts][R][LD], hi first
+  float* red = reinterpret_cast<float*>(As + PARTS * R * LD);        // [warps][R], then [R]
   const int cn = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const long long base = static_cast<long long>(cn) * H + head;
-  const int first = p.chunk_first[cn], n = p.chunk_len[cn];
-  const float* qd = p.qd + base * kC * D;
-  const float* ag = p.a + base * kC * kC;
+  const int row0 = PARTS == 2 ? 0 : blockIdx.z * R, first = p.chunk_first[cn] + row0, n = p.chunk_len[cn] - row0;
+  if (n <= 0) return;
+  const float* qd = p.qd + (base * kC + row0) * D;
+  const float* ag = p.a + (base * kC + row0) * kC;
+  // a pair of numbers as PARTS packed pairs
+  auto parts = [](float x0, float x1, uint32_t (&o)[PARTS]) {
+#pragma unroll
+    for (int i = 0; i < PARTS; ++i) {
+      o[i] = pack_bf16(x0, x1);
+      x0 -= __uint_as_float(o[i] << 16);
+      x1 -= __uint_as_float(o[i] & 0xffff0000u);
+    }
+  };
   auto put = [&](int i, int c, const float (&x)[4]) {
-    uint2 hi, lo;
-    hi.x = split_pair(x[0], x[1], lo.x);
-    hi.y = split_pair(x[2], x[3], lo.y);
-    *reinterpret_cast<uint2*>(Ah + i * LD + c) = hi;
-    *reinterpret_cast<uint2*>(Al + i * LD + c) = lo;
+    uint32_t a[PARTS], b[PARTS];
+    parts(x[0], x[1], a);
+    parts(x[2], x[3], b);
+#pragma unroll
+    for (int y = 0; y < PARTS; ++y) *reinterpret_cast<uint2*>(As + (y * R + i) * LD + c) = make_uint2(a[y], b[y]);
   };
   // (place x of the warp's tile q is its column 4 x + q: a lane's four values of a row are neighbours)
-  const int c0 = warp * 32 + 4 * g, KD = D16 / 16, KT = KD + kC / 16;
+  const int c0 = warp * 32 + 4 * g, KD = D16 / 16, KT = KD + (PARTS == 2 ? kC : row0 + R) / 16;   // (`a` is zero behind the block's tokens)
   const float* sg = p.s + base * D * V;
   const float* ug = p.u + base * kC * V;
   const bool quads = V % 4 == 0;
@@ -1590,13 +1604,13 @@ __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const
       b[3][h] = x.w;
     }
   };
-  float acc[4][4][4], nx[4][4];
+  float acc[4][MT][4], nx[4][4];
 #pragma unroll
   for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int m = 0; m < 4; ++m) acc[q][m][0] = acc[q][m][1] = acc[q][m][2] = acc[q][m][3] = 0.f;
+    for (int m = 0; m < MT; ++m) acc[q][m][0] = acc[q][m][1] = acc[q][m][2] = acc[q][m][3] = 0.f;
   load(0, nx);
-  const int per = D16 / 4, pieces = kC * (per + kC / 4);   // a row's pieces of qd, then of a
+  const int per = D16 / 4, pieces = R * (per + kC / 4);   // a row's pieces of qd, then of a
   for (int e0 = tid; e0 < pieces; e0 += 4 * nthr) {        // (four requests before the first is used)
     float x[4][4];
 #pragma unroll
@@ -1626,33 +1640,55 @@ __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const
     }
   }
   __syncthreads();
-  const uint32_t a_hi = static_cast<uint32_t>(__cvta_generic_to_shared(Ah)) + ((lane & 15) * LD + (lane >> 4) * 8) * 2, a_lo = a_hi + kC * LD * 2;
+  const uint32_t a_base = static_cast<uint32_t>(__cvta_generic_to_shared(As)) + ((lane & 15) * LD + (lane >> 4) * 8) * 2;
 #pragma unroll 1
   for (int kt = 0; kt < KT; ++kt) {
-    uint32_t bh[4][2], bl[4][2];
+    uint32_t b[4][2][PARTS];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      bh[q][0] = split_pair(nx[q][0], nx[q][1], bl[q][0]);
-      bh[q][1] = split_pair(nx[q][2], nx[q][3], bl[q][1]);
+      parts(nx[q][0], nx[q][1], b[q][0]);
+      parts(nx[q][2], nx[q][3], b[q][1]);
     }
     load(kt + 1, nx);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      if (m < kt - KD) continue;   // `a` is zero above the diagonal
-      uint32_t h0, h1, h2, h3, l0, l1, l2, l3;
-      ldsm_x4(a_hi + (m * 16 * LD + kt * 16) * 2, h0, h1, h2, h3);
-      ldsm_x4(a_lo + (m * 16 * LD + kt * 16) * 2, l0, l1, l2, l3);
+    for (int m = 0; m < MT; ++m) {
+      if (m + row0 / 16 < kt - KD) continue;   // `a` is zero above the diagonal
+      uint32_t x[PARTS][4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) mma_bf16(acc[q][m], h0, h1, h2, h3, bh[q][0], bh[q][1]);
+      for (int i = 0; i < PARTS; ++i) ldsm_x4(a_base + ((i * R + m * 16) * LD + kt * 16) * 2, x[i][0], x[i][1], x[i][2], x[i][3]);
+      if constexpr (PARTS == 2) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) mma_bf16(acc[q][m], h0, h1, h2, h3, bl[q][0], bl[q][1]);
+        for (int q = 0; q < 4; ++q) mma_bf16(acc[q][m], x[0][0], x[0][1], x[0][2], x[0][3], b[q][0][0], b[q][1][0]);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) mma_bf16(acc[q][m], l0, l1, l2, l3, bh[q][0], bh[q][1]);
+        for (int q = 0; q < 4; ++q) mma_bf16(acc[q][m], x[0][0], x[0][1], x[0][2], x[0][3], b[q][0][1], b[q][1][1]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mma_bf16(acc[q][m], x[1][0], x[1][1], x[1][2], x[1][3], b[q][0][0], b[q][1][0]);
+      } else {
+        float step[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) step[q][0] = step[q][1] = step[q][2] = step[q][3] = 0.f;
+        auto product = [&](int i, int j) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) mma_bf16(step[q], x[i][0], x[i][1], x[i][2], x[i][3], b[q][0][j], b[q][1][j]);
+        };
+        product(2, 0);
+        if (kt < KD) {   // (u has no further parts)
+          product(1, 1);
+          product(0, 2);
+          product(0, 1);
+        }
+        product(1, 0);
+        product(0, 0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[q][m][e] += step[q][e];
+      }
     }
   }
   // the head's mean square per token: a row's columns are spread over 4 lanes and all warps
 #pragma unroll
-  for (int m = 0; m < 4; ++m)
+  for (int m = 0; m < MT; ++m)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       float ss = 0.f;
@@ -1660,16 +1696,16 @@ __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const
       for (int q = 0; q < 4; ++q) ss = fmaf(acc[q][m][2 * h], acc[q][m][2 * h], fmaf(acc[q][m][2 * h + 1], acc[q][m][2 * h + 1], ss));
       ss += __shfl_xor_sync(0xffffffffu, ss, 1);
       ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-      if (t == 0) red[warp * kC + 16 * m + g + 8 * h] = ss;
+      if (t == 0) red[warp * R + 16 * m + g + 8 * h] = ss;
     }
   __syncthreads();
   float inv = 0.f;
-  for (int i = tid; i < kC; i += nthr) {   // (at least two warps)
-    for (int w = 0; w < nthr / 32; ++w) inv += red[w * kC + i];
+  for (int i = tid; i < R; i += nthr) {   // (at least two warps)
+    for (int w = 0; w < nthr / 32; ++w) inv += red[w * R + i];
     inv = o.out_scale / sqrtf(inv / static_cast<float>(V) + o.eps);
   }
   __syncthreads();
-  if (tid < kC) red[tid] = inv;
+  if (tid < R) red[tid] = inv;
   __syncthreads();
   const __nv_bfloat16* gate = static_cast<const __nv_bfloat16*>(o.g) + static_cast<long long>(first) * o.g_stride + head * V;
   const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(o.w);
@@ -1683,20 +1719,20 @@ __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const
   };
   auto gated = [&](float x, float f, float wv, float gv) { return x * f * wv * sigmoidf_(gv) * (o.silu ? gv : 1.f); };
 #pragma unroll
-  for (int e = 0; e < 2; ++e) {   // this lane's columns c .. c + 3 (places 2t + e), eight tokens: all gates are requested before the first result leaves
+  for (int e = 0; e < 2; ++e) {   // this lane's columns c .. c + 3 (places 2t + e), all its tokens: all gates are requested before the first result leaves
     const int c = warp * 32 + 4 * (2 * t + e);
     if (c >= V) continue;
     if (vec) {
-      uint2 gv[8];
+      uint2 gv[2 * MT];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
+      for (int k = 0; k < 2 * MT; ++k) {
         const int i = 16 * (k >> 1) + g + 8 * (k & 1);
         gv[k] = i < n ? *reinterpret_cast<const uint2*>(gate + static_cast<long long>(i) * o.g_stride + c) : make_uint2(0u, 0u);
       }
       float wv[4];
       unpack(*reinterpret_cast<const uint2*>(w + c), wv);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
+      for (int k = 0; k < 2 * MT; ++k) {
         const int m = k >> 1, x = 2 * (k & 1) + e, i = 16 * m + g + 8 * (k & 1);
         if (i >= n) continue;
         const float f = red[i];
@@ -1709,7 +1745,7 @@ __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const
       }
     } else {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
+      for (int k = 0; k < 2 * MT; ++k) {
         const int m = k >> 1, x = 2 * (k & 1) + e, i = 16 * m + g + 8 * (k & 1);
         if (i >= n) continue;
         const float f = red[i];
@@ -1899,10 +1935,15 @@ PCS_API int pcs_delta_chunk_out(const pcs_delta_chunk_params* p, const pcs_headn
   PCS_REQUIRE(p->dtype == PCS_BF16 && p->heads > 0 && p->heads <= 65535 && p->dim > 0 && p->dim <= 256 && p->vdim > 0 && p->vdim <= 32 * pcs::kDoMaxWarps,
               "pcs_delta_chunk_out: serves bfloat16, dim up to 256 and vdim up to %d", 32 * pcs::kDoMaxWarps);
   PCS_REQUIRE(((reinterpret_cast<uintptr_t>(p->qd) | reinterpret_cast<uintptr_t>(p->a)) & 15) == 0, "pcs_delta_chunk_out: qd and a must be 16-byte aligned");
+  PCS_REQUIRE(p->parts == 0 || p->parts == 2 || p->parts == 3, "pcs_delta_chunk_out: operands enter in two parts or in three");
   const int warps = (p->vdim + 31) / 32 < 2 ? 2 : (p->vdim + 31) / 32, D16 = (p->dim + 15) & ~15;
-  const size_t smem = static_cast<size_t>(2) * pcs::kC * (D16 + pcs::kC + 8) * sizeof(__nv_bfloat16) + static_cast<size_t>(warps) * pcs::kC * sizeof(float);
-  PCS_CHECK_CUDA(cudaFuncSetAttribute(pcs::delta_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  pcs::delta_chunk_out_kernel<<<dim3(p->n_chunks, p->heads), warps * 32, smem, static_cast<cudaStream_t>(stream)>>>(*p, *o);
+  auto launch = [&](auto kernel, int parts, int tokens) -> int {
+    const size_t smem = static_cast<size_t>(parts) * tokens * (D16 + pcs::kC + 8) * sizeof(__nv_bfloat16) + static_cast<size_t>(warps) * tokens * sizeof(float);
+    PCS_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    kernel<<<dim3(p->n_chunks, p->heads, pcs::kC / tokens), warps * 32, smem, static_cast<cudaStream_t>(stream)>>>(*p, *o);
+    return PCS_OK;
+  };
+  if (int rc = p->parts == 3 ? launch(pcs::delta_chunk_out_kernel<3>, 3, 32) : launch(pcs::delta_chunk_out_kernel<2>, 2, 64)) return rc;
   PCS_CHECK_CUDA(cudaGetLastError());
   pcs::count_launch();
   return PCS_OK;
