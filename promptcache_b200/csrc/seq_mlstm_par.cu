@@ -25,9 +25,6 @@ constexpr int OT = 512;     // and of `out`
 constexpr int US = 128;     // columns of a block of `sums`
 constexpr int UROW = US + 8, PROW = CL + 8;
 
-// sigmoid for a result that is rounded to 16 bits (a few units in the last of 24)
-__device__ __forceinline__ float gate_of(float z) { return __fdividef(1.f, 1.f + ex2(-1.4426950408889634f * z)); }
-
 // The scratch of one launch.  Chunk c of entry b is slot (seq_off[b] / 64) + b + c: slots of different entries never meet, and there are at most
 // n_tokens / 64 + n_seqs of them.
 struct Scratch {
@@ -512,7 +509,7 @@ __global__ void __launch_bounds__(OT, 1) mlstm_par_out_kernel(const pcs_mlstm_pa
       const int col = wc + j * 8 + qd * 2;
       if (col >= V) continue;
       const float2 w2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(nw + col)), g2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gate[i][j]));
-      *reinterpret_cast<uint32_t*>(o + col) = pack_bf16(acc[j][i * 2] * inv * w2.x * gate_of(g2.x), acc[j][i * 2 + 1] * inv * w2.y * gate_of(g2.y));
+      *reinterpret_cast<uint32_t*>(o + col) = pack_bf16(acc[j][i * 2] * inv * w2.x * sigmoidf_(g2.x), acc[j][i * 2 + 1] * inv * w2.y * sigmoidf_(g2.y));
     }
   }
 }
