@@ -25,18 +25,19 @@ constexpr int OT = 512;     // and of `out`
 constexpr int US = 128;     // columns of a block of `sums`
 constexpr int UROW = US + 8, PROW = CL + 8;
 
-// The scratch of one launch.  Chunk c of entry b is slot (seq_off[b] / 64) + b + c: slots of different entries never meet, and there are at most
-// n_tokens / 64 + n_seqs of them.
+// The scratch of one launch.  An entry's chunks are consecutive slots behind those of the entries before it (whatever the order of their rows); there are at
+// most n_tokens / 64 + n_seqs of them.
 struct Scratch {
   float *u, *n, *tok, *ce;   // [slot][head][dim * vdim], [slot][head][dim], [slot][head][5][64], [slot][head]
+  int* first;                // [entry] its first slot
   __host__ __device__ Scratch(float* base, long long slots, int H, int D, int V) {
     u = base;
     n = u + slots * H * D * V;
     tok = n + slots * H * D;
     ce = tok + slots * H * 5 * CL;
+    first = reinterpret_cast<int*>(ce + slots * H);
   }
 };
-__device__ __forceinline__ long long slot_of(const pcs_mlstm_params& p, int b, int c) { return (p.seq_off[b] >> 6) + b + c; }
 
 // a chunk's running sums b and a_s = i_s - b_s, two tokens per lane, and the running maximum of a
 struct ChunkGates {
@@ -72,6 +73,11 @@ __global__ void __launch_bounds__(512) mlstm_par_gates_kernel(const pcs_mlstm_pa
   const int len = p.seq_len[b], off = p.seq_off[b];
   if (len <= 0) return;
   const int nc = (len + CL - 1) / CL;
+  int at0 = 0;   // the chunks of the entries before this one
+  for (int i = lane; i < b; i += 32) at0 += (max(p.seq_len[i], 0) + CL - 1) / CL;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) at0 += __shfl_xor_sync(0xffffffffu, at0, o);
+  if (head == 0 && threadIdx.x == 0) sc.first[b] = at0;
   float *be = sm, *am = sm + nc;
   float* mg = p.m_pool + static_cast<long long>(p.seq_slot[b]) * H + head;
   for (int c = warp; c < nc; c += nw) {
@@ -99,7 +105,7 @@ __global__ void __launch_bounds__(512) mlstm_par_gates_kernel(const pcs_mlstm_pa
     if (lane == 0) before = -INFINITY;
     const float g0 = fmaxf(fmaxf(m_in, before), g.a0), g1 = fmaxf(g0, g.a1);
     const float ge = __shfl_sync(0xffffffffu, (e & 1) ? g1 : g0, e >> 1);
-    const long long at = slot_of(p, b, c) * H + head;
+    const long long at = static_cast<long long>(at0 + c) * H + head;
     float2* t = reinterpret_cast<float2*>(sc.tok + at * 5 * CL) + lane;
     t[0] = make_float2(g.a0, g.a1);
     t[CL / 2] = make_float2(g0, g1);
@@ -122,7 +128,7 @@ __global__ void __launch_bounds__(PT) mlstm_par_sums_kernel(const pcs_mlstm_para
   const int len = p.seq_len[b], i0 = c * CL;
   if (i0 >= len) return;
   const int n = min(CL, len - i0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = lane >> 2, qd = lane & 3;
-  const long long at = slot_of(p, b, c) * H + head;
+  const long long at = static_cast<long long>((b ? sc.first[b] : 0) + c) * H + head;
   const __nv_bfloat16* rows = static_cast<const __nv_bfloat16*>(p.proj) + static_cast<long long>(p.seq_off[b] + i0) * p.row_stride;
   const int pieces = D / 8;
   for (int e = tid; e < CL * pieces; e += PT) {
@@ -221,7 +227,7 @@ __global__ void __launch_bounds__(PT) mlstm_par_scan_kernel(const pcs_mlstm_para
   if (len <= 0) return;
   const int nc = (len + CL - 1) / CL;
   const bool fresh = p.seq_pos0[b] == 0;
-  const long long at0 = slot_of(p, b, 0) * H + head, pool = static_cast<long long>(p.seq_slot[b]) * H + head;
+  const long long at0 = static_cast<long long>(b ? sc.first[b] : 0) * H + head, pool = static_cast<long long>(p.seq_slot[b]) * H + head;
   if (blockIdx.x == gridDim.x - 1) {
     for (int d = threadIdx.x; d < D; d += PT) {
       float* ng = p.n_pool + pool * D + d;
@@ -306,7 +312,7 @@ __global__ void __launch_bounds__(OT, 1) mlstm_par_out_kernel(const pcs_mlstm_pa
   const int len = p.seq_len[b], i0 = c * CL;
   if (i0 >= len) return;
   const int n = min(CL, len - i0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = lane >> 2, qd = lane & 3;
-  const long long at = slot_of(p, b, c) * H + head, t0 = p.seq_off[b] + i0;
+  const long long at = static_cast<long long>((b ? sc.first[b] : 0) + c) * H + head, t0 = p.seq_off[b] + i0;
   const __nv_bfloat16* rows = static_cast<const __nv_bfloat16*>(p.proj) + t0 * p.row_stride;
   const int pieces = D / 8, ksteps = D / 16, vp8 = V / 8;
   const float* S = sc.u + at * D * V;
@@ -530,7 +536,7 @@ int launch_out(const pcs_mlstm_params& p, float* scratch, long long slots, dim3 
 
 long long mlstm_par_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim) {
   const long long slots = n_tokens / CL + n_seqs;
-  return slots * heads * (static_cast<long long>(dim) * vdim + dim + 5 * CL + 1);
+  return slots * heads * (static_cast<long long>(dim) * vdim + dim + 5 * CL + 1) + n_seqs;
 }
 
 // The caller has checked type, alignment and dim (a multiple of 16, at most 256).  Four launches against one walk and two: fewer than four chunks (eight where
