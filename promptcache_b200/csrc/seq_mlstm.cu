@@ -423,13 +423,11 @@ PCS_API int pcs_mlstm_scan(const pcs_mlstm_params* p, void* stream) {
   const int es = p->dtype == PCS_BF16 ? 2 : 4, per = 16 / es;
   const bool aligned = p->dim % per == 0 && p->vdim % per == 0 && p->q_off % per == 0 && p->k_off % per == 0 && p->v_off % per == 0 &&
                        p->row_stride % per == 0 && reinterpret_cast<uintptr_t>(p->proj) % 16 == 0;
-  if ((p->impl == 0 || p->impl == 3) && p->dtype == PCS_BF16 && aligned && p->dim % 16 == 0 && p->dim <= 256 && p->max_len >= pcs::kChunkMinLen) {
+  if (p->impl == 0 && p->dtype == PCS_BF16 && aligned && p->dim % 16 == 0 && p->dim <= 256 && p->max_len >= pcs::kChunkMinLen) {
     // prompts in bfloat16: 64 tokens at a time on the tensor cores
-    if (p->impl == 0) {
-      bool handled = false;
-      if (int rc = pcs::launch_mlstm_par(*p, st, &handled)) return rc;
-      if (handled) return PCS_OK;
-    }
+    bool handled = false;
+    if (int rc = pcs::launch_mlstm_par(*p, st, &handled)) return rc;
+    if (handled) return PCS_OK;
     if (int rc = pcs::launch_mlstm_chunk(*p, nm_new, st)) return rc;
   } else if (p->impl != 1 && p->dim <= 256 && aligned) {
     // register-resident state: warps per block halve until the launch has two blocks per SM (or 2 warps are left)
