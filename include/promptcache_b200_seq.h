@@ -219,10 +219,12 @@ typedef struct pcs_mlstm_params {
                                the per-head norm, and the new n / m of every entry until they are committed */
   int32_t n_tokens, reserved;
   float* chunk_scratch;     /* fp32 scratch of pcs_mlstm_scratch_floats() elements, 16-byte aligned, or NULL: with it the chunks of a prompt
-                               run side by side (vdim <= 512), without it one after the other */
+                               run side by side where that is the faster form, without it one after the other */
   int64_t chunk_floats;
 } pcs_mlstm_params;
 int64_t pcs_mlstm_scratch_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim);
+/* the scratch this call would make use of (its chunk_scratch and chunk_floats are not read): 0 where its chunks never run side by side */
+int64_t pcs_mlstm_scratch_wanted(const pcs_mlstm_params* p);
 int pcs_mlstm_scan(const pcs_mlstm_params* p, void* stream);
 
 /* out[t, :] = table[ids[t], :] * scale + pair[r, :], r = (prev_ids[t] * mul_prev + ids[t] * mul_cur) mod buckets, or r = buckets (the

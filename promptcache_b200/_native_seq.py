@@ -17,7 +17,7 @@ from ._native import NativeError, note_replayed_launches  # noqa: F401  (one err
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libpromptcache_b200_seq.so")
 PCS_BF16, PCS_F32 = 0, 1
-EXPORTS = ("pcs_version", "pcs_last_error", "pcs_launch_count", "pcs_attn_workspace_floats", "pcs_mlstm_scratch_floats", "pcs_attn_timeouts", "pcs_embed", "pcs_rmsnorm", "pcs_gate_norm_add", "pcs_xielu", "pcs_linear_rows",
+EXPORTS = ("pcs_version", "pcs_last_error", "pcs_launch_count", "pcs_attn_workspace_floats", "pcs_mlstm_scratch_floats", "pcs_mlstm_scratch_wanted", "pcs_attn_timeouts", "pcs_embed", "pcs_rmsnorm", "pcs_gate_norm_add", "pcs_xielu", "pcs_linear_rows",
            "pcs_qk_prep", "pcs_attn", "pcs_mlstm_gates", "pcs_mlstm_scan", "pcs_embed_bigram", "pcs_norm_conv", "pcs_rope_kv_prep", "pcs_moe_route",
            "pcs_moe_rows_up", "pcs_moe_rows_down", "pcs_moe_plan", "pcs_moe_gather", "pcs_moe_gemm", "pcs_moe_combine", "pcs_silu_mul", "pcs_glu_mul",
            "pcs_depth_mix", "pcs_latent_prep", "pcs_latent_q", "pcs_latent_gather", "pcs_latent_expand", "pcs_head_gate", "pcs_gla_decay", "pcs_gla_scan", "pcs_gla_chunk_prep", "pcs_gla_chunk_sums", "pcs_gla_chunk_scan", "pcs_gla_chunk_out",
@@ -235,6 +235,8 @@ def load() -> C.CDLL:
     lib.pcs_launch_count.restype = C.c_int64
     lib.pcs_mlstm_scratch_floats.argtypes = [C.c_int] * 5
     lib.pcs_mlstm_scratch_floats.restype = C.c_int64
+    lib.pcs_mlstm_scratch_wanted.argtypes = [C.POINTER(pcs_mlstm_params)]
+    lib.pcs_mlstm_scratch_wanted.restype = C.c_int64
     lib.pcs_embed.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_float, C.c_int, C.c_void_p]
     lib.pcs_rmsnorm.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_float, C.c_int, C.c_void_p]
     lib.pcs_gate_norm_add.argtypes = [C.POINTER(pcs_gna_params), C.c_void_p]
@@ -291,7 +293,7 @@ def load() -> C.CDLL:
     lib.pcs_delta_chunk_out.argtypes = [C.POINTER(pcs_delta_chunk_params), C.POINTER(pcs_headnorm_params), C.c_void_p]
     lib.pcs_side_boundary.argtypes = [C.POINTER(pcs_side_params), C.c_void_p]
     lib.pcs_side_gate.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
-    for name in EXPORTS[5:]:   # the first five: a version, a string and three 64-bit counts
+    for name in EXPORTS[6:]:   # the first six: a version, a string and four 64-bit counts
         getattr(lib, name).restype = C.c_int
     _lib = lib
     return lib
@@ -566,15 +568,17 @@ def mlstm_scan(proj: torch.Tensor, offs, ig: torch.Tensor, fg: torch.Tensor, nor
     p.seq_slot, p.seq_pos0, p.seq_len, p.seq_off = (batch.seq_slot.data_ptr(), batch.seq_pos0.data_ptr(), batch.seq_len.data_ptr(),
                                                     batch.seq_off.data_ptr())
     p.n_seqs, p.dtype, p.max_len, p.impl = batch.n_seqs, dtype_code(dt), batch.max_len, impl
-    # prompts in bfloat16: the chunks side by side, as long as their states take at most a gigabyte (beyond: one after the other)
-    if dt == torch.bfloat16 and impl == 0 and batch.max_len > 192:   # (fewer chunks never run side by side)
-        floats = int(load().pcs_mlstm_scratch_floats(batch.n_tokens, batch.n_seqs, p.heads, p.dim, p.vdim))
-        if floats <= MLSTM_SCRATCH_MAX:
-            scratch = torch.empty(floats, dtype=torch.float32, device=proj.device)
-            p.chunk_scratch, p.chunk_floats = scratch.data_ptr(), floats
     # scratch: the recurrence's raw result per token, and the new n / m per entry until the commit launch stores them
     o_raw = torch.empty(batch.n_tokens * p.heads * p.vdim + batch.n_seqs * p.heads * (p.dim + 1), dtype=torch.float32, device=proj.device)
     p.o_raw, p.n_tokens = o_raw.data_ptr(), batch.n_tokens
+    # prompts in bfloat16: the chunks side by side, as long as their states take at most a gigabyte and there is room (else: one after the other)
+    floats = int(load().pcs_mlstm_scratch_wanted(C.byref(p)))
+    if 0 < floats <= MLSTM_SCRATCH_MAX:
+        try:
+            scratch = torch.empty(floats, dtype=torch.float32, device=proj.device)
+            p.chunk_scratch, p.chunk_floats = scratch.data_ptr(), floats
+        except torch.OutOfMemoryError:
+            pass
     _check(load().pcs_mlstm_scan(C.byref(p), _stream()), "pcs_mlstm_scan")
 
 

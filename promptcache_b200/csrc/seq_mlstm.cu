@@ -397,8 +397,25 @@ __global__ void __launch_bounds__(256) mlstm_out_kernel(const pcs_mlstm_params p
 namespace pcs {
 int launch_mlstm_chunk(const pcs_mlstm_params& p, float* nm_new, cudaStream_t st);
 int launch_mlstm_par(const pcs_mlstm_params& p, cudaStream_t st, bool* handled);
+bool mlstm_par_serves(const pcs_mlstm_params& p);
+long long mlstm_par_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim);
 constexpr int kChunkMinLen = 24;  // shorter steps (decoding, tails of a prompt) go token by token
+// rows in 16-byte pieces
+static bool mlstm_aligned(const pcs_mlstm_params& p) {
+  const int per = p.dtype == PCS_BF16 ? 8 : 4;
+  return p.dim % per == 0 && p.vdim % per == 0 && p.q_off % per == 0 && p.k_off % per == 0 && p.v_off % per == 0 && p.row_stride % per == 0 &&
+         reinterpret_cast<uintptr_t>(p.proj) % 16 == 0;
+}
+// prompts in bfloat16 go 64 tokens at a time on the tensor cores
+static bool mlstm_in_chunks(const pcs_mlstm_params& p) {
+  return p.impl == 0 && p.dtype == PCS_BF16 && mlstm_aligned(p) && p.dim % 16 == 0 && p.dim <= 256 && p.max_len >= kChunkMinLen;
+}
 }  // namespace pcs
+
+PCS_API int64_t pcs_mlstm_scratch_wanted(const pcs_mlstm_params* p) {
+  if (!p || p->n_seqs <= 0 || p->n_tokens <= 0 || p->heads <= 0 || p->dim <= 0 || p->vdim <= 0 || !pcs::mlstm_in_chunks(*p) || !pcs::mlstm_par_serves(*p)) return 0;
+  return pcs::mlstm_par_floats(p->n_tokens, p->n_seqs, p->heads, p->dim, p->vdim);
+}
 
 PCS_API int pcs_mlstm_gates(const void* h, int64_t h_stride, const void* w_i, const void* w_f, const float* b_i, const float* b_f,
                             float* ig, float* fg, int n_tokens, int width, int heads, float cap, int dtype, void* stream) {
@@ -420,11 +437,9 @@ PCS_API int pcs_mlstm_scan(const pcs_mlstm_params* p, void* stream) {
   PCS_REQUIRE(p->heads > 0 && p->heads <= 65535 && p->dim > 0 && p->vdim > 0 && p->n_tokens > 0, "pcs_mlstm_scan: bad sizes");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   float* nm_new = p->o_raw + static_cast<long long>(p->n_tokens) * p->heads * p->vdim;  // behind the raw outputs
-  const int es = p->dtype == PCS_BF16 ? 2 : 4, per = 16 / es;
-  const bool aligned = p->dim % per == 0 && p->vdim % per == 0 && p->q_off % per == 0 && p->k_off % per == 0 && p->v_off % per == 0 &&
-                       p->row_stride % per == 0 && reinterpret_cast<uintptr_t>(p->proj) % 16 == 0;
-  if (p->impl == 0 && p->dtype == PCS_BF16 && aligned && p->dim % 16 == 0 && p->dim <= 256 && p->max_len >= pcs::kChunkMinLen) {
-    // prompts in bfloat16: 64 tokens at a time on the tensor cores
+  const int es = p->dtype == PCS_BF16 ? 2 : 4;
+  const bool aligned = pcs::mlstm_aligned(*p);
+  if (pcs::mlstm_in_chunks(*p)) {
     bool handled = false;
     if (int rc = pcs::launch_mlstm_par(*p, st, &handled)) return rc;
     if (handled) return PCS_OK;

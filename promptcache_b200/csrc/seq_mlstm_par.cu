@@ -542,16 +542,19 @@ long long mlstm_par_floats(int n_tokens, int n_seqs, int heads, int dim, int vdi
 // The caller has checked type, alignment and dim (a multiple of 16, at most 256).  Four launches against one walk and two: fewer than four chunks (eight where
 // a head has more than 256 columns, whose last kernel alone takes 40 us) stay with the serial form.  Serial / side by side, B200, us: 100 tokens of 2 heads 64 x 128
 // 22 / 32, 200 tokens of 2 heads 128 x 256 37 / 35, 128 tokens of a head 256 x 512 31 / 72, 700 tokens of 8 heads 256 x 512 218 / 107.
+bool mlstm_par_serves(const pcs_mlstm_params& p) {
+  auto al4 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 3) == 0; };
+  return p.vdim <= 512 && p.max_len > CL * (p.vdim > 256 ? 7 : 3) && p.g_off % 2 == 0 && al4(p.norm_w) && al4(p.out) &&
+         (reinterpret_cast<uintptr_t>(p.s_pool) & 15) == 0 && static_cast<long long>(p.n_seqs) * p.heads <= 65535 && (p.max_len + CL - 1) / CL <= 5000;
+}
+
 int launch_mlstm_par(const pcs_mlstm_params& p, cudaStream_t st, bool* handled) {
   *handled = false;
-  auto al4 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 3) == 0; };
-  if (!p.chunk_scratch || p.vdim > 512 || p.max_len <= CL * (p.vdim > 256 ? 7 : 3) || p.g_off % 2 != 0 || !al4(p.norm_w) || !al4(p.out) ||
-      (reinterpret_cast<uintptr_t>(p.s_pool) & 15) != 0 || (reinterpret_cast<uintptr_t>(p.chunk_scratch) & 15) != 0 ||
+  if (!p.chunk_scratch || !mlstm_par_serves(p) || (reinterpret_cast<uintptr_t>(p.chunk_scratch) & 15) != 0 ||
       p.chunk_floats < mlstm_par_floats(p.n_tokens, p.n_seqs, p.heads, p.dim, p.vdim))
     return PCS_OK;
   const long long slots = p.n_tokens / CL + p.n_seqs;
   const int chunks = (p.max_len + CL - 1) / CL;
-  if (static_cast<long long>(p.n_seqs) * p.heads > 65535 || chunks > 5000) return PCS_OK;
   *handled = true;
   float* s = p.chunk_scratch;
   mlstm_par_gates_kernel<<<dim3(p.n_seqs, p.heads), 512, 2 * chunks * sizeof(float), st>>>(p, s, slots);

@@ -30,3 +30,28 @@ def test_entries_in_any_order(lens, H, D, V):
     order = torch.randperm(len(lens), generator=torch.Generator().manual_seed(1)).flip(0).to(DEV)
     for a, b in zip(scan(lens, H, D, V), scan(lens, H, D, V, order)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("lens,V", [((300, 65), 128), ((500,), 512)])
+def test_no_room_for_the_chunks_side_by_side(monkeypatch, lens, V):
+    """Where their states find no memory, or more than the limit, the chunks run one after the other."""
+    from promptcache_b200 import _native_seq as nsq
+    empty, refused = torch.empty, []
+
+    def no_room(n, *a, **k):
+        if isinstance(n, int) and n == wanted:
+            refused.append(n)
+            raise torch.OutOfMemoryError("no room")
+        return empty(n, *a, **k)
+    wanted = int(nsq.load().pcs_mlstm_scratch_floats(sum(lens), len(lens), 1, 64, V))
+    ref = scan(lens, 1, 64, V)
+    monkeypatch.setattr(nsq, "MLSTM_SCRATCH_MAX", wanted - 1)
+    beyond = scan(lens, 1, 64, V)
+    monkeypatch.setattr(nsq, "MLSTM_SCRATCH_MAX", wanted)
+    short = scan(lens, 1, 64, V, before=lambda: monkeypatch.setattr(nsq.torch, "empty", no_room))
+    monkeypatch.setattr(nsq.torch, "empty", empty)
+    assert refused
+    for a, b, c in zip(ref, beyond, short):
+        assert torch.equal(b, c)
+        # two forms of one recurrence: sums of up to 64 products in another order, weights and states of 16 bits, results rounded to bfloat16
+        assert float((a.float() - b.float()).abs().max()) <= (2.0 ** -7 if a.dtype == BF16 else 2.0 ** -14) * float(a.float().abs().max())
