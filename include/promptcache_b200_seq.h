@@ -149,8 +149,8 @@ typedef struct pcs_attn_params {
   const int32_t* seq_len;
   const int32_t* seq_off;
   int32_t n_tokens, n_seqs, max_len, dtype;   /* max_len: host upper bound of the new tokens of one entry */
-  int32_t impl;             /* 0 = automatic, 1 = the plain kernel, 2 = the plain kernels with the split of the keys, 3 = automatic without the tcgen05
-                               prompt kernel */
+  int32_t impl;             /* 0 = automatic, 1 = the plain kernel, 2 = the plain kernels with the split of the keys, 3 = automatic, but in most blocks of the
+                               tcgen05 prompt kernel a warp gives up as if its wait had run out (tests of what follows) */
   int32_t max_keys;         /* host upper bound of the keys one token sees (sizes the split of the keys); 0: one split (prompts: cap) */
   float* workspace;         /* fp32 scratch of pcs_attn_workspace_floats() elements, or NULL (one split) */
   int64_t workspace_floats;
@@ -181,7 +181,8 @@ typedef struct pcs_attn_params {
 /* scratch the key split of pcs_attn needs for n_tokens tokens */
 int64_t pcs_attn_workspace_floats(int n_tokens, int n_heads, int vdim);
 int pcs_attn(const pcs_attn_params* p, void* stream);
-/* blocks of the tcgen05 prompt kernel that gave up a wait after two seconds, since the library was loaded (0 in a working system); synchronises */
+/* blocks of the tcgen05 prompt kernel that gave up a wait, since the library was loaded (0 in a working system); synchronises.  A wait tries some
+ * 2^22 times; the rows of a block that gave up are formed from their keys without the tensor cores, so results stay right. */
 int pcs_attn_timeouts(void);
 
 /* ig = cap * tanh((w_i h + b_i) / cap);  fg = logsigmoid(cap * tanh((w_f h + b_f) / cap))    (fp32 [n_tokens, heads]) */

@@ -507,14 +507,14 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
     }
     return PCS_OK;
   }
-  if (p->impl == 0 || p->impl == 3) {  // (impl 2: the plain kernels with the split of the keys, never a tensor-core kernel; 3: not the tcgen05 prompt kernel)
+  // (impl 2: the plain kernels with the split of the keys, never a tensor-core kernel; 3: as 0, with warps of the tcgen05 prompt kernel that give up)
+  const bool automatic = p->impl == 0 || p->impl == 3;
+  if (automatic) {
     bool handled = false;
-    if (p->impl == 0) {
-      if (int rc = pcs::launch_attn_tc5(*p, st, &handled)) return rc;
-      if (handled) return PCS_OK;
-      if (int rc = pcs::launch_attn_f32(*p, st, &handled)) return rc;
-      if (handled) return PCS_OK;
-    }
+    if (int rc = pcs::launch_attn_tc5(*p, st, &handled)) return rc;
+    if (handled) return PCS_OK;
+    if (int rc = pcs::launch_attn_f32(*p, st, &handled)) return rc;
+    if (handled) return PCS_OK;
     if (int rc = pcs::launch_attn_tc(*p, st, &handled)) return rc;
     if (handled) return PCS_OK;
     int latent_splits = 0;   // few tokens over rows that all heads share: the tensor-core kernel, then the merge of its partial results
@@ -532,7 +532,7 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
   PCS_REQUIRE(smem <= 48 * 1024, "pcs_attn: dim %d exceeds the shared-memory query row", p->dim);
   // few tokens over many keys (decoding): the keys are split so that the launch fills the GPU; each split has >= 128 keys
   const int piece = p->dtype == PCS_BF16 ? 8 : 4;
-  const bool decode = (p->impl == 0 || p->impl == 2) && p->workspace != nullptr && p->dim % piece == 0 && p->vdim % piece == 0 &&
+  const bool decode = (automatic || p->impl == 2) && p->workspace != nullptr && p->dim % piece == 0 && p->vdim % piece == 0 &&
                       p->vdim / piece <= pcs::kAttnThreads && p->v_row_stride % piece == 0;
   int splits = 1;
   if (p->workspace != nullptr && p->max_keys > 512) {
@@ -545,7 +545,7 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
     PCS_REQUIRE(splits == 1 || p->workspace_floats >= static_cast<long long>(p->n_tokens) * p->n_heads * splits * (p->vdim + 2),
                 "pcs_attn: workspace too small for %d splits", splits);
   }
-  if (decode && p->impl == 0) {
+  if (decode && automatic) {
     int parts = 0;
     if (int rc = pcs::launch_attn_group_decode(*p, st, &parts)) return rc;
     if (parts > 1) {

@@ -210,7 +210,7 @@ int launch_attn_talk(const pcs_attn_params& p, cudaStream_t st, int* splits_out)
   const int H = p.n_heads;
   PCS_REQUIRE(p.bias_r1 == nullptr && p.softcap == 0.f && !p.sink, "pcs_attn: mixed head scores do not combine with a distance bias, a cap or a sink");
   PCS_REQUIRE(H <= TK_THREADS, "pcs_attn: mixed head scores serve at most %d heads", TK_THREADS);
-  if (p.impl == 0) {
+  if (p.impl == 0 || p.impl == 3) {
     bool handled = false;
     if (int rc = launch_attn_talk_tc(p, st, &handled)) return rc;
     if (handled) { *splits_out = 1; return PCS_OK; }

@@ -35,7 +35,7 @@ constexpr float kRescale = 8.0f;
 constexpr int kMaxSplits = 8;  // blocks of a cluster that share one walk
 constexpr int kTab = 192;      // distances of a tile pair of 128 rows and 64 keys (191)
 
-__device__ int attn_tc5_timeouts;  // blocks whose waits ran out
+__device__ int attn_tc5_timeouts;  // blocks one of whose waits ran out
 
 template <int DP, int VP>
 struct Cfg {
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
   uint64_t* s_full = kv_empty + 2 * ST;   // [2 halves][2 buffers]
   uint64_t* p_full = s_full + 4;
   uint64_t* o_full = p_full + 4;
-  uint64_t* drained = o_full + 4;         // [2 halves], only when a wait ran out
+  uint64_t* drained = o_full + 4;         // [2 halves] every product has ended
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 2);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
     b = rem / p.n_heads;
     h = rem - b * p.n_heads;
     const int n = (p.seq_len[b] + BM - 1) / BM, n_max = (p.max_len + BM - 1) / BM;
-    if (ends) {
+    if (ends & 1) {
       t0 = n - 1 - tile; t1 = tile;
       if (t1 > t0) return;
       if (t1 == t0) t1 = -1;
@@ -152,6 +152,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
   float m = -INFINITY, l = 0.f;  // (softmax threads) the row's running maximum and sum
   int j = 0;                     // and its tiles so far
   bool again = false;            // its result is not finite
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, abort_word); };
+  // (ends bit 1) tests: in three blocks of four the TMA warp or one of the MMA warps gives up at some tile of the walk, as if its wait had run out
+  auto dropped = [&](int it) {
+    if (!(ends & 2) || warp != 8 + static_cast<int>(blockIdx.x & 3) || it != static_cast<int>(blockIdx.x >> 2 & 7)) return false;
+    *abort_word = 1;
+    return true;
+  };
 
   if (warp == 8 && lane == 0) {
     tma_prefetch_desc(&map_q);
@@ -189,15 +196,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
         if (rg[x].rows > 0)
           for (int f = 0; f < DP / 64; ++f) tma_load_3d(sQ + x * C::kQBytes + f * BM * 128, &map_q, q_full, f * 64, h, off + rg[x].q0);
     }
-    int it = 0;
-    bool ok = true;
-    for (; it < n_it; ++it) {
+    int issued = 0, ragged_it = -1;   // tiles asked for so far, the one that passes the `ragged` barrier
+    for (int it = 0; it < n_it; ++it) {
       const int s = it % ST, key0 = tile_of(it) * BN;
+      if (dropped(it)) break;
       if (it >= ST) {
         const uint32_t par = static_cast<uint32_t>((it / ST - 1) & 1);
-        ok = mbar_wait(&kv_empty[s], par, abort_word);
-        ok = __all_sync(0xffffffffu, mbar_wait(&kv_empty[ST + s], par, abort_word) && ok);
-        if (!ok) break;
+        const bool free = wait(&kv_empty[s], par) && wait(&kv_empty[ST + s], par);
+        if (!__all_sync(0xffffffffu, free)) break;
       }
       unsigned char* dk = sKV + s * (C::kKBytes + C::kVBytes);
       unsigned char* dv = dk + C::kKBytes;
@@ -213,10 +219,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
         for (int f = 0; f < DP / 64; ++f) tma_load_3d(dk + f * BN * 128, &map_k, bk, f * 64, key0, plane);
         for (int f = 0; f < VP / 64; ++f) tma_load_3d(dv + f * BN * 128, &map_v, bv, f * 64, key0, plane);
       }
+      ++issued;
       if (left < BN) {  // the sequence's last tile: rows behind its end hold anything, and 0 * NaN is not 0
+        ragged_it = it;
         __syncwarp();
-        mbar_wait(ragged, 0, abort_word);
-        __syncwarp();
+        if (!__all_sync(0xffffffffu, wait(ragged, 0))) break;
         for (int f = 0; f < (DP + VP) / 64; ++f)
           for (int i = left * 8 + lane; i < BN * 8; i += 32) *reinterpret_cast<uint4*>(dk + f * BN * 128 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
         fence_proxy_async_smem();
@@ -227,22 +234,23 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
         }
       }
     }
-    if (*abort_word) {  // copies still in flight must land before the block may end
-      if (lane == 0) {
-        const long long t_end = clock64() + (1ll << 28);
-        for (int i = max(0, it - ST); i < it; ++i)
-          while (!(mbar_try_wait(&k_full[i % ST], static_cast<uint32_t>((i / ST) & 1)) && mbar_try_wait(&v_full[i % ST], static_cast<uint32_t>((i / ST) & 1))) &&
-                 clock64() < t_end) {}
-        atomicAdd(&attn_tc5_timeouts, 1);
+    // all of it has landed when this warp is done (in a walk that was given up, the tiles nobody waited for)
+    mbar_drain(q_full, 0);
+    for (int i = max(0, issued - ST); i < issued; ++i) {
+      if (i == ragged_it) {
+        mbar_drain(ragged, 0);
+      } else {
+        mbar_drain(&k_full[i % ST], static_cast<uint32_t>((i / ST) & 1));
+        mbar_drain(&v_full[i % ST], static_cast<uint32_t>((i / ST) & 1));
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else if (warp >= 9) {
     // ===================== MMA issuers: warp 9 drives half 0, warp 10 half 1 =====================
     const int x = warp - 9;
     const Range r = x ? rg[1] : rg[0];
     const int leader = lane == 0;
-    auto all_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_word)) != 0; };
+    auto all_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };
     constexpr uint32_t idesc_qk = idesc_bf16(BM, BN, 0), idesc_pv = idesc_bf16(BM, VP, 1);
     const uint64_t q_desc = smem_desc_sw128(smem_u32(sQ + x * C::kQBytes), 16, 1024);
     const uint64_t k_desc0 = smem_desc_sw128(smem_u32(sKV), 16, 1024);
@@ -251,6 +259,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
     int jS = 0, itS = 0, jP = 0;   // scores issued, the walk's next tile for them; weights x values issued
     bool ok = all_wait(q_full, 0);
     for (int ip = 0; ip < n_it && ok; ++ip) {
+      if (dropped(ip)) break;
       // scores up to two tiles ahead of the weights, as long as the tile can arrive without this half's next release
       while (ok && jS < jP + 2) {
         while (itS < n_it && !r.has(tile_of(itS))) ++itS;
@@ -289,11 +298,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
       tc_commit(&kv_empty[x * ST + s], leader);
       ++jP;
     }
-    if (!ok) {  // products in flight end before TMEM is given back
-      tc_commit(&drained[x], leader);
-      const long long t_end = clock64() + (1ll << 28);
-      while (!mbar_try_wait(&drained[x], 0) && clock64() < t_end) {}
-    }
+    __syncwarp();
+    tc_commit(&drained[x], leader);   // and all products have ended
+    mbar_drain(&drained[x], 0);
     __syncwarp();
   } else {
     // ===================== softmax: warpgroup x owns half x, a thread one query row =====================
@@ -314,6 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
       m = p.sink_logit ? p.sink_logit[h] * kLog2e : 0.f;
       l = 1.f;
     }
+    // (a thread whose wait ran out goes on: the barriers below count on every thread, and the block's results are not used)
     if (r.rows > 0) {
       for (int it = 0; it < n_it; ++it) {
         const int k = tile_of(it);
@@ -335,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
           tb = dst + row + 63;
         }
         const uint32_t tmem_s = tmem_s0 + (j & 1) * BN;
-        mbar_wait(&s_full[x * 2 + (j & 1)], static_cast<uint32_t>((j >> 1) & 1), abort_word);
+        wait(&s_full[x * 2 + (j & 1)], static_cast<uint32_t>((j >> 1) & 1));
         __syncwarp();
         tc_fence_after();
         float sv[BN];
@@ -388,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
         const float alpha = grow ? ex2(m - m_new) : 1.f;
         if (grow) { m = m_new; l *= alpha; }
         if (j > 0 && __any_sync(0xffffffffu, grow)) {
-          mbar_wait(&o_full[x * 2 + ((j - 1) & 1)], static_cast<uint32_t>(((j - 1) >> 1) & 1), abort_word);
+          wait(&o_full[x * 2 + ((j - 1) & 1)], static_cast<uint32_t>(((j - 1) >> 1) & 1));
           __syncwarp();
           tc_fence_after();
 #pragma unroll 1
@@ -426,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
         mbar_arrive(&p_full[x * 2 + (j & 1)]);
         ++j;
       }
-      if (j > 0) mbar_wait(&o_full[x * 2 + ((j - 1) & 1)], static_cast<uint32_t>(((j - 1) >> 1) & 1), abort_word);
+      if (j > 0) wait(&o_full[x * 2 + ((j - 1) & 1)], static_cast<uint32_t>(((j - 1) >> 1) & 1));
       __syncwarp();
       tc_fence_after();
       if (splits == 1) {  // the result: O / l, times the constant and the head's gate
@@ -467,6 +475,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
     float* ml = reinterpret_cast<float*>(smem + C::kPartBytes);
     __syncwarp();
     cluster_barrier();
+    if (*abort_word) m = l = __int_as_float(0x7fffffff);   // (NaN: what the cluster sees of a walk that was given up)
     if (mine) {
       const uint32_t tmem_o = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + C::kColO + x * VP;
       for (int q = 0; q < splits; ++q) st_cluster(cluster_addr(ml + ((rank * 2 + x) * BM + row) * 2, q), m, l);
@@ -531,6 +540,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc5_kernel(const __grid_cons
   }
   tc_fence_before();
   __syncthreads();   // TMEM has been read
+  if (*abort_word) {   // a wait ran out: the block is counted, and its rows are formed again
+    again = warp < 8 && (tid & 127) < ((warp >> 2) ? rg[1].rows : rg[0].rows);
+    if (tid == 0) atomicAdd(&attn_tc5_timeouts, 1);
+  }
   if (warp < 8) {   // rows whose result is not finite: from the keys they see alone (this block's columns of them)
     const int q0 = (warp >> 2) ? rg[1].q0 : rg[0].q0, cols = VP / splits, c0 = splits > 1 ? rank * cols : 0;
     for (uint32_t w = __ballot_sync(0xffffffffu, again && c0 < p.vdim); w; w &= w - 1) {
@@ -620,7 +633,7 @@ int launch(const pcs_attn_params& p, cudaStream_t st) {
   const Plan plan(p, DP, VP, slots);
   cfg.gridDim = dim3(static_cast<unsigned>(((p.max_len + BM - 1) / BM + 1) / 2) * p.n_seqs * p.n_heads * plan.splits);
   attr[0].val.clusterDim.x = static_cast<unsigned>(plan.splits);
-  PCS_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p, plan.ends, plan.splits));
+  PCS_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p, plan.ends | (p.impl == 3 ? 2 : 0), plan.splits));
   count_launch();
   return PCS_OK;
 }
@@ -656,7 +669,8 @@ int launch_attn_tc5(const pcs_attn_params& p, cudaStream_t st, bool* handled) {
 
 }  // namespace pcs
 
-// blocks of the tcgen05 attention kernel whose bounded waits ran out so far (0 in a working system); synchronises
+// blocks of the tcgen05 attention kernel one of whose bounded waits ran out so far (0 in a working system; their rows were formed without tensor cores);
+// synchronises
 PCS_API int pcs_attn_timeouts(void) {
   int n = -1;
   if (cudaMemcpyFromSymbol(&n, pcs::attn_tc5_timeouts, sizeof(n)) != cudaSuccess) return -1;
