@@ -13,8 +13,6 @@
 // 16 sequences at 2 - 4 thousand keys, 16 heads over 4 K/V heads of 128, bfloat16 (B200): 115 -> 39 us (2.6 TB/s of distinct bytes; attn_decode_kernel, one
 // block per head, reads every row four times through L2 and adds a merge launch of 4 us).  16 heads of their own: 16 sequences at 2048 keys 83 -> 54 us; one
 // sequence stays launch-sized (15 us).  Eight row loads at a time need 233 registers, two blocks per SM and a second wave: 53 us.
-#include <mutex>
-
 #include "seq_attn.cuh"
 #include "seq_tc5.cuh"
 
@@ -303,18 +301,20 @@ int launch(const pcs_attn_params& p, int* splits_io, int per_group, cudaStream_t
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  static int room[kMaxCluster + 1];   // clusters of s blocks that run side by side
-  static std::once_flag once;
-  cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(full));
-    for (int s = 1; s <= kMaxCluster && err == cudaSuccess; ++s) {
-      attr[0].val.clusterDim.x = s;
-      cfg.gridDim = dim3(s);
-      err = cudaOccupancyMaxActiveClusters(&room[s], kernel, &cfg);
-    }
-  });
-  PCS_CHECK_CUDA(err);
+  struct Info { int room[kMaxCluster + 1]; };   // clusters of s blocks that run side by side
+  static PerDevice<Info> per_device;
+  const Info* info;
+  if (int rc = per_device.get(&info, [&](Info& x) {
+        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(full));
+        for (int s = 1; s <= kMaxCluster && err == cudaSuccess; ++s) {
+          attr[0].val.clusterDim.x = s;
+          cfg.gridDim = dim3(s);
+          err = cudaOccupancyMaxActiveClusters(&x.room[s], kernel, &cfg);
+        }
+        return err;
+      }))
+    return rc;
+  const int* room = info->room;
   // One wave: the largest cluster of which all fit side by side.  Where even the largest leaves more than half of the GPU idle and the keys allow more
   // splits, the splits go through the workspace and a second launch (4 us) instead.
   const long long groups = static_cast<long long>(p.n_tokens) * p.n_kv_heads * per_group;

@@ -10,8 +10,6 @@
 //
 // 8 heads of 128 (B200), against the plain kernel (one block per token and head, every row read again): 1024 tokens 818 -> 103 us (21 TFLOP/s), 2048: 2.92 -> 0.32
 // ms, 64 behind 400 stored 76 -> 21 us, 16 behind 4000 100 -> 69 us.  A cluster shares a walk where there are few blocks (choose_splits).
-#include <mutex>
-
 #include "seq_attn.cuh"
 #include "seq_mma.cuh"
 #include "seq_tc5.cuh"
@@ -292,24 +290,24 @@ int launch(const pcs_attn_params& p, unsigned grid, cudaStream_t st) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  // blocks that run side by side in clusters of 2^i, at rows of up to 128 elements and of more
-  static int slots[2][4];
-  static std::once_flag once;
-  cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    for (int w = 0; w < 2; ++w)
-      for (int i = 0; i < 4 && err == cudaSuccess; ++i) {
-        int n = 0;
-        attr[0].val.clusterDim.x = 1u << i;
-        cfg.gridDim = dim3(1u << i);
-        cfg.dynamicSmemBytes = (static_cast<size_t>(FM + FN) * ((w ? 256 : 128) + 4) + FN * VP + FM * (FN + 4) + 96) * sizeof(float);
-        err = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-        slots[w][i] = n << i;
-      }
-  });
-  PCS_CHECK_CUDA(err);
-  const int splits = choose_splits(p, slots[p.dim > 128]);
+  struct Info { int slots[2][4]; };   // blocks that run side by side in clusters of 2^i, at rows of up to 128 elements and of more
+  static PerDevice<Info> per_device;
+  const Info* info;
+  if (int rc = per_device.get(&info, [&](Info& x) {
+        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        for (int w = 0; w < 2; ++w)
+          for (int i = 0; i < 4 && err == cudaSuccess; ++i) {
+            int n = 0;
+            attr[0].val.clusterDim.x = 1u << i;
+            cfg.gridDim = dim3(1u << i);
+            cfg.dynamicSmemBytes = (static_cast<size_t>(FM + FN) * ((w ? 256 : 128) + 4) + FN * VP + FM * (FN + 4) + 96) * sizeof(float);
+            err = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+            x.slots[w][i] = n << i;
+          }
+        return err;
+      }))
+    return rc;
+  const int splits = choose_splits(p, info->slots[p.dim > 128]);
   cfg.gridDim = dim3(grid * splits);
   cfg.dynamicSmemBytes = smem;
   attr[0].val.clusterDim.x = static_cast<unsigned>(splits);

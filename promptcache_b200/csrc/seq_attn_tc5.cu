@@ -610,27 +610,28 @@ int launch(const pcs_attn_params& p, cudaStream_t st) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  static int slots[4];
-  static std::once_flag once;
-  cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
-    for (int i = 0; i < 4 && err == cudaSuccess; ++i) {
-      int n = 0;
-      attr[0].val.clusterDim.x = 1u << i;
-      cfg.gridDim = dim3(1u << i);
-      err = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-      slots[i] = n << i;
-    }
-  });
-  PCS_CHECK_CUDA(err);
+  struct Info { int slots[4]; };   // blocks that run side by side in clusters of 2^i
+  static PerDevice<Info> per_device;
+  const Info* info;
+  if (int rc = per_device.get(&info, [&](Info& x) {
+        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+        for (int i = 0; i < 4 && err == cudaSuccess; ++i) {
+          int n = 0;
+          attr[0].val.clusterDim.x = 1u << i;
+          cfg.gridDim = dim3(1u << i);
+          err = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+          x.slots[i] = n << i;
+        }
+        return err;
+      }))
+    return rc;
   const unsigned long long D = p.dim, V = p.vdim, cap = p.cap, H = p.n_heads;
   const unsigned long long planes = 1ull << 30;  // (slot, K/V head) planes: the pool's slot count is the caller's
   CUtensorMap mq, mk, mv;
   if (int rc = tensor_map_bf16(&mq, p.q, {D, H, static_cast<unsigned long long>(p.n_tokens)}, {D * 2, H * D * 2}, {64, 1, BM})) return rc;
   if (int rc = tensor_map_bf16(&mk, p.k_pool, {D, cap, planes}, {D * 2, cap * D * 2}, {64, BN, 1})) return rc;
   if (int rc = tensor_map_bf16(&mv, p.v_pool, {V, cap, planes}, {V * 2, cap * V * 2}, {64, BN, 1})) return rc;
-  const Plan plan(p, DP, VP, slots);
+  const Plan plan(p, DP, VP, info->slots);
   cfg.gridDim = dim3(static_cast<unsigned>(((p.max_len + BM - 1) / BM + 1) / 2) * p.n_seqs * p.n_heads * plan.splits);
   attr[0].val.clusterDim.x = static_cast<unsigned>(plan.splits);
   PCS_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, p, plan.ends | (p.impl == 3 ? 2 : 0), plan.splits));
