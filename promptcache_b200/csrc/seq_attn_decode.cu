@@ -11,8 +11,7 @@
 // workspace to attn_combine_kernel.
 //
 // 16 sequences at 2 - 4 thousand keys, 16 heads over 4 K/V heads of 128, bfloat16 (B200): 115 -> 39 us (2.6 TB/s of distinct bytes; attn_decode_kernel, one
-// block per head, reads every row four times through L2 and adds a merge launch of 4 us).  16 heads of their own: 16 sequences at 2048 keys 83 -> 54 us; one
-// sequence stays launch-sized (15 us).  Eight row loads at a time need 233 registers, two blocks per SM and a second wave: 53 us.
+// block per head, reads every row four times through L2 and adds a merge launch of 4 us).  16 heads of their own: 16 sequences at 2048 keys 83 -> 54 us.  Eight row loads at a time need 233 registers, two blocks per SM and a second wave: 53 us.
 #include "seq_attn.cuh"
 #include "seq_tc5.cuh"
 
@@ -214,75 +213,82 @@ __global__ void __launch_bounds__(kThreads) attn_group_decode_kernel(const pcs_a
     if constexpr (N == 8) stx(d, acc[hh]); else stx(d, acc[hh]);
   }
   __syncthreads();
-  auto block_ml = [&](int hh, float* f, float& M, float& L) {   // the warps' factors, the common maximum and the sum of one head
-    M = -INFINITY;
+  // per head, once: the warps' factors (in the place of their maxima), the common maximum, the sum, and what a finished result is multiplied by.  (Formed
+  // again for every column, the end of a block of eight heads of 256 columns took 9 us in a cluster.)
+  float* common = ml + 1;   // [3][head], in the places of the first three warps' sums
+  if (tid < GP) {
+    float M = -INFINITY, L = 0.f;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) M = fmaxf(M, ml[(w * GP + hh) * 2]);
-    L = 0.f;
+    for (int w = 0; w < kWarps; ++w) M = fmaxf(M, ml[(w * GP + tid) * 2]);
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      const float mw = ml[(w * GP + hh) * 2];
-      f[w] = mw == -INFINITY ? 0.f : expf(mw - M);
-      L = fmaf(ml[(w * GP + hh) * 2 + 1], f[w], L);
+      float* x = ml + (w * GP + tid) * 2;
+      const float f = x[0] == -INFINITY ? 0.f : expf(x[0] - M);
+      L = fmaf(x[1], f, L);
+      x[0] = f;
     }
-  };
-  auto block_sum_of = [&](int hh, int c, const float* f) {
+    common[tid * 2] = M;
+    common[(GP + tid) * 2] = L;
+    if (tid < heads) common[(2 * GP + tid) * 2] = (L > 0.f ? 1.f / L : 0.f) * out_factor<T>(p, t, hb + tid);
+  }
+  __syncthreads();
+  auto block_sum_of = [&](int hh, int c) {
     float a = 0.f;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
       float x = 0.f;
 #pragma unroll
       for (int r = 0; r < C::RV; ++r) x += part[((w * C::RV + r) * GP + hh) * C::VMAX + c];
-      a = fmaf(x, f[w], a);
+      a = fmaf(x, ml[(w * GP + hh) * 2], a);
     }
     return a;
   };
-  float f[kWarps], M, L;
-  if (S == 1) {
-    for (int i = tid; i < heads * C::VMAX; i += kThreads) {
-      const int hh = i / C::VMAX, c = i - hh * C::VMAX;
-      if (c >= V) continue;
-      block_ml(hh, f, M, L);
-      stf(out_row<T>(p, t, hb + hh) + c, block_sum_of(hh, c, f) * (L > 0.f ? 1.f / L : 0.f) * out_factor<T>(p, t, hb + hh));
-    }
-    return;
-  }
   if (!cluster) {
     for (int i = tid; i < heads * C::VMAX; i += kThreads) {
       const int hh = i / C::VMAX, c = i - hh * C::VMAX;
       if (c >= V) continue;
-      block_ml(hh, f, M, L);
-      float* ws = p.workspace + ((static_cast<long long>(t) * p.n_heads + hb + hh) * S + sp) * (V + 2);
-      if (c == 0) { ws[0] = M; ws[1] = L; }
-      ws[2 + c] = block_sum_of(hh, c, f);
+      const float a = block_sum_of(hh, c);
+      if (S == 1) {
+        stf(out_row<T>(p, t, hb + hh) + c, a * common[(2 * GP + hh) * 2]);
+      } else {
+        float* ws = p.workspace + ((static_cast<long long>(t) * p.n_heads + hb + hh) * S + sp) * (V + 2);
+        if (c == 0) { ws[0] = common[hh * 2]; ws[1] = common[(GP + hh) * 2]; }
+        ws[2 + c] = a;
+      }
     }
     return;
   }
   // a cluster's splits: block q writes every S-th group of eight columns; everybody sends it the sums of them
+  float* mm = merge + kMaxCluster * GP * C::VMAX;
   __syncwarp();
   cluster_wait();
   for (int i = tid; i < heads * C::VMAX; i += kThreads) {
     const int hh = i / C::VMAX, c = i - hh * C::VMAX;
     if (c >= V) continue;
-    block_ml(hh, f, M, L);
-    const int q8 = (c / 8) % S;
-    st_cluster(cluster_addr(merge + (sp * GP + hh) * C::VMAX + c, q8), block_sum_of(hh, c, f));
-    if (c < S) st_cluster(cluster_addr(merge + kMaxCluster * GP * C::VMAX + (sp * GP + hh) * 2, c), M, L);
+    st_cluster(cluster_addr(merge + (sp * GP + hh) * C::VMAX + c, (c / 8) % S), block_sum_of(hh, c));
+    if (c < S) st_cluster(cluster_addr(mm + (sp * GP + hh) * 2, c), common[hh * 2], common[(GP + hh) * 2]);
   }
   __syncwarp();
   cluster_barrier();
-  for (int i = tid; i < heads * C::VMAX; i += kThreads) {
-    const int hh = i / C::VMAX, c = i - hh * C::VMAX;
-    if (c >= V || (c / 8) % S != sp) continue;
-    const float* mm = merge + kMaxCluster * GP * C::VMAX;
-    float mt = -INFINITY, lt = 0.f, a = 0.f;
-    for (int r = 0; r < S; ++r) mt = fmaxf(mt, mm[(r * GP + hh) * 2]);
+  if (tid < heads) {   // the splits' factors, in the place of their maxima
+    float mt = -INFINITY, lt = 0.f;
+    for (int r = 0; r < S; ++r) mt = fmaxf(mt, mm[(r * GP + tid) * 2]);
     for (int r = 0; r < S; ++r) {
-      const float mr = mm[(r * GP + hh) * 2], fr = mr == -INFINITY ? 0.f : expf(mr - mt);
-      lt = fmaf(mm[(r * GP + hh) * 2 + 1], fr, lt);
-      a = fmaf(merge[(r * GP + hh) * C::VMAX + c], fr, a);
+      float* x = mm + (r * GP + tid) * 2;
+      const float f = x[0] == -INFINITY ? 0.f : expf(x[0] - mt);
+      lt = fmaf(x[1], f, lt);
+      x[0] = f;
     }
-    stf(out_row<T>(p, t, hb + hh) + c, a * (lt > 0.f ? 1.f / lt : 0.f) * out_factor<T>(p, t, hb + hh));
+    mm[tid * 2 + 1] = (lt > 0.f ? 1.f / lt : 0.f) * out_factor<T>(p, t, hb + tid);
+  }
+  __syncthreads();
+  const int mine = (C::VMAX / 8 - sp + S - 1) / S * 8;   // this block's columns of a head
+  for (int i = tid; i < heads * mine; i += kThreads) {
+    const int hh = i / mine, j = i - hh * mine, c = ((j >> 3) * S + sp) * 8 + (j & 7);
+    if (c >= V) continue;
+    float a = 0.f;
+    for (int r = 0; r < S; ++r) a = fmaf(merge[(r * GP + hh) * C::VMAX + c], mm[(r * GP + hh) * 2], a);
+    stf(out_row<T>(p, t, hb + hh) + c, a * mm[hh * 2 + 1]);
   }
 }
 
@@ -315,14 +321,19 @@ int launch(const pcs_attn_params& p, int* splits_io, int per_group, cudaStream_t
       }))
     return rc;
   const int* room = info->room;
-  // One wave: the largest cluster of which all fit side by side.  Where even the largest leaves more than half of the GPU idle and the keys allow more
-  // splits, the splits go through the workspace and a second launch (4 us) instead.
-  const long long groups = static_cast<long long>(p.n_tokens) * p.n_kv_heads * per_group;
+  // One wave: the largest cluster of which all fit side by side.  Few heads over many keys: more splits than a cluster has, through the workspace and a second
+  // launch (6 us with the merge).  max_keys is what the pool holds, and the sequence may be short, so neither end may lose: one token of 8 heads of 128 over 2, 300,
+  // 1000, 4000, 8000 keys of a pool of 8192 takes 7, 8, 10, 19, 29 us in a cluster, 12, 12, 12, 16, 19 with 24 splits (64 splits: 14 to 18; one block per head: 14
+  // to 21); two tokens 8, 8, 10, 19, 28 and 12, 14, 14, 19, 20.  Rows of 8 lanes cost half, rows of 32 lanes twice as much per key.
+  const long long groups = static_cast<long long>(p.n_tokens) * p.n_kv_heads * per_group, all_heads = static_cast<long long>(p.n_tokens) * p.n_heads;
   int splits = *splits_io;
   bool cluster = true;
-  if (splits > 2 * kMaxCluster && groups * kMaxCluster * 2 <= room[1]) {
+  const bool few = LK == 32 ? all_heads <= 16 : LK == 16 ? all_heads <= (p.max_keys > 4096 ? 16 : 8) : all_heads <= 8 && p.max_keys > 16384;
+  if (few && p.max_keys >= (2 * kMaxCluster + 1) * 128 && groups * kMaxCluster * 2 <= room[1]) {
     const long long want = room[1] / groups;
-    int wide = splits > want ? static_cast<int>(want) : splits;
+    int wide = p.max_keys > 341 * 24 ? p.max_keys / 341 : 24;
+    if (wide > p.max_keys / 128) wide = p.max_keys / 128;
+    if (wide > want) wide = static_cast<int>(want);
     if (wide > kAttnMaxSplits) wide = kAttnMaxSplits;
     // (a workspace that holds only the fewer splits that pcs_attn asks for: a cluster, which needs none)
     if (p.workspace_floats >= static_cast<long long>(p.n_tokens) * p.n_heads * wide * (p.vdim + 2)) {
@@ -376,7 +387,12 @@ int launch_attn_group_decode(const pcs_attn_params& p, cudaStream_t st, int* spl
   if (p.dim > pieces * N || p.vdim > pieces * N || !al16(p.q) || !al16(p.k_pool) || !al16(p.v_pool) || p.n_tokens > 65535) return PCS_OK;
   const int G = p.n_heads / p.n_kv_heads, gp = G >= 8 ? 8 : G > 2 ? 4 << (G > 4) : G, per_group = (G + gp - 1) / gp;
   if (static_cast<long long>(p.n_kv_heads) * per_group > 65535) return PCS_OK;
-  int splits = p.max_keys > 128 ? p.max_keys / 128 : 1, rc;   // a split has at least 128 keys
+  // Eight heads per block take a block 2 us longer to begin and to end than one head does: with 24 (token, head) pairs or fewer over many keys, or 128 keys at most, a
+  // block per head is the faster form (16 heads of 256 over one K/V head, one token: 50 keys 8.3 against 10.4 us, 50 of a pool of 8192 14.5 / 15.5, 4000 of them
+  // 27 / 27; of 64 over two: 4000 keys 16.5 / 18.6), and a split has 48 keys (300 keys of 20 heads of 128: 11.2 instead of 13.3 us; one head per block 12.4).
+  if (gp == 8 && (p.max_keys <= 128 || static_cast<long long>(p.n_tokens) * p.n_heads <= 24)) return PCS_OK;
+  const int least = gp == 8 ? 48 : 128;
+  int splits = p.max_keys > least ? p.max_keys / least : 1, rc;
   PCS_DISPATCH(p.dtype, rc = launch_t<T>(p, gp, &splits, per_group, st));
   if (rc) return rc;
   *splits_out = splits;
