@@ -648,15 +648,41 @@ int launch_opt(const pcs_attn_params& p, cudaStream_t st) {
 
 }  // namespace
 
-// Sixteen or more new tokens of some entry, heads of up to 192 / 128 elements in 16-byte pieces: measured faster than the mma.sync kernel at every size tried
-// (40 new tokens 9.6 -> 9.1 us, 66 behind 500 stored 29 -> 13 us).
+// Entries of at most one tile of query rows, each of which leaves half of its block idle: where the mma.sync kernel (64 rows per block, three blocks per SM) is
+// expected to be faster.  Both sides in microseconds, from 564 shapes of 16 to 128 new tokens x 1 to 48 entries behind 0 to 1000 stored (B200): a block here takes
+// 3.4 to 4.1 and 1.1 per key tile, one at a time on an SM; there a key tile takes an SM 1.8 to 4.5 with one to three blocks on it.  At 16 heads of 64, mma.sync / tcgen05:
+// 16 x 48 entries 12 / 31, 64 x 16 8.3 / 12.4, 64 x 48 behind 500 60 / 81, 64 behind 500 22 / 11; of 128: 64 x 48 21 / 33, 16 x 16 10 / 15, 64 x 48 behind 500 92 / 90.
+bool short_entries(const pcs_attn_params& p) {
+  if (p.max_len > BM || p.dim > 128) return false;
+  constexpr int kSMs = 148, kOld = 64;
+  const int wide = (p.dim > 64) + (p.vdim > 64);
+  static const double kBase[3] = {4.6, 5.0, 6.0}, kTile[3][4] = {{0.0, 1.8, 2.1, 2.6}, {0.0, 1.95, 2.55, 3.5}, {0.0, 2.45, 3.2, 4.46}};
+  const bool cap = p.softcap > 0.f;
+  const double set_up = wide ? 4.1 : 3.4, tile = (wide ? 1.16 : 1.09) + (cap ? 0.45 : 0.0), merge[4] = {0.0, 3.0, 3.5, 5.0};
+  double keys = p.max_keys > 0 && p.max_keys < p.cap ? p.max_keys : p.cap;
+  if (p.window > 0) keys = fmin(keys, p.window + BM + fmax(p.keep_first, 0) + BN);
+  if (p.chunk > 0) keys = fmin(keys, p.chunk + BN);
+  const double tiles = ceil(fmax(keys, 1.0) / BN);
+  const long long blocks = static_cast<long long>(p.n_seqs) * p.n_heads;
+  double here = 3.5 + (blocks + kSMs - 1) / kSMs * (set_up + tile * tiles);
+  for (int i = 1; i < 4; ++i)
+    if (blocks << i <= kSMs) here = fmin(here, 3.5 + set_up + merge[i] + tile * ceil(tiles / (1 << i)));
+  long long there = blocks * ((p.max_len + kOld - 1) / kOld);
+  const long long most = (p.n_tokens / kOld + static_cast<long long>(p.n_seqs)) * p.n_heads;
+  if (there > most) there = most;
+  const long long full = there / (3 * kSMs), rest = there % (3 * kSMs);
+  const double old = kBase[wide] + tiles * (cap ? 1.07 : 1.0) * (full * kTile[wide][3] + kTile[wide][(rest + kSMs - 1) / kSMs]);
+  return old < 0.95 * here;
+}
+
+// Sixteen or more new tokens of some entry, heads of up to 192 / 128 elements in 16-byte pieces
 int launch_attn_tc5(const pcs_attn_params& p, cudaStream_t st, bool* handled) {
   *handled = false;
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if (p.dtype != PCS_BF16 || p.max_len < 16 || (p.v_row_stride != 0 && p.v_row_stride != p.vdim) || p.dim % 8 != 0 || p.vdim % 8 != 0 || p.dim > 192 || p.vdim > 128)
     return PCS_OK;
   if (!p.seq_pos0 || !p.seq_len || !p.seq_off || !al16(p.q) || !al16(p.k_pool) || !al16(p.v_pool) || !al16(p.out) || p.out_stride % 8 != 0) return PCS_OK;
-  if (((p.max_len + BM - 1LL) / BM + 1) / 2 * p.n_seqs * p.n_heads * kMaxSplits > 0x7fffffffLL) return PCS_OK;
+  if (((p.max_len + BM - 1LL) / BM + 1) / 2 * p.n_seqs * p.n_heads * kMaxSplits > 0x7fffffffLL || short_entries(p)) return PCS_OK;
   *handled = true;
   if (p.vdim <= 64) {
     if (p.dim <= 64) return launch_opt<64, 64>(p, st);
