@@ -258,19 +258,19 @@ int choose_splits(const pcs_attn_params& p, const int (&slots)[4]) {
   const double tile = 7.1 * (p.dim + p.vdim) / 256.0, over[4] = {3.0, 6.0, 6.5, 7.0};
   const int keys = p.max_keys > 0 && p.max_keys < p.cap ? p.max_keys : p.cap, n = (p.max_len + FM - 1) / FM;
   const double blocks = fmin(static_cast<double>(p.n_seqs) * n, p.n_tokens / static_cast<double>(FM) + p.n_seqs) * p.n_heads;
-  double sum = 0.0, longest = 0.0, best = 1e30;
+  double sum = 0.0, longest = 0.0, best = 1e30;   // (longest: in tiles)
   for (int t = 0; t < n; ++t) {
     double k = fmax(fmin(keys, keys - p.max_len + (t + 1.0) * FM), 1.0);
     if (p.window > 0) k = fmin(k, p.window + FM + fmax(p.keep_first, 0) + FN);
     if (p.chunk > 0) k = fmin(k, p.chunk + FN);
-    longest = fmax(longest, ceil(k / FN) * tile);
+    longest = fmax(longest, ceil(k / FN));
     sum += ceil(k / FN) * tile;
   }
   int splits = 1;
   for (int i = 0; i < 4; ++i) {
     const int s = 1 << i;
     if (slots[i] < s) continue;
-    double t = longest / s + over[i];
+    double t = ceil(longest / s) * tile + over[i];   // (a walk of one tile is not shared)
     if (blocks * s > slots[i]) t = fmax(t, 1.15 * (sum / n * blocks + blocks * s * over[i]) / slots[i]);
     if (t < best) { best = t; splits = s; }
   }
@@ -324,6 +324,14 @@ int launch_attn_f32(const pcs_attn_params& p, cudaStream_t st, bool* handled) {
   if (p.dtype != PCS_F32 || p.max_len < 16 || (p.v_row_stride != 0 && p.v_row_stride != p.vdim) || p.dim % 4 != 0 || p.vdim % 4 != 0 || p.dim > 256 || p.vdim > 128)
     return PCS_OK;
   if (!p.seq_pos0 || !p.seq_len || !p.seq_off || !al16(p.q) || !al16(p.k_pool) || !al16(p.v_pool) || !al16(p.out) || p.out_stride % 4 != 0) return PCS_OK;
+  // Few tokens over few keys: a block per token and head begins and ends sooner.  Decoding kernels (a workspace is given) / plain kernel / tiles, B200, us: 16 tokens of 8
+  // heads of 128 over 16 keys 6.5 / 10.5 / 12.6, over 66 8.3 / 14.5 / 16.5; 40 over 40 8.5 / 12.4 / 15.2; 24 x 4 entries over 24 - / 10.7 / 12.5, 24 over 72
+  // - / 14.6 / 15.9, 16 x 16 entries over 16 - / 16.5 / 12.6; of 12 heads of 64: 16 over 16 - / 8.5 / 10.4, 48 over 48 - / 10.6 / 10.5.
+  const int keys = p.max_keys > 0 && p.max_keys < p.cap ? p.max_keys : p.cap;
+  const long long pairs = static_cast<long long>(p.n_tokens) * p.n_heads;
+  if (p.workspace ? p.n_tokens <= 16 || (static_cast<long long>(keys) * (p.dim + p.vdim) <= 49152 && pairs <= 1024)
+                  : keys <= (p.dim + p.vdim >= 256 ? 80 : 32) && pairs <= 1024 && pairs * keys <= 32768)
+    return PCS_OK;
   const long long grid = (p.max_len + FM - 1LL) / FM * p.n_seqs * p.n_heads;
   if (grid * kMaxSplits > 0x7fffffffLL) return PCS_OK;
   *handled = true;
