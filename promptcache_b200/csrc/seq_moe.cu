@@ -188,34 +188,50 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const pcs_route_params p
   route_select(p, t, lane, z, c, gs);
 }
 
-// The same for many tokens: two tokens per block, four warps per token.  Each warp takes every fourth router output (a row comes from L1 for the second
-// token), the first one then selects.  Bound by the latency of the dots' loads, so what counts is the warps in flight: with one warp per token (eight
-// tokens per block) 14 warps per SM walked all outputs, 38 us of a feed-forward of 197 us at 2048 tokens, 16 outputs, width 2048 (B200); now it is 188 us.  (Four
-// rows at a time in one warp: 43.8 us, its registers leave one block per SM.)  An output's sum is one warp's, so results equal the block-per-token kernel's.
-constexpr int kWarpRouteOutputs = 256, kRouteTokens = 2, kRouteWarps = 8 / kRouteTokens;
-template <typename T>
+// The same for many tokens: TOKENS per block, 8 / TOKENS warps per token.  Each warp of a token takes its share of the router's outputs (a row comes from L1 for
+// the block's other tokens), the first one then selects.  An output's sum is one warp's, so results equal the block-per-token kernel's.
+//
+// Bound by the latency of the dots' loads, so what counts is the warps in flight while there are few tokens, and the warps that wait for a token's
+// selection when there are many.  Two, four and eight tokens per block, us on B200, width 1024 / 2048 in bfloat16:
+//   tokens x outputs   2                4                8
+//   1500 x 8           14.6 / 16.7      10.5 / 12.6      12.6 / 16.7
+//   2048 x 16          17.7 / 22.8      16.7 / 22.8      18.7 / 26.3
+//   4096 x 16          31.0 / 41.3      24.9 / 37.2      24.9 / 39.2
+//   3000 x 8           18.7 / 22.8      18.7 / 22.8      14.6 / 18.7
+//   2048 x 64          39.2 / 62.7      43.3 / 69.9      51.5 / 82.2
+//   4096 x 128          126 / 211        130 / 215        154 / 255
+//   16384 x 64          253 / 419        247 / 409        240 / 416
+// (Four rows at a time in one warp: slower, its registers leave one block per SM.)
+constexpr int kWarpRouteOutputs = 256;
+static int route_tokens_per_block(int tokens, int outputs) {
+  if ((tokens >= 2500 && outputs < 64) || (tokens >= 7000 && outputs < 128)) return 8;
+  return tokens >= 1200 && outputs < 32 ? 4 : 2;
+}
+template <typename T, int TOKENS>
 __global__ void __launch_bounds__(256) moe_route_warp_kernel(const pcs_route_params p) {
-  __shared__ float buf[kRouteTokens][4 * kWarpRouteOutputs];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = warp % kRouteWarps, E = p.n_outputs, K = p.width;
-  const int t = blockIdx.x * kRouteTokens + warp / kRouteWarps;
-  float* z = buf[warp / kRouteWarps];
+  constexpr int WARPS = 8 / TOKENS;
+  __shared__ float buf[TOKENS][4 * kWarpRouteOutputs];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = warp % WARPS, E = p.n_outputs, K = p.width;
+  const int t = blockIdx.x * TOKENS + warp / WARPS;
+  float* z = buf[warp / WARPS];
   float* c = z + kWarpRouteOutputs;
   float* gs = c + kWarpRouteOutputs;
   if (t < p.n_tokens) {
     const T* h = static_cast<const T*>(p.h) + static_cast<long long>(t) * p.h_stride;
     const T* wr = static_cast<const T*>(p.w_router);
     const bool vec = K % Vec<T>::n == 0 && aligned16(h) && aligned16(wr) && (p.h_stride * sizeof(T)) % 16 == 0;
-    for (int e = sub; e < E; e += kRouteWarps) {
+    for (int e = sub; e < E; e += WARPS) {
       const float d = warp_dot(h, wr + static_cast<long long>(e) * K, K, lane, vec);
       if (lane == 0) z[e] = d;
     }
-    if (p.w_sg && sub == kRouteWarps - 1) {
+    if (p.w_sg && sub == WARPS - 1) {
       const T* ws = static_cast<const T*>(p.w_sg);
       const float d = warp_dot(h, ws, K, lane, vec && aligned16(ws));
       if (lane == 0) p.shared_gate[t] = sigmoidf_(d);
     }
   }
-  __syncthreads();
+  if constexpr (WARPS == 1) __syncwarp();
+  else __syncthreads();
   if (t < p.n_tokens && sub == 0) route_select(p, t, lane, z, c, gs);
 }
 
@@ -359,10 +375,14 @@ PCS_API int pcs_moe_route(const pcs_route_params* p, void* stream) {
   PCS_REQUIRE(p->top <= p->keep_groups * (p->n_outputs / p->n_groups), "pcs_moe_route: top %d exceeds the outputs of the kept groups", p->top);
   PCS_REQUIRE(p->w_sg == nullptr || p->shared_gate != nullptr, "pcs_moe_route: the shared gate needs its output");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (p->n_tokens >= 64 && p->n_outputs <= pcs::kWarpRouteOutputs)
-    PCS_DISPATCH(p->dtype, pcs::moe_route_warp_kernel<T><<<(p->n_tokens + pcs::kRouteTokens - 1) / pcs::kRouteTokens, 256, 0, st>>>(*p));
-  else
+  if (p->n_tokens >= 64 && p->n_outputs <= pcs::kWarpRouteOutputs) {
+    const int per = pcs::route_tokens_per_block(p->n_tokens, p->n_outputs), blocks = (p->n_tokens + per - 1) / per;
+    if (per == 8) PCS_DISPATCH(p->dtype, (pcs::moe_route_warp_kernel<T, 8><<<blocks, 256, 0, st>>>(*p)));
+    else if (per == 4) PCS_DISPATCH(p->dtype, (pcs::moe_route_warp_kernel<T, 4><<<blocks, 256, 0, st>>>(*p)));
+    else PCS_DISPATCH(p->dtype, (pcs::moe_route_warp_kernel<T, 2><<<blocks, 256, 0, st>>>(*p)));
+  } else {
     PCS_DISPATCH(p->dtype, pcs::moe_route_kernel<T><<<p->n_tokens, 256, 0, st>>>(*p));
+  }
   PCS_CHECK_CUDA(cudaGetLastError());
   pcs::count_launch();
   return PCS_OK;
