@@ -1556,7 +1556,7 @@ __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const
   const int cn = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const long long base = static_cast<long long>(cn) * H + head;
   const int row0 = PARTS == 2 ? 0 : blockIdx.z * R, first = p.chunk_first[cn] + row0, n = p.chunk_len[cn] - row0;
-  if (n <= 0) return;
+  if (PARTS == 3 && n <= 0) return;
   const float* qd = p.qd + (base * kC + row0) * D;
   const float* ag = p.a + (base * kC + row0) * kC;
   // a pair of numbers as PARTS packed pairs
@@ -1640,7 +1640,9 @@ __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const
     }
   }
   __syncthreads();
-  const uint32_t a_base = static_cast<uint32_t>(__cvta_generic_to_shared(As)) + ((lane & 15) * LD + (lane >> 4) * 8) * 2;
+  uint32_t a_base[PARTS];
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) a_base[i] = static_cast<uint32_t>(__cvta_generic_to_shared(As)) + ((i * R + (lane & 15)) * LD + (lane >> 4) * 8) * 2;
 #pragma unroll 1
   for (int kt = 0; kt < KT; ++kt) {
     uint32_t b[4][2][PARTS];
@@ -1655,7 +1657,7 @@ __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const
       if (m + row0 / 16 < kt - KD) continue;   // `a` is zero above the diagonal
       uint32_t x[PARTS][4];
 #pragma unroll
-      for (int i = 0; i < PARTS; ++i) ldsm_x4(a_base + ((i * R + m * 16) * LD + kt * 16) * 2, x[i][0], x[i][1], x[i][2], x[i][3]);
+      for (int i = 0; i < PARTS; ++i) ldsm_x4(a_base[i] + (m * 16 * LD + kt * 16) * 2, x[i][0], x[i][1], x[i][2], x[i][3]);
       if constexpr (PARTS == 2) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) mma_bf16(acc[q][m], x[0][0], x[0][1], x[0][2], x[0][3], b[q][0][0], b[q][1][0]);
