@@ -10,7 +10,7 @@
 // The warps meet once, at the end.  Two to eight splits of a token are one cluster and merge through distributed shared memory; more go through the
 // workspace to attn_combine_kernel.
 //
-// 16 sequences at 2 - 4 thousand keys, 16 heads over 4 K/V heads of 128, bfloat16 (B200): 115 -> 39 us (2.6 TB/s of distinct bytes; attn_decode_kernel, one
+// 16 sequences at 2 - 4 thousand keys, 16 heads over 4 K/V heads of 128, bfloat16 (B200): 112 -> 37 us (2.7 TB/s of distinct bytes; attn_decode_kernel, one
 // block per head, reads every row four times through L2 and adds a merge launch of 4 us).  16 heads of their own: 16 sequences at 2048 keys 83 -> 54 us.  Eight row loads at a time need 233 registers, two blocks per SM and a second wave: 53 us.
 #include "seq_attn.cuh"
 #include "seq_tc5.cuh"
@@ -321,17 +321,21 @@ int launch(const pcs_attn_params& p, int* splits_io, int per_group, cudaStream_t
       }))
     return rc;
   const int* room = info->room;
-  // One wave: the largest cluster of which all fit side by side.  Few heads over many keys: more splits than a cluster has, through the workspace and a second
-  // launch (6 us with the merge).  max_keys is what the pool holds, and the sequence may be short, so neither end may lose: one token of 8 heads of 128 over 2, 300,
-  // 1000, 4000, 8000 keys of a pool of 8192 takes 7, 8, 10, 19, 29 us in a cluster, 12, 12, 12, 16, 19 with 24 splits (64 splits: 14 to 18; one block per head: 14
-  // to 21); two tokens 8, 8, 10, 19, 28 and 12, 14, 14, 19, 20.  Rows of 8 lanes cost half, rows of 32 lanes twice as much per key.
+  // One wave: the largest cluster of which all fit side by side.  Few groups over many keys: more splits than a cluster has, through the workspace and a second
+  // launch (6 us with the merge).  max_keys is what the pool holds and the sequence may be short, so neither end may lose much.  Over 50, 300, 1000, 4000, 8000 keys of a
+  // pool of 8192, us: one token of 8 heads of 128 in a cluster 7, 8, 10, 19, 29, with 32 splits 13, 15, 15, 17, 19 (a block per head: 15, 17, 17, 17, 21); four tokens
+  // 8, 8, 10, 19, 29 and, with 24 splits, 12, 15, 17, 19, 24 (13, 15, 15, 27, 43); eight tokens 8, 8, 10, 23, 38 and 12, 15, 17, 23, 28 (13, 15, 19, 41, 76).  A
+  // key of a row over 32 lanes costs twice as much, so splits pay sooner; over 8 lanes half, and clusters win.
   const long long groups = static_cast<long long>(p.n_tokens) * p.n_kv_heads * per_group, all_heads = static_cast<long long>(p.n_tokens) * p.n_heads;
   int splits = *splits_io;
   bool cluster = true;
-  const bool few = LK == 32 ? all_heads <= 16 : LK == 16 ? all_heads <= (p.max_keys > 4096 ? 16 : 8) : all_heads <= 8 && p.max_keys > 16384;
+  const bool few = LK == 32   ? GP < 8 || all_heads <= 48 || p.max_keys > 4096
+                   : LK == 16 ? all_heads <= 8 || p.max_keys > 8192 || (p.max_keys > 4096 && (all_heads <= 16 || all_heads >= 64))
+                              : p.max_keys > 16384;
   if (few && p.max_keys >= (2 * kMaxCluster + 1) * 128 && groups * kMaxCluster * 2 <= room[1]) {
     const long long want = room[1] / groups;
-    int wide = p.max_keys > 341 * 24 ? p.max_keys / 341 : 24;
+    int wide = all_heads <= 8 ? 32 : 24;
+    if (wide < p.max_keys / 341) wide = p.max_keys / 341;
     if (wide > p.max_keys / 128) wide = p.max_keys / 128;
     if (wide > want) wide = static_cast<int>(want);
     if (wide > kAttnMaxSplits) wide = kAttnMaxSplits;
@@ -387,10 +391,10 @@ int launch_attn_group_decode(const pcs_attn_params& p, cudaStream_t st, int* spl
   if (p.dim > pieces * N || p.vdim > pieces * N || !al16(p.q) || !al16(p.k_pool) || !al16(p.v_pool) || p.n_tokens > 65535) return PCS_OK;
   const int G = p.n_heads / p.n_kv_heads, gp = G >= 8 ? 8 : G > 2 ? 4 << (G > 4) : G, per_group = (G + gp - 1) / gp;
   if (static_cast<long long>(p.n_kv_heads) * per_group > 65535) return PCS_OK;
-  // Eight heads per block take a block 2 us longer to begin and to end than one head does: with 24 (token, head) pairs or fewer over many keys, or 128 keys at most, a
-  // block per head is the faster form (16 heads of 256 over one K/V head, one token: 50 keys 8.3 against 10.4 us, 50 of a pool of 8192 14.5 / 15.5, 4000 of them
-  // 27 / 27; of 64 over two: 4000 keys 16.5 / 18.6), and a split has 48 keys (300 keys of 20 heads of 128: 11.2 instead of 13.3 us; one head per block 12.4).
-  if (gp == 8 && (p.max_keys <= 128 || static_cast<long long>(p.n_tokens) * p.n_heads <= 24)) return PCS_OK;
+  // Eight heads per block take a block 2 us longer to begin and to end than one head does: over 128 keys at most, and with 24 (token, head) pairs or fewer of narrow
+  // bfloat16 rows, a block per head is the faster form (16 heads of 256 over one K/V head, 50 keys: 8.3 against 10.4 us; 20 heads of 128, one token, 300 and
+  // 1000 keys of 8192: 14.5 and 14.5 against 16.5 and 17.5), and a split has 48 keys (300 keys of 20 heads of 128: 11.2 instead of 13.3 us; one head per block 12.4).
+  if (gp == 8 && (p.max_keys <= 128 || (p.dtype == PCS_BF16 && p.dim <= 128 && p.vdim <= 128 && static_cast<long long>(p.n_tokens) * p.n_heads <= 24))) return PCS_OK;
   const int least = gp == 8 ? 48 : 128;
   int splits = p.max_keys > least ? p.max_keys / least : 1, rc;
   PCS_DISPATCH(p.dtype, rc = launch_t<T>(p, gp, &splits, per_group, st));
