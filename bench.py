@@ -3,7 +3,7 @@
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference] [--config C1|C2|C3|C4|C5]
 
-One step = one request on BASELINE config C2 (code-generation-game shape: 7 cached segments [24,400x5,24] = 2048
+One step = one request on config C2 (code-generation-game shape: 7 cached segments [24,400x5,24] = 2048
 tokens, 16-token uncached suffix): request plan -> splice of ALL segments (retained-prefix shortcut off) -> 32-layer
 prefill of the suffix over the spliced cache (per layer: QKV projection with RoPE at position ids + in-place append in
 its epilogue, tcgen05 attention, o_proj / MLP as weight-streaming tcgen05 kernels) -> logits.  TTFT = ms_per_step;
@@ -12,7 +12,7 @@ random fp16 at the real dims, token ids synthetic (no network).
 
 N>1: one rank per GPU, every rank serves its own prompt against its own HBM-resident segment store (weak scaling, no
 data-path collective); NCCL only for the barrier, the max-over-ranks time and the one-time broadcast of the encoded
-segment store.  Every line also carries a `c5` block: BASELINE config C5 (B=64 prompts, each 32 of a 64-segment pool
+segment store.  Every line also carries a `c5` block: config C5 (B=64 prompts, each 32 of a 64-segment pool
 = 8192 cached tokens + 32-token suffix) served through `parallel.serve_batch`'s partition (prompt b -> rank b mod G),
 with the NCCL pool broadcast timed against the NVLink peer rate.  At N=1 the line also carries `c4` (Falcon-7B real
 dims, parameterized schema), the suffix sweep S and the CPU baseline.
@@ -111,7 +111,7 @@ SEG_LENS = {"C1": [24] + [92] * 6 + [24], "C2": [24] + [400] * 5 + [24], "C3": [
 
 
 def build_lm(model_key, dev, layers=None):
-    """The CUDA-path LanguageModel of a BASELINE config at real dims, seeded random fp16 weights."""
+    """The CUDA-path LanguageModel of a config at real dims, seeded random fp16 weights."""
     from promptcache_b200.model import Falcon, Llama2, LlamaConfigLite, LlamaForCausalLM
     from promptcache_b200.model.falcon import FalconConfigLite, FalconForCausalLM
     from promptcache_b200.synthetic import MODEL_DIMS, IdTokenizer
@@ -145,7 +145,7 @@ def weight_bytes(md, model_key):
 
 
 class RequestStep:
-    """One request of a flat BASELINE config (C1-C4) on one GPU: device-resident arm and public-API arm."""
+    """One request of a flat config (C1-C4) on one GPU: device-resident arm and public-API arm."""
 
     def __init__(self, lm, case, dev, world, rank, seg_lens=None):
         from promptcache_b200 import CacheEngine, GenerationEngine, GenerationParameters, Prompt, parallel
@@ -244,7 +244,7 @@ def timed_broadcast(schema_cache, dev):
 
 
 def c5_block(lm, dev, world, rank, batch=64, pool=64, picks=32, seg_len=256, suffix=32):
-    """Llama-2-7B, a pool of 64 segments x 256 tokens, B=64 prompts each choosing 32 (seed 5) ->
+    """Config C5: Llama-2-7B, a pool of 64 segments x 256 tokens, B=64 prompts each choosing 32 (seed 5) ->
     N=8192 cached tokens + 32-token suffix, sharded b mod G over the ranks.  Timed through the public calls
     (CacheEngine.process + GenerationEngine.generate(max_new_tokens=1)), host id lists in, token out."""
     import random
@@ -311,7 +311,7 @@ def c5_block(lm, dev, world, rank, batch=64, pool=64, picks=32, seg_len=256, suf
 
 
 def family_block(model_key, cfg_name, dev, steps, warmup):
-    """Another model family on the same engine, one request per step.  C4 = BASELINE configs[3]: Falcon-7B at real dims
+    """Another model family on the same engine, one request per step.  C4: Falcon-7B at real dims
     (H=71, Hkv=1, D=64, hidden 4544, 32 layers), parameterized schema: 5 segments = 256 cached tokens, 21-token suffix of
     which 5 sit at interior parameter slots (non-monotone ids).  MPT-7B (ALiBi at key ids, full position ids) is run on
     the C2 schema shape."""
@@ -401,7 +401,7 @@ def attention_point(nat, dev, H, Hkv, D, q, N, peak, tflops_peak, rounding=None,
 
 
 def suffix_sweep(nat, dev, peak, tflops_peak):
-    """q in {16, 64, 256, 1024} over the C2 and C5 cached lengths, no-cache full prefill q=N, and the
+    """The suffix sweep: q in {16, 64, 256, 1024} over the C2 and C5 cached lengths, no-cache full prefill q=N, and the
     Falcon MQA geometry."""
     pts = []
     for (H, Hkv, D, q, N, rnd, tag) in [(32, 32, 128, 16, 2048, None, "C2"), (32, 32, 128, 64, 2048, None, "C2"),
@@ -726,7 +726,7 @@ def main():
         peak, peak_kind, tflops_peak = load_peaks()
         L, Hkv, D = lm.get_cache_shape()
         H = model.n_heads
-        splice_bytes = 8.0 * L * Hkv * case.n_cached * D  # read + write of K and V, fp16 (SURVEY.md section 8d)
+        splice_bytes = 8.0 * L * Hkv * case.n_cached * D  # read + write of K and V, fp16
         attn_bytes = L * (4.0 * Hkv * (case.n_cached + w.q_len) * D + 4.0 * H * w.q_len * D)
         wbytes = weight_bytes(md, model_key)
         step_bytes = (0.0 if w.virtual else splice_bytes) + attn_bytes + wbytes

@@ -36,7 +36,7 @@ enum {
   PC_ERR_WORKSPACE = -4    /* caller-provided workspace too small                      */
 };
 
-/* Rounding points of the reference attention that the kernels reproduce (SURVEY.md section 7):
+/* Rounding points of the reference attention that the kernels reproduce:
  *   PC_ROUND_QK     : Q.K^T is rounded to fp16 before scaling   (llama2.py:371, mpt.py:156 -- fp16 matmul output)
  *   PC_ROUND_SCALED : the scaled score is rounded to fp16       (llama2.py:371 "/ sqrt(d)", mpt.py:156 "* scale")
  * P is always rounded to fp16 before P.V (llama2.py:387, mpt.py:181) and the context to fp16 at the end.
@@ -166,7 +166,7 @@ typedef struct pc_attn_params {
                               * ZERO it once before first use (arrival counters; kernels     *
                               * leave them zeroed); one workspace per concurrent stream      */
   size_t workspace_bytes;
-  /* ---- virtual splice (SURVEY.md section 8 row f2): the copy of PromptCache.update (cache_engine.py:135-151) is
+  /* ---- virtual splice: the copy of PromptCache.update (cache_engine.py:135-151) is
    * not made; the kernel reads the cached keys straight from the schema's segment ARENA through a per-request
    * tile list.  With kv_tiles != NULL the first `kv_rows` of the n_cached keys are NOT read from k/v: they are the
    * `kv_n_tiles` tiles listed in kv_tiles, each {first arena row, valid rows (1..128)} -- one tile never spans two
@@ -195,7 +195,7 @@ int pc_prefill_attn(const pc_attn_params* p, void* stream);
 int pc_decode_attn(const pc_attn_params* p, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
- * Support kernels (SURVEY.md section 8 row a13: not part of the parity scope; they replace ~25 eager
+ * Support kernels (not part of the parity scope; they replace ~25 eager
  * launches per layer so that the TTFT step is not launch-bound).  fp16 tensors, rounding as the reference:
  *   pc_add_rmsnorm: x[rows][hidden] += delta (fp16 add, written back; delta may be NULL), then
  *                   h_out = weight * half(x_f32 * rsqrt(mean(x_f32^2) + eps))   (llama2.py:104-109,636,644)
@@ -220,7 +220,7 @@ int pc_add_rmsnorm_partials(void* x, const void* delta_partials, int n_splits, c
                             int hidden, float eps, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
- * Skinny linear layers of the step (SURVEY.md section 8 row a13): y = x . W^T for q_len <= 32 tokens,
+ * Skinny linear layers of the step: y = x . W^T for q_len <= 32 tokens,
  * one weight-streaming stream-K tcgen05 kernel per layer with the following op fused into its epilogue.
  *   q/k/v projections + RoPE + KV append   llama2.py:345-351,357-364   (PC_LIN_ROPE_APPEND)
  *   o_proj, down_proj, lm_head             llama2.py:405,241,1050      (PC_LIN_PLAIN)

@@ -20,7 +20,7 @@ from oracle import ref_shim  # noqa: E402
 OUT = os.path.join(os.path.dirname(HERE), "tests", "golden")
 
 # no whitespace between elements: a whitespace-only text run would become a zero-token TokenSequence, which the
-# reference cannot encode (cache_engine.py:278 raises) -- see SURVEY.md section 7
+# reference cannot encode (cache_engine.py:278 raises)
 SCHEMA = ('<schema name="demo"><module name="a">alpha beta gamma<parameter name="p" length="3"/>delta</module>'
           '<union><module name="b1">one two three four</module><module name="b2">five six</module></union>'
           '<module name="c">red green blue cyan</module></schema>')

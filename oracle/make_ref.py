@@ -4,7 +4,7 @@
 
 The reference (yale-sys/prompt-cache) is pure Python; "/root/reference" exists only in the build container.  This
 recipe copies its package `promptcache/` and the example schemas `examples/` byte for byte into `oracle/_ref/`
-(git-ignored, NOT gpurun-ignored, so it travels with the snapshot like the built .so) and records a manifest with the
+(git-ignored; it travels with a copy of the tree like the built .so) and records a manifest with the
 SHA-256 of every file.  Nothing is edited: the shims that make it importable under transformers 5 / without lxml live
 in `oracle/ref_shim.py` and `oracle/_shims/`.  On the GPU box `oracle/ref_shim.py` finds `oracle/_ref/` and
   * `bench.py --impl reference` runs the reference's own CacheEngine.process -> GenerationEngine.generate on the host

@@ -16,7 +16,7 @@ from . import ref_shim
 
 def hf_config(arch: str, dims: Dict):
     """transformers config object for the reference's vendored model files, with the attributes transformers 5 dropped
-    restored (SURVEY.md section 8c shim 4/5)."""
+    restored."""
     if arch == "llama":
         from transformers import LlamaConfig
         cfg = LlamaConfig(vocab_size=dims["vocab_size"], hidden_size=dims["hidden_size"],

@@ -1,8 +1,8 @@
 """TEST INFRASTRUCTURE ONLY -- loader for the *unmodified* reference (yale-sys/prompt-cache).
 
 Imports ``promptcache`` from ``oracle/_ref`` (the byte-for-byte copy staged by ``oracle/make_ref.py``; git-ignored,
-travels to the GPU box) or from ``/root/reference`` (build container only) through the shim set of SURVEY.md
-section 8c, so that ``oracle/gen_golden.py`` can freeze the reference's outputs under ``tests/golden/``, the
+travels to the GPU box) or from ``/root/reference`` (build container only) through the shims
+below, so that ``oracle/gen_golden.py`` can freeze the reference's outputs under ``tests/golden/``, the
 ``-m gpu`` tests can run the reference's own modules in fp16 on the B200 next to the CUDA path, and
 ``bench.py --impl reference`` can time the reference's own classes on the host cores.
 

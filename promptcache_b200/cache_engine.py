@@ -9,7 +9,7 @@
   CacheEngine          add_schema / process / remove_schema with the reference's signatures and ValueErrors
                        (reference :331-522)
 
-Deliberate deviations from the reference, both called out in SURVEY.md section 7:
+Deliberate deviations from the reference:
   * `PromptCache.staged` records the layout actually written (the usage-ordered list), so the retained-prefix
     shortcut can never hand back stale rows (the reference stores the unsorted list, :155);
   * zero-length token sequences are skipped instead of raising in `list.index` (:278).
@@ -180,7 +180,7 @@ class PromptCache:
 
         virtual=False: the rows are copied into the contiguous buffer now (one pc_splice_kv launch; with
         `retain_prefix` only the segments behind the longest common prefix with what the buffer already holds).
-        virtual=True ("virtual splice", SURVEY.md 8 f2): nothing is copied.  When every segment lives in ONE arena the
+        virtual=True ("virtual splice"): nothing is copied.  When every segment lives in ONE arena the
         request's tile list {first arena row, valid rows} goes to the device (one small pinned copy) and the short-suffix
         attention kernel reads the segments in place; the copy is made later only if somebody asks for the contiguous
         rows (`materialise`).  Either way rows >= N of the buffer receive the suffix / decode rows in place."""
@@ -374,7 +374,7 @@ class SchemaCache:
                             paths.append(Path(here + [member.name]).next)
         return paths
 
-    reuse_prefix = True  # encode non-default union members over the default scaffold's KV prefix (SURVEY 8f-1)
+    reuse_prefix = True  # encode non-default union members over the default scaffold's KV prefix
 
     def _forward(self, token_ids: List[int], position_ids: List[int], past=None):
         device = self.lm.device
@@ -404,7 +404,7 @@ class SchemaCache:
         `batch_size` paths (pad_batch, :228-248).  Attention is causal, so the KV of a member only depends on the tokens
         before it: with `reuse_prefix` a member's path is encoded as a cached prefill over the longest token/position
         prefix it shares with the default scaffold and stops at the last token the path has to store -- prompt caching
-        applied to its own encoder.  Those member prefills are BATCHED (SURVEY.md 8 f1): the tokens of up to `batch_size`
+        applied to its own encoder.  Those member prefills are BATCHED: the tokens of up to `batch_size`
         members (or `batch_token_budget` tokens when batch_size is 1) go through the model's linears as one
         concatenated sequence -- no padding -- and only RoPE+append / attention run per member, each over its own copy
         of the shared prefix (`forward_many`)."""

@@ -1,5 +1,5 @@
-// A CHAIN of the step's skinny linears and the norms between them as ONE persistent launch (SURVEY.md section 8 row a13;
-// reference promptcache/model/llama2.py:623-648 decoder layer: o_proj -> residual add + post_attention_layernorm -> gate/up
+// A CHAIN of the step's skinny linears and the norms between them as ONE persistent launch (reference
+// promptcache/model/llama2.py:623-648 decoder layer: o_proj -> residual add + post_attention_layernorm -> gate/up
 // -> SiLU*up -> down_proj -> residual add + next input_layernorm -> q/k/v projections + RoPE + KV append).
 //
 // Why: launched one by one (linear_small.cu) every linear pays, per SM, the dead time between its last weight load and

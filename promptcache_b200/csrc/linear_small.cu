@@ -1,5 +1,5 @@
-// Skinny-M linear layers of the prefill / decode step as ONE weight-streaming tcgen05 kernel (SURVEY.md
-// section 8 row a13: q/k/v/o projections, MLP and lm_head -- reference promptcache/model/llama2.py:345-351,
+// Skinny-M linear layers of the prefill / decode step as ONE weight-streaming tcgen05 kernel
+// (q/k/v/o projections, MLP and lm_head -- reference promptcache/model/llama2.py:345-351,
 // :405, :213-244, :1050).  With q <= 32 uncached tokens these GEMMs are pure HBM streams of the fp16 weights
 // (13.5 GB per Llama-2-7B forward, two thirds of the TTFT step) and every epilogue (RoPE + KV append, SiLU*up)
 // used to cost another launch.

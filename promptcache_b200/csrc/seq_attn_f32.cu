@@ -9,7 +9,7 @@
 // from the keys it sees alone (attn_row_again).
 //
 // 8 heads of 128 (B200), against the plain kernel (one block per token and head, every row read again): 1024 tokens 818 -> 103 us (21 TFLOP/s), 2048: 2.92 -> 0.32
-// ms, 64 behind 400 stored 76 -> 21 us, 16 behind 4000 100 -> 69 us.  A cluster shares a walk where there are few blocks (choose_splits).
+// ms, 64 behind 400 stored 76 -> 21 us, 16 behind 4000 473 -> 68 us.  A cluster shares a walk where there are few blocks (choose_splits).
 #include "seq_attn.cuh"
 #include "seq_mma.cuh"
 #include "seq_tc5.cuh"

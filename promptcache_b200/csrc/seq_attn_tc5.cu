@@ -17,9 +17,9 @@
 // 4 or 8 blocks shares the walk over the keys and merges through distributed shared memory.  The choice is a cost model on the host (Plan).
 //
 // What bounds it (B200, bfloat16, 16 heads, dim = vdim = 128): 1.4 us per key tile of both halves, of which the 24 products take 0.95 us at full
-// rate; without any softmax arithmetic the walk takes 1.24 us.  Against the mma.sync kernel it replaces (seq_attn_tc.cu, which still serves wider heads):
-//   2048 new tokens                  120 ->  44 us        6144 and 2311 new tokens          836 -> 247 us (714 TFLOP/s of the two-product count)
-//   256 behind 4000 stored           167 ->  37 us        four continued prompts, window 1024, cap  172 -> 84 us
+// rate; without any softmax arithmetic the walk takes 1.24 us.  Against the mma.sync kernel it replaces (seq_attn_tc.cu, which still serves wider heads and short entries):
+//   2048 new tokens        122 -> 47 us        6144 and 2311 new tokens                      842 -> 286 us (617 TFLOP/s of the two-product count)
+//   256 behind 4000 stored 164 -> 50 us (8 heads 164 -> 27)      four continued prompts, window 1024, cap  177 -> 85 us
 #include "seq_attn.cuh"
 #include "seq_mma.cuh"
 #include "seq_tc5.cuh"

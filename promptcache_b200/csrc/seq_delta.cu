@@ -1543,7 +1543,8 @@ static int launch_delta_chunk_scan(const pcs_delta_chunk_params& p, size_t smem,
 // about 2^-16 of a product); the state itself stays as it is.  [qd | a] is staged in shared memory as such pairs, S and u are read once, a step ahead.
 // Three parts (gated linear attention, whose read-out was a 32-bit product): all 24 bits of qd, a and S (u holds bfloat16 numbers there and is its own first
 // part), six products per step of sixteen terms, the smallest first, and the steps' sums join in rounded additions (the tensor core's running sum cuts
-// bits off).  That takes registers for half of the tokens only: a block of 32 tokens, S is read by two blocks.
+// bits off).  That takes registers for half of the tokens only: a block of 32 tokens, S is read by two blocks.  34 chunks
+// of 4 heads of 256 x 512: 70 us (42 with two parts).
 constexpr int kDoMaxWarps = 16;
 
 template <int PARTS>

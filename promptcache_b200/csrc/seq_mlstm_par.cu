@@ -10,8 +10,8 @@
 // Products are m16n8k16 bfloat16 with 32-bit accumulators; every 32-bit factor enters as hi + lo, as in the serial form.  Bound by the traffic of the
 // states (written twice and read twice, 4 bytes an element; half of it stays in L2) and by the legacy tensor path in `out`.
 //
-// 2048 tokens, 4 heads of 256 x 512 (B200): 304 -> 117 us (gates 6, sums 26, scan 20, out 58); 3900 tokens, 2 heads of 128 x 256: 380 -> 65 us.  `out` with 256
-// threads and operand loads directly before their products took 79 us, with the index divisions of a run-time width 68 us.
+// 2048 tokens, 4 heads of 256 x 512 (B200): 317 -> 123 us (gates 6, sums 26, scan 20, out 63); 3900 tokens, 2 heads of 128 x 256: 377 -> 66 us.  `out` with 256
+// threads and operand loads directly before their products took 21 us more, with the index divisions of a run-time width 10 us more.
 #include "seq_common.cuh"
 #include "seq_mma.cuh"
 

@@ -1,6 +1,6 @@
 // Splice kernel: PromptCache.update (reference promptcache/cache_engine.py:116-156).
 //
-// The splice is L*2*Hkv*M independent contiguous runs (SURVEY.md section 7 "Splice geometry").
+// The splice is L*2*Hkv*M independent contiguous runs.
 // Each run is cut into <=32 KiB tiles; a persistent grid (one CTA per SM) walks the tiles
 // round-robin.  A tile moves global -> shared with one 1-D TMA bulk load (UBLKCP) and shared ->
 // global with one 1-D TMA bulk store: 128 B-coalesced on both sides, no register staging, and a

@@ -1,4 +1,4 @@
-// Support kernels around the hot path (SURVEY.md section 8 row a13: norms / activation are unchanged by
+// Support kernels around the hot path (norms / activation are unchanged by
 // prompt caching and stay outside the parity scope, but as ~25 eager launches per layer they made the
 // TTFT step launch-bound).  Rounding points follow the reference so the residual stream stays within
 // fp16 round-off of promptcache/model/llama2.py:

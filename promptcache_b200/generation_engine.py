@@ -7,7 +7,7 @@ use_full_position_ids)` yields `Output`s exactly like the reference, including i
     `.response_time` is the cumulative model time and `.elapsed_time` the prefill time (:53-58,201).
 What changes is underneath: the KV is appended in place (no torch.cat per step) and every forward runs
 pc_rope_append + pc_prefill_attn / pc_decode_attn.  Greedy decoding without a repetition penalty additionally
-samples ON THE DEVICE (SURVEY.md section 8 row f3): the argmax of a step feeds the next step's graph without going
+samples ON THE DEVICE: the argmax of a step feeds the next step's graph without going
 through the host, and the host reads the pending token ids only where the reference loop would yield
 (`i % stream_interval == 0`, the last step) -- same tokens, same texts, same per-step event times, fewer syncs.
 """

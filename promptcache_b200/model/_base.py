@@ -47,7 +47,7 @@ class B200CausalLM(nn.Module):
         # experiment, off: the linears and norms between two attention launches as ONE persistent launch (pc_linear_chain, grid
         # barriers between the ops).  Measured SLOWER: 106 vs 87 us per Llama-2-7B layer (4.22 vs 3.30 ms per C2 step) -- each
         # of the 5 grid barriers + 2 in-kernel norms of a layer is a chain of L2 round trips under a saturated memory system,
-        # ~33 us of consumer stalls per layer against the ring's 4.3 us of run-ahead (DESIGN.md 4.5)
+        # ~33 us of consumer stalls per layer against the ring's 4.3 us of run-ahead
         self.linear_chain = os.environ.get("PC_LINEAR_CHAIN", "0") != "0"
         # experiment, off: the short-suffix attention kernel asks L2 for the output projection's weight stream once its own K/V
         # loads are out (that projection's CTAs cannot start before the attention CTAs leave their SMs).  Measured same-box:

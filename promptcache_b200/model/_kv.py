@@ -79,7 +79,7 @@ def buffer_of(t: torch.Tensor) -> Optional[KVBuffer]:
 
 
 class VirtualKV:
-    """The cached rows [0, rows) of a KVBuffer that have NOT been copied into it ("virtual splice", SURVEY.md 8 f2):
+    """The cached rows [0, rows) of a KVBuffer that have NOT been copied into it ("virtual splice"):
     they are read in place from the schema's segment arena [L,2,Hkv,R,D] through `tiles` (int32 [T,2] on the device:
     first arena row, valid rows).  `materialise()` makes the copy after all, for consumers that need the contiguous rows
     (long-suffix / ALiBi attention kernels, callers indexing the reference-shaped views)."""

@@ -4,7 +4,7 @@ Same forward signature and outputs as reference promptcache/model/llama2.py (Lla
 :986-1076 -> LlamaModel.forward :822-951 -> LlamaDecoderLayer :600-654 -> LlamaAttention :315-410).
 The per-layer attention core (llama2.py:353-398: RoPE at explicit ids, KV concat, repeat_kv, mask, QK^T,
 softmax, PV, transpose) is TWO kernel launches here -- pc_rope_append and pc_prefill_attn/pc_decode_attn --
-called through the C ABI; projections, norms and the MLP stay torch/cuBLAS (SURVEY.md section 8 row a13).
+called through the C ABI; projections, norms and the MLP stay torch/cuBLAS.
 """
 from __future__ import annotations
 
@@ -157,7 +157,7 @@ class LlamaForCausalLM(B200CausalLM):
 
     @torch.inference_mode()
     def forward_many(self, items, max_position: Optional[int] = None):
-        """Cached prefill of SEVERAL independent sequences in one pass (schema encoding, SURVEY.md 8 f1; the reference
+        """Cached prefill of SEVERAL independent sequences in one pass (schema encoding; the reference
         pads whole scaffolds into a batch instead, cache_engine.py:228-248).  `items` = [(ids [n_b], position ids [n_b],
         past_key_values or None)].  The tokens of all sequences run through the norms / projections / MLP as ONE
         concatenated [sum n_b, hidden] matrix (no padding, one weight stream for all of them); RoPE + append and

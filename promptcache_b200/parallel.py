@@ -1,4 +1,4 @@
-"""Batch partition across the GPUs of one node (SURVEY.md section 8e).
+"""Batch partition across the GPUs of one node.
 
 Prompts are independent, so the hot path shards with NO data-path collective: prompt b is served by rank
 b mod G, every rank holds the full weights and its own HBM copy of the schema's segment store.  NCCL (over

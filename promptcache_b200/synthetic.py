@@ -1,8 +1,7 @@
 """Synthetic schemas and a numeric tokenizer for benchmarks and tests.
 
-There are no tokenizers, weights or datasets on disk (and no network), so the BASELINE configs are
+There are no tokenizers, weights or datasets on disk (and no network), so the configs C1 to C5 are
 realised as PML schemas whose text is made of pseudo-words `t<id>`; `IdTokenizer` maps `t123` <-> 123.
-Shapes follow SURVEY.md section 8d (C1..C5).
 """
 from __future__ import annotations
 
@@ -95,7 +94,7 @@ def pool_prompt(name: str, picks: Sequence[str], suffix: int, vocab: int, seed: 
 
 
 CONFIGS: Dict[str, dict] = {
-    # BASELINE.json configs -> concrete shapes
+    # the configs' concrete shapes
     "C1": dict(model="llama2-7b", desc="persona: 8 segments [24,92x6,24], N=600, q=16, union gaps"),
     "C2": dict(model="llama2-7b", desc="code-generation-game: 7 segments [24,400x5,24], N=2048, q=16"),
     "C3": dict(model="llama2-13b", desc="LongBench multi-doc: 8 segments x512, N=4096, q=32"),
