@@ -327,9 +327,11 @@ int launch_attn_f32(const pcs_attn_params& p, cudaStream_t st, bool* handled) {
   // Few tokens over few keys: a block per token and head begins and ends sooner.  Decoding kernels (a workspace is given) / plain kernel / tiles, B200, us: 16 tokens of 8
   // heads of 128 over 16 keys 6.5 / 10.5 / 12.6, over 66 8.3 / 14.5 / 16.5; 40 over 40 8.5 / 12.4 / 15.2; 24 x 4 entries over 24 - / 10.7 / 12.5, 24 over 72
   // - / 14.6 / 15.9, 16 x 16 entries over 16 - / 16.5 / 12.6; of 12 heads of 64: 16 over 16 - / 8.5 / 10.4, 48 over 48 - / 10.6 / 10.5.
+  // (Rows of more than 128 are not the grouped decoding kernel's: 16 tokens over 1016 keys, 8 heads of 192, a block per head 45, tiles 27.)
   const int keys = p.max_keys > 0 && p.max_keys < p.cap ? p.max_keys : p.cap;
   const long long pairs = static_cast<long long>(p.n_tokens) * p.n_heads;
-  if (p.workspace ? p.n_tokens <= 16 || (static_cast<long long>(keys) * (p.dim + p.vdim) <= 49152 && pairs <= 1024)
+  const bool workspace = p.workspace && p.workspace_floats >= pairs * kAttnMaxSplits * (p.vdim + 2);   // (the decoding kernels refuse one that is too small)
+  if (workspace ? (p.n_tokens <= 16 && p.dim <= 128) || (static_cast<long long>(keys) * (p.dim + p.vdim) <= 49152 && pairs <= 1024)
                   : keys <= (p.dim + p.vdim >= 256 ? 80 : 32) && pairs <= 1024 && pairs * keys <= 32768)
     return PCS_OK;
   const long long grid = (p.max_len + FM - 1LL) / FM * p.n_seqs * p.n_heads;
