@@ -253,7 +253,8 @@ __global__ void __launch_bounds__(F_THREADS) attn_f32_kernel(const __grid_consta
 }
 
 // The blocks of a cluster that share a walk: a key tile costs a block 7 us at dim + vdim = 256 whether it has its SM alone or not (its four warps wait for
-// their own products), set-up and end 3, with a merge 6; a launch of more than one wave ends 15 % behind its average.
+// their own products), set-up and end 3, with a merge 6, 1 less where every block has an SM to itself (64 tokens behind 100, 4 heads of 36: a block per
+// walk 17 us, four 11; with 16 entries, 512 blocks of four, 17 and 26); a launch of more than one wave ends 15 % behind its average.
 int choose_splits(const pcs_attn_params& p, const int (&slots)[4]) {
   const double tile = 7.1 * (p.dim + p.vdim) / 256.0, over[4] = {3.0, 6.0, 6.5, 7.0};
   const int keys = p.max_keys > 0 && p.max_keys < p.cap ? p.max_keys : p.cap, n = (p.max_len + FM - 1) / FM;
@@ -270,7 +271,7 @@ int choose_splits(const pcs_attn_params& p, const int (&slots)[4]) {
   for (int i = 0; i < 4; ++i) {
     const int s = 1 << i;
     if (slots[i] < s) continue;
-    double t = ceil(longest / s) * tile + over[i];   // (a walk of one tile is not shared)
+    double t = ceil(longest / s) * tile + over[i] - (s > 1 && blocks * s <= FSMs);   // (a walk of one tile is not shared)
     if (blocks * s > slots[i]) t = fmax(t, 1.15 * (sum / n * blocks + blocks * s * over[i]) / slots[i]);
     if (t < best) { best = t; splits = s; }
   }
