@@ -1,12 +1,12 @@
 """TEST INFRASTRUCTURE ONLY -- freeze outputs of the UNMODIFIED reference into tests/golden/.
 
-Run in the build container (needs /root/reference):   python oracle/gen_golden.py
+Needs /root/reference:   python oracle/gen_golden.py
 Imports the reference through oracle/ref_shim.py, runs its own classes on CPU with seeded tiny models and
 writes
   tests/golden/llama_tiny.pt     state dict, schema/prompt XML, plans (cached / no_cache / full ids), the spliced
                                  PromptCache contents, per-segment KV, prefill logits and greedy decode ids
   tests/golden/attn_cores.pt     inputs/outputs of the reference attention modules (Llama fp32+fp16, Falcon, MPT)
-The GPU box has no /root/reference; tests read only these files.
+Tests read only these files.
 """
 import os
 import sys

@@ -1,12 +1,12 @@
-"""TEST INFRASTRUCTURE ONLY -- stage the UNMODIFIED reference where the GPU box can see it.
+"""TEST INFRASTRUCTURE ONLY -- stage the UNMODIFIED reference inside the tree.
 
     python oracle/make_ref.py            (also called by __graft_entry__.build() when /root/reference is mounted)
 
-The reference (yale-sys/prompt-cache) is pure Python; "/root/reference" exists only in the build container.  This
+The reference (yale-sys/prompt-cache) is pure Python; "/root/reference" exists only where it is mounted.  This
 recipe copies its package `promptcache/` and the example schemas `examples/` byte for byte into `oracle/_ref/`
 (git-ignored; it travels with a copy of the tree like the built .so) and records a manifest with the
 SHA-256 of every file.  Nothing is edited: the shims that make it importable under transformers 5 / without lxml live
-in `oracle/ref_shim.py` and `oracle/_shims/`.  On the GPU box `oracle/ref_shim.py` finds `oracle/_ref/` and
+in `oracle/ref_shim.py` and `oracle/_shims/`.  Elsewhere `oracle/ref_shim.py` finds `oracle/_ref/` and
   * `bench.py --impl reference` runs the reference's own CacheEngine.process -> GenerationEngine.generate on the host
     cores (`cpu_baseline.kind == "reference"`),
   * the `-m gpu` tests run the reference's own attention modules / models in fp16 ON THE B200 beside the CUDA path.
@@ -35,7 +35,7 @@ def _sha(path: str) -> str:
 
 def make_ref(verbose: bool = False) -> str:
     """Copy the reference package into oracle/_ref/ (idempotent).  Returns the destination, or '' when the source is
-    absent (GPU box: the prebuilt copy that travelled with the snapshot is used as is)."""
+    absent (then the copy staged before is used as is)."""
     if not os.path.isdir(os.path.join(SRC, "promptcache")):
         return DST if os.path.isdir(os.path.join(DST, "promptcache")) else ""
     manifest = {}

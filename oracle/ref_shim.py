@@ -1,7 +1,7 @@
 """TEST INFRASTRUCTURE ONLY -- loader for the *unmodified* reference (yale-sys/prompt-cache).
 
-Imports ``promptcache`` from ``oracle/_ref`` (the byte-for-byte copy staged by ``oracle/make_ref.py``; git-ignored,
-travels to the GPU box) or from ``/root/reference`` (build container only) through the shims
+Imports ``promptcache`` from ``oracle/_ref`` (the byte-for-byte copy staged by ``oracle/make_ref.py``; git-ignored)
+or from ``/root/reference`` through the shims
 below, so that ``oracle/gen_golden.py`` can freeze the reference's outputs under ``tests/golden/``, the
 ``-m gpu`` tests can run the reference's own modules in fp16 on the B200 next to the CUDA path, and
 ``bench.py --impl reference`` can time the reference's own classes on the host cores.
@@ -30,8 +30,8 @@ _SHIMS = os.path.join(_HERE, "_shims")
 
 
 def _find_reference() -> str:
-    """PC_REFERENCE_ROOT, else the staged byte-for-byte copy oracle/_ref (made by oracle/make_ref.py; the only one
-    that exists on the GPU box), else the read-only mount of the build container."""
+    """PC_REFERENCE_ROOT, else the staged byte-for-byte copy oracle/_ref (made by
+    oracle/make_ref.py), else the read-only mount."""
     for cand in (os.environ.get("PC_REFERENCE_ROOT"), os.path.join(_HERE, "_ref"), "/root/reference"):
         if cand and os.path.isdir(os.path.join(cand, "promptcache")):
             return cand

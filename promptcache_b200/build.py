@@ -3,7 +3,7 @@
 `python -m promptcache_b200.build` or `build()` builds libpromptcache_b200.so (the prompt-cache hot path);
 `build_seq()` builds libpromptcache_b200_seq.so (the sequence-batch kernels: slot-pool attention, recurrent scan, gated
 norms), which is all a model of that family needs -- a first run in a fresh checkout compiles only the library its model
-loads.  nvcc cross-compiles without a GPU.  The .so files are git-ignored but travel to the GPU box with the snapshot.
+loads.  nvcc cross-compiles without a GPU.  The .so files are git-ignored.
 """
 from __future__ import annotations
 

@@ -1,5 +1,5 @@
 """Shared test helpers: the deterministic toy tokenizer (same algorithm as oracle/ref_shim.WordTokenizer, restated
-here so the GPU box needs nothing from the reference) and golden loading."""
+here so that nothing of the reference is needed) and golden loading."""
 import os
 
 import torch

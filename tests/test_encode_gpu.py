@@ -1,5 +1,5 @@
 """Schema encoding (SchemaCache._process, reference cache_engine.py:186-307): union members are encoded as BATCHED cached
-prefills over the default scaffold's prefix (SURVEY.md 8 f1) and must store the same KV as the reference's way of doing
+prefills over the default scaffold's prefix and must store the same KV as the reference's way of doing
 it -- one whole-scaffold forward per member."""
 import pytest
 import torch

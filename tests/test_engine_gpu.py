@@ -114,7 +114,7 @@ def test_full_position_ids_and_no_cache(native, gold):
 
 
 def test_usage_reorder_and_retained_prefix_never_serve_stale_rows(native, gold):
-    """The latent `staged` bug of the reference (SURVEY.md section 7) must not be reproduced."""
+    """The latent `staged` bug of the reference must not be reproduced."""
     from promptcache_b200 import CacheEngine, Prompt
     lm = _tiny_lm(gold, native)
     eng = CacheEngine(64, lm)

@@ -200,7 +200,7 @@ def test_attention_llama_rounding(native, impl, H, Hkv, D, q, N):
                      impl=native.PC_ATTN_SIMT if impl == "simt" else native.PC_ATTN_TCGEN05, decode=(q == 1))
     torch.cuda.synchronize()
     ref = _oracle_llama(Q, K, V, N, q)
-    # north_star tolerance: 1e-3 fp16-relative against the reference's own (rounding) attention path
+    # tolerance: 1e-3 fp16-relative against the reference's own (rounding) attention path
     assert _rel(out, ref) <= 1e-3, _rel(out, ref)
     assert torch.allclose(out.float(), ref.float(), rtol=1e-3, atol=1e-3)
 
@@ -327,7 +327,7 @@ def test_attention_runtime_length_equals_host_length(native):
 ])
 def test_attention_cluster_merge_equals_global_merge(native, monkeypatch, H, Hkv, q, N):
     """Split-KV merge through the cluster leader's shared memory (DSMEM) vs through global partials + arrival counter:
-    same partials, same summation order -> the same bits; both within the north-star tolerance of the reference."""
+    same partials, same summation order -> the same bits; both within 1e-3 of the reference."""
     D = 128
     Q, K, V = _attn_case(H, Hkv, D, q, N, seed=H + q + N, std=1.28)
     ws = torch.zeros(max(native.attn_workspace_bytes(H, q, D), 1), dtype=torch.uint8, device=DEV)

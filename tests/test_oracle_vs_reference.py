@@ -1,5 +1,5 @@
 """Live cross-check of the oracle and of the product front-end against the unmodified reference.  Runs only where
-/root/reference is mounted (the build container); the GPU box relies on the goldens generated from it."""
+/root/reference is mounted; elsewhere the goldens generated from it stand in."""
 import pytest
 import torch
 

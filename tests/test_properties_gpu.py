@@ -1,4 +1,4 @@
-"""Size-independent properties at BASELINE.json's full sizes (where the oracle would take too long or too much
+"""Size-independent properties at full sizes (where the oracle would take too long or too much
 memory): checksums, idempotence, linearity, row-stochasticity."""
 import math
 

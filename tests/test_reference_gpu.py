@@ -1,16 +1,16 @@
-"""GPU parity against the UNMODIFIED reference running in fp16 ON THE SAME B200 (SURVEY.md section 8c-ii).
+"""GPU parity against the UNMODIFIED reference running in fp16 ON THE SAME B200.
 
-The reference package is the byte-for-byte copy `oracle/make_ref.py` stages under `oracle/_ref/` (git-ignored, travels
-with the gpurun snapshot); it is imported through `oracle/ref_shim.py`.  Here the reference's own modules
+The reference package is the byte-for-byte copy `oracle/make_ref.py` stages under `oracle/_ref/` (git-ignored);
+it is imported through `oracle/ref_shim.py`.  Here the reference's own modules
 (`LlamaAttention`, `FalconAttention`, `MptAttention`) and whole models / engines run at REAL head geometry beside the
 CUDA path on the same weights and inputs:
-  * attention modules: context (input of the output projection) within 1e-3 relative -- the north-star tolerance --
+  * attention modules: context (input of the output projection) within 1e-3 relative
     and the appended K rows bit-exact (RoPE at discontiguous ids);
-  * Falcon-7B dims (H=71, Hkv=1, D=64, hidden 4544), 2 layers, BASELINE config C4 end to end through both engines:
+  * Falcon-7B dims (H=71, Hkv=1, D=64, hidden 4544), 2 layers, end to end through both engines:
     plans exact, segment KV, prefill logits, greedy token;
-  * Llama-2-7B FULL depth (32 layers) on BASELINE config C2 through both engines: plans exact, logits at the fp16
+  * Llama-2-7B FULL depth (32 layers) through both engines: plans exact, logits at the fp16
     noise floor (the CUDA path is as close to the reference-in-fp32 as the reference-in-fp16 is).
-Skipped when the staged reference is missing (never the case after `__graft_entry__.build()` in the build container).
+Skipped when the staged reference is missing (never the case after `__graft_entry__.build()`).
 """
 import math
 
@@ -201,7 +201,7 @@ def test_mpt_attention_module_fp16_on_device(native, N, q):
 
 
 # ---------------------------------------------------------------------------------------------------------------------
-# whole engines at real dims: BASELINE config C4 (Falcon-7B dims) and C2 (Llama-2-7B, full depth)
+# whole engines at real dims: Falcon-7B dims and Llama-2-7B at full depth
 # ---------------------------------------------------------------------------------------------------------------------
 def _both_engines(arch, dims, case, max_ctx, ref_dtype=torch.float16):
     """(reference lm + engine on the GPU, CUDA-path lm + engine) holding the same weights and the same schema."""
@@ -238,7 +238,7 @@ def _prefill_logits(lm, ids, pos, cache):
 
 
 def test_c4_falcon7b_dims_parameterized_schema_end_to_end(native):
-    """BASELINE configs[3]: Falcon-7B geometry (2 layers), travel-like schema with parameter slots -> 5 interior-position
+    """Falcon-7B geometry (2 layers), travel-like schema with parameter slots -> 5 interior-position
     suffix tokens + 16 trailing (non-monotone ids), MQA cache shape (L, 1, 64) (model/__init__.py:256-258)."""
     from promptcache_b200 import Prompt
     from promptcache_b200.synthetic import MODEL_DIMS, make_case
@@ -261,7 +261,7 @@ def test_c4_falcon7b_dims_parameterized_schema_end_to_end(native):
 
 
 def test_c2_llama7b_full_depth_logits_at_the_fp16_noise_floor(native):
-    """BASELINE configs[1] at FULL depth (32 layers, real dims) through both engines.  fp16 end-to-end logits of two
+    """Llama-2-7B at FULL depth (32 layers, real dims) through both engines.  fp16 end-to-end logits of two
     different-but-equivalent pipelines differ by rounding noise that grows with depth, so the bar is the noise floor
     itself: the CUDA path must be as close to the reference run in fp32 as the reference run in fp16 is (x1.5), and
     within 2.5 noise floors of the fp16 reference; the greedy token must agree with the fp32 reference whenever the

@@ -1,8 +1,8 @@
-"""Virtual splice (SURVEY.md section 8 row f2): the short-suffix attention kernel reads the cached segments in place from
+"""Virtual splice: the short-suffix attention kernel reads the cached segments in place from
 the schema's arena through a per-request tile list instead of from a copy (reference copy loop:
 promptcache/cache_engine.py:135-151).  Checked against (a) the copied path of the same kernel -- bit-identical whenever
 the segment lengths are multiples of the 128-key tile, because the tiles are then the same -- and (b) the oracle's eager
-attention over the oracle's spliced cache within the north-star tolerance; plus the engine-level behaviour: no splice
+attention over the oracle's spliced cache within 1e-3; plus the engine-level behaviour: no splice
 launch on the engine's own path, lazy materialisation when a caller looks at the reference-shaped views, staleness."""
 import pytest
 import torch

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""eval_sys-style system evaluation on the B200 path (SURVEY.md section 8 row f4; reference eval_sys.py:88-215, :300-375).
+"""eval_sys-style system evaluation on the B200 path (reference eval_sys.py:88-215, :300-375).
 
     python tools/eval_sys.py critical_point [--model llama2-7b] [--out gpurun_out/eval_sys_critical_point.json]
     python tools/eval_sys.py latency        [--model llama2-7b] [--out gpurun_out/eval_sys_latency.json]
