@@ -203,6 +203,8 @@ int pc_decode_attn(const pc_attn_params* p, void* stream);
 int pc_add_rmsnorm(void* x, const void* delta, const void* weight, void* h_out, int rows, int hidden,
                    float eps, void* stream);
 int pc_silu_mul(const void* gate_up, void* out, int rows, int inter, int64_t row_stride, void* stream);
+/* dst[i] = (float)src[i], i < n (fp16 -> fp32, exact); both 16-byte aligned */
+int pc_half_to_float(const void* src, void* dst, int64_t n, void* stream);
 /* LayerNorm families (Falcon, MPT): x[rows][hidden] = half(x + half(d1 + d2)) written back (d1 / d2 may be NULL: no add), then
  * h_out = half(((x - mean) * rstd) * weight + bias) with fp32 statistics -- F.layer_norm on fp16 input; bias may be NULL.
  *   Falcon  x + (mlp_out += attn_out), next input_layernorm   falcon.py:781,796-810

@@ -29,7 +29,7 @@ PC_ATTN_GLOBAL_MERGE = 0x100
 
 EXPORTS = ("pc_version", "pc_last_error", "pc_device_info", "pc_splice_kv", "pc_splice_kv_strided", "pc_splice_kv_tensors",
            "pc_rope_append", "pc_rope_append_dyn", "pc_attn_workspace_bytes", "pc_prefill_attn", "pc_decode_attn", "pc_launch_count",
-           "pc_add_rmsnorm", "pc_add_layernorm", "pc_add_layernorm_partials", "pc_silu_mul", "pc_linear_workspace_bytes", "pc_linear_small",
+           "pc_add_rmsnorm", "pc_add_layernorm", "pc_add_layernorm_partials", "pc_silu_mul", "pc_half_to_float", "pc_linear_workspace_bytes", "pc_linear_small",
            "pc_linear_tiled_bytes", "pc_linear_tile_weights", "pc_linear_partial_splits", "pc_add_rmsnorm_partials", "pc_linear_chain")
 PC_CHAIN_LINEAR = 0
 PC_CHAIN_ADD_RMSNORM = 1
@@ -140,6 +140,8 @@ def load() -> C.CDLL:
     lib.pc_linear_chain.restype = C.c_int
     lib.pc_silu_mul.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int64, C.c_void_p]
     lib.pc_silu_mul.restype = C.c_int
+    lib.pc_half_to_float.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]
+    lib.pc_half_to_float.restype = C.c_int
     lib.pc_linear_workspace_bytes.argtypes = []
     lib.pc_linear_workspace_bytes.restype = C.c_size_t
     lib.pc_linear_small.argtypes = [C.POINTER(pc_linear_params), C.c_void_p]
@@ -498,6 +500,16 @@ def silu_mul(gate_up: torch.Tensor, out: torch.Tensor, inter: int) -> None:
         raise NativeError("silu_mul: tensors must be fp16 with contiguous rows")
     _check(load().pc_silu_mul(gate_up.data_ptr(), out.data_ptr(), gate_up.shape[0], inter, gate_up.stride(0), _stream_flush()),
            "pc_silu_mul")
+
+
+def half_to_float(x: torch.Tensor) -> torch.Tensor:
+    """A float32 copy of a contiguous fp16 tensor."""
+    _require_cuda(x)
+    if x.dtype != torch.float16 or not x.is_contiguous() or x.data_ptr() % 16 != 0:
+        return x.float()
+    out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+    _check(load().pc_half_to_float(x.data_ptr(), out.data_ptr(), x.numel(), _stream_flush()), "pc_half_to_float")
+    return out
 
 
 def linear_workspace(device) -> torch.Tensor:

@@ -107,6 +107,7 @@ class B200CausalLM(nn.Module):
 
     # ---- forward ---------------------------------------------------------------------------------------
     def _layers(self, ids: torch.Tensor, pos: torch.Tensor, kv, extra) -> torch.Tensor:
+        """The logits as the last linear leaves them (fp16); `_forward_one` widens them, as the reference does (llama2.py:1048)."""
         raise NotImplementedError
 
     def _graph_extra(self, pos_host_max: int):
@@ -181,7 +182,7 @@ class B200CausalLM(nn.Module):
             graph = torch.cuda.CUDAGraph()
             before = nat.launch_count()
             with torch.cuda.graph(graph):
-                s_logits = self._layers(s_ids, s_pos, kv, (), n_dev=s_n)
+                s_logits = nat.half_to_float(self._layers(s_ids, s_pos, kv, (), n_dev=s_n))
             entry = (graph, s_ids, s_pos, s_n, s_logits, nat.launch_count() - before)
             self._graphs[key] = entry
         graph, s_ids, s_pos, s_n, s_logits, n_native = entry
@@ -230,8 +231,9 @@ class B200CausalLM(nn.Module):
                 graph.replay()
                 nat.note_replayed_launches(n_native)
                 kv.wrote(N + q_len)
-                return (s_logits if static_ok else s_logits.clone()), (kv.views(N + q_len) if use_cache else None)
-        logits = self._layers(ids, pos, kv, extra)
+                # (the widened copy is the caller's own, so the graph's buffer needs no other one)
+                return nat.half_to_float(s_logits), (kv.views(N + q_len) if use_cache else None)
+        logits = nat.half_to_float(self._layers(ids, pos, kv, extra))
         kv.wrote(N + q_len)
         return logits, (kv.views(N + q_len) if use_cache else None)
 

@@ -157,5 +157,5 @@ class FalconForCausalLM(B200CausalLM):
             logits = torch.empty(q_len, self.vocab_size, dtype=torch.float16, device=self.device)
             nat.linear_small(ln, self.word_embeddings, logits, lws,
                              w_tiled=self._wt(("lm_head", 0), self.word_embeddings, nat.PC_LIN_PLAIN))
-            return logits.float()
-        return F.linear(ln, self.word_embeddings).float()
+            return logits
+        return F.linear(ln, self.word_embeddings)

@@ -153,7 +153,7 @@ class LlamaForCausalLM(B200CausalLM):
         logits = torch.zeros(q_len, self.vocab_size, dtype=torch.float16, device=self.device)
         if "linear" not in ab:
             nat.linear_small(h, self.lm_head, logits, lws, w_tiled=self._wt(("lm_head", 0), self.lm_head, nat.PC_LIN_PLAIN))
-        return logits.float()
+        return logits
 
     @torch.inference_mode()
     def forward_many(self, items, max_position: Optional[int] = None):
@@ -322,5 +322,5 @@ class LlamaForCausalLM(B200CausalLM):
                 logits = torch.empty(q_len, self.vocab_size, dtype=torch.float16, device=self.device)
                 nat.linear_small(h, self.lm_head, logits, lws, w_tiled=self._wt(("lm_head", 0), self.lm_head, nat.PC_LIN_PLAIN))
         if lin_head:
-            return logits.float()
-        return F.linear(h, self.lm_head).float()
+            return logits
+        return F.linear(h, self.lm_head)

@@ -171,5 +171,5 @@ class MptForCausalLM(B200CausalLM):
         if lin:
             logits = torch.empty(q_len, self.vocab_size, dtype=torch.float16, device=self.device)
             nat.linear_small(ln, self.wte, logits, lws, w_tiled=self._wt(("lm_head", 0), self.wte, nat.PC_LIN_PLAIN))
-            return logits.float()
-        return F.linear(ln, self.wte).float()
+            return logits
+        return F.linear(ln, self.wte)

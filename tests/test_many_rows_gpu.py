@@ -1,0 +1,56 @@
+"""Kernels of the long-suffix path that take another form for many rows or for aligned ones: the residual add with its norm (more than one row per SM, every
+number of register pieces), the rotation in 16-byte pieces against rows that are only 4-byte aligned, and the widening of logits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("rows", [148, 149, 700])
+@pytest.mark.parametrize("hidden", [8, 1024, 1032, 2048, 2056, 4096, 8192, 8200])
+@pytest.mark.parametrize("with_delta", [False, True])
+def test_add_rmsnorm(rows, hidden, with_delta):
+    from promptcache_b200 import _native as nat
+    g = torch.Generator(device=DEV).manual_seed(rows + hidden)
+    x, d = (torch.randn(rows, hidden, generator=g, device=DEV).half() for _ in range(2))
+    w, h, want_x = (1 + 0.1 * torch.randn(hidden, generator=g, device=DEV)).half(), torch.empty(rows, hidden, device=DEV, dtype=torch.half), x.clone()
+    if with_delta:
+        want_x = (want_x.float() + d.float()).half()
+    y = want_x.double() * torch.rsqrt(want_x.double().pow(2).mean(-1, keepdim=True) + 1e-5)
+    nat.add_rmsnorm(x, d if with_delta else None, w, h, 1e-5)
+    assert torch.equal(x, want_x)
+    # two roundings to fp16 (2^-11 each) of the 32-bit value, and that value's own error
+    want = y * w.double()
+    assert bool(((h.double() - want).abs() <= want.abs() * 2 ** -9.9 + 1e-7).all())
+
+
+@pytest.mark.parametrize("H,Hkv,D,q", [(32, 32, 128, 70), (4, 1, 64, 3), (3, 3, 16, 17), (71, 1, 64, 150), (2, 2, 80, 5), (2, 1, 8, 9)])
+@pytest.mark.parametrize("rotary", [False, True])
+def test_rope_pieces(H, Hkv, D, q, rotary):
+    """The same rows, aligned and shifted by two numbers: bit for bit the same."""
+    from promptcache_b200 import _native as nat
+    g = torch.Generator(device=DEV).manual_seed(D + q)
+    width, rows, max_ctx = (H + 2 * Hkv) * D, 400, q + 21
+    qkv = torch.randn(q, width, generator=g, device=DEV).half()
+    pos = torch.randint(0, rows, (q,), generator=g, device=DEV) if rotary else None
+    cos, sin = (torch.randn(rows, D, generator=g, device=DEV).half() if rotary else None for _ in range(2))
+    got = []
+    for shift in (0, 2):
+        wide = torch.zeros(q, width + 8, device=DEV, dtype=torch.half)
+        src = wide[:, shift:shift + width]
+        src.copy_(qkv)
+        out = [torch.zeros(n, device=DEV, dtype=torch.half) for n in (H * q * D, Hkv * max_ctx * D, Hkv * max_ctx * D)]
+        qo, k, v = out[0].view(H, q, D), out[1].view(Hkv, max_ctx, D), out[2].view(Hkv, max_ctx, D)
+        nat.rope_append(src[:, :H * D], src[:, H * D:(H + Hkv) * D], src[:, (H + Hkv) * D:], pos, cos, sin, qo, k, v, 13, H, Hkv, D)
+        got.append(out)
+    for a, b in zip(*got):
+        assert torch.equal(a, b) and bool((a != 0).any())
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 2047, 2049, 148 * 16 * 2048 + 5])
+def test_half_to_float(n):
+    from promptcache_b200 import _native as nat
+    x = torch.randn(n, device=DEV).half()
+    assert torch.equal(nat.half_to_float(x), x.float())
+    assert torch.equal(nat.half_to_float(x[1:]), x[1:].float())   # (not 16-byte aligned)
