@@ -66,7 +66,7 @@
 extern "C" {
 #endif
 
-#define PCS_ABI_VERSION 8
+#define PCS_ABI_VERSION 9
 #define PCS_BF16 0
 #define PCS_F32 1
 
@@ -177,10 +177,15 @@ typedef struct pcs_attn_params {
   float out_scale;          /* the result is multiplied by this before it is rounded (0 counts as 1) */
   int32_t reserved;
   int64_t out_stride;       /* elements between the result rows of neighbouring tokens (0: H * vdim) */
+  float* prompt_scratch;    /* fp32 scratch of pcs_attn_prompt_scratch_wanted() elements, 16-byte aligned, used by this launch alone until it has ended, or
+                               NULL: with it the walks of a prompt are cut into runs of equal length, without it a block or a cluster has one */
+  int64_t prompt_scratch_floats;
 } pcs_attn_params;        /* (head_scale to out_stride: not with `talk`) */
 /* scratch the key split of pcs_attn needs for n_tokens tokens */
 int64_t pcs_attn_workspace_floats(int n_tokens, int n_heads, int vdim);
 int pcs_attn(const pcs_attn_params* p, void* stream);
+/* the prompt scratch this call would make use of (its prompt_scratch is not read): 0 where it takes another form or kernel.  Under stream capture it is not used. */
+int64_t pcs_attn_prompt_scratch_wanted(const pcs_attn_params* p);
 /* blocks of the tcgen05 prompt kernel that gave up a wait, since the library was loaded (0 in a working system); synchronises.  A wait tries some
  * 2^22 times; the rows of a block that gave up are formed from their keys without the tensor cores, so results stay right. */
 int pcs_attn_timeouts(void);

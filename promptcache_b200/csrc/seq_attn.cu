@@ -472,6 +472,7 @@ PCS_API int pcs_qk_prep(const pcs_qkprep_params* p, void* stream) {
 namespace pcs {
 int launch_attn_tc(const pcs_attn_params& p, cudaStream_t st, bool* handled);
 int launch_attn_tc5(const pcs_attn_params& p, cudaStream_t st, bool* handled);
+int launch_attn_tc5w(const pcs_attn_params& p, cudaStream_t st, bool* handled, long long* wanted);
 int launch_attn_f32(const pcs_attn_params& p, cudaStream_t st, bool* handled);
 int launch_attn_group_decode(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
 int launch_attn_latent(const pcs_attn_params& p, cudaStream_t st, int* splits_out);
@@ -511,6 +512,8 @@ PCS_API int pcs_attn(const pcs_attn_params* p, void* stream) {
   const bool automatic = p->impl == 0 || p->impl == 3;
   if (automatic) {
     bool handled = false;
+    if (int rc = pcs::launch_attn_tc5w(*p, st, &handled, nullptr)) return rc;
+    if (handled) return PCS_OK;
     if (int rc = pcs::launch_attn_tc5(*p, st, &handled)) return rc;
     if (handled) return PCS_OK;
     if (int rc = pcs::launch_attn_f32(*p, st, &handled)) return rc;

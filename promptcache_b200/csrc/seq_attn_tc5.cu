@@ -694,12 +694,15 @@ int launch_attn_tc5(const pcs_attn_params& p, cudaStream_t st, bool* handled) {
   return launch_opt<192, 128>(p, st);
 }
 
+int attn_tc5w_timeouts_so_far();   // of the form for much work
+
 }  // namespace pcs
 
 // blocks of the tcgen05 attention kernel one of whose bounded waits ran out so far (0 in a working system; their rows were formed without tensor cores);
 // synchronises
 PCS_API int pcs_attn_timeouts(void) {
   int n = -1;
-  if (cudaMemcpyFromSymbol(&n, pcs::attn_tc5_timeouts, sizeof(n)) != cudaSuccess) return -1;
-  return n;
+  const int more = pcs::attn_tc5w_timeouts_so_far();
+  if (more < 0 || cudaMemcpyFromSymbol(&n, pcs::attn_tc5_timeouts, sizeof(n)) != cudaSuccess) return -1;
+  return n + more;
 }

@@ -1,0 +1,126 @@
+"""Prompt attention of much work (runs of equal length over the tiles of all items): entries whose tiles end anywhere, every option, rows that hide NaN, two
+streams at once, a captured launch (which takes the other form), and waits that run out."""
+import math
+import multiprocessing
+import traceback
+
+import pytest
+import torch
+
+from tests.test_attention_bias_table_gpu import BF16, DEV, F64, bound, nsq, reference  # noqa: F401  (nsq: the fixture)
+
+pytestmark = pytest.mark.gpu
+SHAPES = [  # heads, kv heads, dim, vdim, new tokens, stored tokens: more than ten key tiles of 128 per SM
+    (8, 2, 128, 128, (3601,), (0,)),
+    (12, 6, 72, 80, (130, 1, 2500, 257, 128), (700, 3000, 1024, 64, 0)),
+    (8, 4, 192, 128, (1921, 1200), (1333, 2000)),
+    (16, 1, 136, 72, (1999, 640), (1, 2048)),
+]
+
+
+def options(H, T, g):
+    dist = torch.arange(900, device=DEV).float()
+    table = (torch.randn(H, 1, generator=g, device=DEV) * 0.3 - 0.2 * torch.log1p(dist / 8)).contiguous()
+    return [{}, dict(softcap=20.0, window=2048, keep_first=70), dict(chunk=3000, bias_table=table), dict(bias_table=table, softcap=9.0),
+            dict(head_scale=-(torch.rand(H, generator=g, device=DEV) + 0.5))]
+
+
+def inputs(H, G, D, V, lens, pos0, seed=3):
+    g = torch.Generator(device=DEV).manual_seed(seed + D + H)
+    T, B, cap = sum(lens), len(lens), (max(n + p for n, p in zip(lens, pos0)) + 127) // 128 * 128
+    q = (torch.randn(T, H * D, generator=g, device=DEV) * 2).to(BF16)
+    k, v = torch.randn(B, G, cap, D, generator=g, device=DEV).to(BF16), torch.randn(B, G, cap, V, generator=g, device=DEV).to(BF16)
+    return g, q, k, v
+
+
+def check(out, q, k, v, H, G, D, V, lens, pos0, o):
+    off = 0
+    for b, (n, p) in enumerate(zip(lens, pos0)):
+        for h in range(H):
+            kk, vv = k[b, h * G // H, :n + p].to(F64), v[b, h * G // H, :n + p].to(F64)
+            want = reference(q[off:off + n, h * D:(h + 1) * D].to(F64), kk, vv, p, D ** -0.5, h, o)
+            got = out[off:off + n, h * V:(h + 1) * V].to(F64)
+            assert bool(((got - want).abs() <= bound(want, vv, BF16)).all()), (H, D, list(o), b, h)
+        off += n
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_every_option(nsq, shape):  # noqa: F811
+    H, G, D, V, lens, pos0 = shape
+    g, q, k, v = inputs(*shape)
+    batch = nsq.Batch(range(len(lens)), pos0, lens, torch.device(DEV))
+    for o in options(H, sum(lens), g):
+        out = torch.full((sum(lens), H * V), 7.0, device=DEV, dtype=BF16)
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        nsq.attention(q, k, v, out, H, D ** -0.5, None, None, False, batch, **o)
+        assert torch.cuda.max_memory_allocated() - before > 148 * 2 * 128 * 128 * 4   # the scratch: the form that is tested here
+        check(out, q, k, v, H, G, D, V, lens, pos0, o)
+        again = torch.full_like(out, 7.0)
+        nsq.attention(q, k, v, again, H, D ** -0.5, None, None, False, batch, **o)
+        assert torch.equal(out, again)
+
+
+def test_hidden_rows_that_are_not_finite(nsq):  # noqa: F811
+    H, G, D, V, lens, pos0 = SHAPES[0]
+    _, q, k, v = inputs(*SHAPES[0])
+    batch, key = nsq.Batch([0], pos0, lens, torch.device(DEV)), 2077
+    out, clean = (torch.full((lens[0], H * V), 7.0, device=DEV, dtype=BF16) for _ in range(2))
+    nsq.attention(q, k, v, clean, H, D ** -0.5, None, None, False, batch)
+    k[0, :, key, 3], v[0, :, key + 1] = math.nan, math.inf
+    nsq.attention(q, k, v, out, H, D ** -0.5, None, None, False, batch)
+    assert bool(((out[:key].double() - clean[:key].double()).abs() <= bound(clean[:key].double(), v[0, :, :key].double(), BF16)).all()) and not bool(out[key:].isfinite().any())
+
+
+def test_streams_and_capture(nsq):  # noqa: F811
+    H, G, D, V, lens, pos0 = SHAPES[2]
+    _, q, k, v = inputs(*SHAPES[2])
+    batch = nsq.Batch(range(len(lens)), pos0, lens, torch.device(DEV))
+    call = lambda out: nsq.attention(q, k, v, out, H, D ** -0.5, None, None, False, batch, softcap=25.0)
+    want = torch.empty(sum(lens), H * V, device=DEV, dtype=BF16)
+    call(want)
+    outs, streams = [torch.zeros_like(want) for _ in range(6)], [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for i, out in enumerate(outs):
+        with torch.cuda.stream(streams[i % 2]):
+            call(out)
+    torch.cuda.synchronize()
+    assert all(torch.equal(out, want) for out in outs)
+    graph, out = torch.cuda.CUDAGraph(), torch.zeros_like(want)
+    with torch.cuda.graph(graph):
+        call(out)
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        check(out, q, k, v, H, G, D, V, lens, pos0, dict(softcap=25.0))
+
+
+def _run(queue):
+    from promptcache_b200 import _native_seq as nsq
+    try:
+        counts = []
+        for shape in SHAPES[:2]:
+            H, G, D, V, lens, pos0 = shape
+            g, q, k, v = inputs(*shape)
+            batch = nsq.Batch(range(len(lens)), pos0, lens, torch.device(DEV))
+            for o in options(H, sum(lens), g)[:2]:
+                for impl in (3, 0):
+                    out = torch.full((sum(lens), H * V), 7.0, device=DEV, dtype=BF16)
+                    nsq.attention(q, k, v, out, H, D ** -0.5, None, None, False, batch, impl=impl, **o)
+                    counts.append(nsq.load().pcs_attn_timeouts())
+                    check(out, q, k, v, H, G, D, V, lens, pos0, o)
+        queue.put(counts)
+    except BaseException:
+        queue.put(traceback.format_exc())
+
+
+def test_waits_that_run_out():
+    ctx = multiprocessing.get_context("spawn")
+    queue = ctx.Queue()
+    child = ctx.Process(target=_run, args=(queue,))
+    child.start()
+    counts = queue.get(timeout=240)
+    child.join(60)
+    assert isinstance(counts, list), counts
+    assert counts[::2] == counts[1::2] and all(a < b for a, b in zip([0] + counts[::2], counts[::2]))
