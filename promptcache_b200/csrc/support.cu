@@ -162,8 +162,6 @@ add_rmsnorm_many_kernel(__half* __restrict__ x, const __half* __restrict__ delta
 // fp16 -> fp32 (exact): eight numbers per thread and step.  Bound by HBM: 6 bytes per number.  Logits of 700 tokens (32000 words): 31 us, where a library
 // conversion and a copy of its result took 95.
 __global__ void __launch_bounds__(256) half_to_float_kernel(const __half* __restrict__ src, float* __restrict__ dst, long long n) {
-  pc::pdl_launch_dependents();
-  pc::pdl_wait();
   const long long stride = static_cast<long long>(gridDim.x) * 256 * 8;
   for (long long i = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 8; i < n; i += stride) {
     if (i + 8 <= n) {
@@ -418,8 +416,10 @@ PC_API int pc_half_to_float(const void* src, void* dst, int64_t n, void* stream)
   PC_REQUIRE(src && dst && n > 0, "pc_half_to_float: null tensor");
   PC_REQUIRE((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) % 16 == 0, "pc_half_to_float: tensors must be 16B aligned");
   const long long blocks = (n + 2047) / 2048;
-  PC_CHECK_CUDA(pc::launch_pdl(half_to_float_kernel, dim3(static_cast<unsigned>(blocks < 148 * 16 ? blocks : 148 * 16)), dim3(256), 0,
-                               static_cast<cudaStream_t>(stream), static_cast<const __half*>(src), static_cast<float*>(dst), static_cast<long long>(n)));
+  // (an ordinary launch: as a dependent one its blocks waited on the SMs beside the product before; a suffix of 700 tokens 1634 -> 1593 us)
+  half_to_float_kernel<<<static_cast<unsigned>(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __half*>(src), static_cast<float*>(dst), static_cast<long long>(n));
+  PC_CHECK_CUDA(cudaGetLastError());
   pc::count_launch();
   return PC_OK;
 }
