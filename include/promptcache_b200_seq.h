@@ -176,7 +176,7 @@ typedef struct pcs_attn_params {
   const void* head_gate;    /* [n_tokens, head_gate_stride] `dtype` or NULL: head h's result *= sigmoid(head_gate[t, h]) */
   int64_t head_gate_stride;
   float out_scale;          /* the result is multiplied by this before it is rounded (0 counts as 1) */
-  int32_t reserved;
+  int32_t n_slots;          /* slots of k_pool and v_pool; 0: not told.  The tensor-map kernels read zeros, and no memory, behind the last one */
   int64_t out_stride;       /* elements between the result rows of neighbouring tokens (0: H * vdim) */
 } pcs_attn_params;        /* (head_scale to out_stride: not with `talk`) */
 /* scratch the key split of pcs_attn needs for n_tokens tokens */

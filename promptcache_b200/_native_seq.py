@@ -57,7 +57,7 @@ class pcs_attn_params(C.Structure):
                 ("softcap", C.c_float), ("window", C.c_int32), ("keep_first", C.c_int32), ("v_row_stride", C.c_int32),
                 ("sink_logit", C.c_void_p), ("pool_slot", C.c_void_p), ("talk", C.c_void_p),
                 ("out_gate", C.c_void_p), ("out_gate_stride", C.c_int64), ("head_scale", C.c_void_p), ("bias_table", C.c_void_p), ("bias_len", C.c_int32),
-                ("chunk", C.c_int32), ("head_gate", C.c_void_p), ("head_gate_stride", C.c_int64), ("out_scale", C.c_float), ("reserved", C.c_int32),
+                ("chunk", C.c_int32), ("head_gate", C.c_void_p), ("head_gate_stride", C.c_int64), ("out_scale", C.c_float), ("n_slots", C.c_int32),
                 ("out_stride", C.c_int64)]
 
 
@@ -507,7 +507,7 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: 
             raise NativeError("attention: the distance-bias numbers must be float32 [H]")
     p = pcs_attn_params()
     p.q, p.k_pool, p.v_pool, p.out = q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr()
-    p.n_heads, p.n_kv_heads, p.dim, p.cap = n_heads, k_pool.shape[1], k_pool.shape[3], k_pool.shape[2]
+    p.n_heads, p.n_kv_heads, p.dim, p.cap, p.n_slots = n_heads, k_pool.shape[1], k_pool.shape[3], k_pool.shape[2], min(k_pool.shape[0], v_pool.shape[0])
     p.vdim = out.shape[1] // n_heads if v_row_stride else v_pool.shape[3]
     p.v_row_stride, p.sink_logit, p.pool_slot, p.talk = int(v_row_stride), _ptr(sink_logit), _ptr(pool_slot), _ptr(talk)
     if out_gate is not None:

@@ -35,6 +35,16 @@ class PerDevice {
   Info info_[kDevices] = {};
 };
 
+// (slot, K/V head) planes of a pool for its tensor maps: they end where the pool ends, if the caller says where that is
+inline unsigned long long pool_planes(const pcs_attn_params& p) {
+  return p.n_slots > 0 ? static_cast<unsigned long long>(p.n_slots) * p.n_kv_heads : 1ull << 30;
+}
+
+// A launch over a step's own dense K/V (`pool_slot`) with rows of 96 and 64 numbers once ended with an illegal memory access.  What raised it is not known: the sizes, strides and slots it
+// got are in range, and so is every index that the kernel forms from them.  Such pools with rows that a tensor map's boxes of 64 columns do not divide are served by the mma.sync kernel, which
+// reads by plain loads, until it is known.
+inline bool dense_rows_off_boxes(const pcs_attn_params& p) { return p.pool_slot && (p.dim % 64 != 0 || p.vdim % 64 != 0); }
+
 // the launch chooses the kernel (1 and 2 name one)
 inline bool automatic(const pcs_attn_params& p) { return p.impl == 0 || p.impl == 3 || p.impl == 4 || p.impl == 7; }
 

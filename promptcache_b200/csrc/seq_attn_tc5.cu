@@ -606,7 +606,7 @@ int launch(const pcs_attn_params& p, cudaStream_t st) {
       }))
     return rc;
   const unsigned long long D = p.dim, V = p.vdim, cap = p.cap, H = p.n_heads;
-  const unsigned long long planes = 1ull << 30;  // (slot, K/V head) planes: the pool's slot count is the caller's
+  const unsigned long long planes = pool_planes(p);
   CUtensorMap mq, mk, mv;
   if (int rc = tensor_map_bf16(&mq, p.q, {D, H, static_cast<unsigned long long>(p.n_tokens)}, {D * 2, H * D * 2}, {64, 1, BM})) return rc;
   if (int rc = tensor_map_bf16(&mk, p.k_pool, {D, cap, planes}, {D * 2, cap * D * 2}, {64, BN, 1})) return rc;
@@ -758,6 +758,7 @@ double attn_tc5_expected(const pcs_attn_params& p, const Entries& entries) {
 int launch_attn_tc5(const pcs_attn_params& p, cudaStream_t st, bool* handled) {
   *handled = false;
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (dense_rows_off_boxes(p)) return PCS_OK;
   if (p.dtype != PCS_BF16 || p.max_len < 16 || (p.v_row_stride != 0 && p.v_row_stride != p.vdim) || p.dim % 8 != 0 || p.vdim % 8 != 0 || p.dim > 192 || p.vdim > 128)
     return PCS_OK;
   if (!p.seq_pos0 || !p.seq_len || !p.seq_off || !al16(p.q) || !al16(p.k_pool) || !al16(p.v_pool) || !al16(p.out) || p.out_stride % 8 != 0) return PCS_OK;

@@ -897,7 +897,7 @@ int launch(const pcs_attn_params& p, float* scratch, long long floats, cudaStrea
   const Info* info;
   if (int rc = per_device.get(&info, [&](Info&) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem); })) return rc;
   const unsigned long long D = p.dim, V = p.vdim, cap = p.cap, H = p.n_heads;
-  const unsigned long long planes = 1ull << 30;  // (slot, K/V head) planes: the pool's slot count is the caller's
+  const unsigned long long planes = pool_planes(p);
   CUtensorMap mq, mk, mv;
   if (int rc = tensor_map_bf16(&mq, p.q, {D, H, static_cast<unsigned long long>(p.n_tokens)}, {D * 2, H * D * 2}, {64, 1, BM})) return rc;
   if (int rc = tensor_map_bf16(&mk, p.k_pool, {D, cap, planes}, {D * 2, cap * D * 2}, {64, BN, 1})) return rc;
@@ -927,7 +927,7 @@ namespace {
 // Forms this kernel has: an even number of heads per K/V group, heads of 65 to 192 / 65 to 128 elements in 16-byte pieces, at most 256 entries
 bool serves(const pcs_attn_params& p) {
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  return p.dtype == PCS_BF16 && p.max_len >= 16 && (p.v_row_stride == 0 || p.v_row_stride == p.vdim) && p.dim % 8 == 0 && p.vdim % 8 == 0 && p.dim > 64 && p.dim <= 192 &&
+  return !dense_rows_off_boxes(p) && p.dtype == PCS_BF16 && p.max_len >= 16 && (p.v_row_stride == 0 || p.v_row_stride == p.vdim) && p.dim % 8 == 0 && p.vdim % 8 == 0 && p.dim > 64 && p.dim <= 192 &&
          p.vdim > 64 && p.vdim <= 128 && p.n_heads / p.n_kv_heads % 2 == 0 && p.n_seqs <= kMaxStreamSeqs && p.seq_pos0 && p.seq_len && p.seq_off && al16(p.q) &&
          al16(p.k_pool) && al16(p.v_pool) && al16(p.out) && p.out_stride % 8 == 0;
 }

@@ -90,11 +90,8 @@ def latent_attention(h: torch.Tensor, blk: dict, ckv: torch.Tensor, batch, step:
         c_ctx = nsq.latent_gather(ckv, C, ctx)
         kv = nsq.linear(c_ctx, blk["w_ukv"])             # [N, H * D + H * V]
         dense = ((most + 63) // 64) * 64
-        # One plane more than is used lies behind the last one: a prompt over rows of 96 numbers whose K ended 5.5 KB before its 2 MB segment raised an illegal memory access in the tensor-map
-        # kernel, with every index in range; the cause is not shown, the same call anywhere else in memory passes.
-        n = batch.n_seqs * H
-        kd = torch.empty(n + 1, dense, D + R, dtype=dt, device=dev)[:n].view(batch.n_seqs, H, dense, D + R)
-        vd = torch.empty(n + 1, dense, V, dtype=dt, device=dev)[:n].view(batch.n_seqs, H, dense, V)
+        kd = torch.empty(batch.n_seqs, H, dense, D + R, dtype=dt, device=dev)
+        vd = torch.empty(batch.n_seqs, H, dense, V, dtype=dt, device=dev)
         nsq.latent_expand(kv, ckv, C, R, H, D, V, kd, vd, ctx, seq_base=base)
         nsq.latent_q(q, H, D, R, blk["freqs"], blk["rot_mult"], batch, interleaved=il)
         o = torch.empty(T, H * V, dtype=dt, device=dev) if blk["gated"] else mixed
