@@ -122,14 +122,6 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 }
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + expf(-z)); }
-// the same for a result that leaves in bfloat16: exponential and reciprocal of the special function unit (some 2^-18 of the result, against 2^-9 of its rounding),
-// without the branches of the divide.  Results below 2^-126 stay (no flush to zero).
-__device__ __forceinline__ float sigmoid16_(float z) {
-  float e, r;
-  asm("ex2.approx.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-  return r;
-}
 __device__ __forceinline__ float softplusf_(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 __device__ __forceinline__ float logsigmoidf_(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 

@@ -386,8 +386,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const pcs_combine_para
   }
 }
 
-// 16-byte pieces: a block takes two rows, both requested before either is used, with as many threads as a row has pieces; the SiLU of bfloat16 runs is the special function unit's (the
-// branches of exponential and divide bounded it).  8192 rows of 1024: 13.0 us with half of 256 threads idle on one row, 10.9 so.
+// 16-byte pieces: a block takes two rows, both requested before either is used, with as many threads as a row has pieces.
 constexpr int kSiluRows = 2;
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ gu, long long gu_stride, T* __restrict__ out, int ff, int n_rows, const GluAct glu) {
@@ -397,7 +396,6 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ gu,
     const int r0 = blockIdx.x * kSiluRows;
     const T* g = gu + r0 * gu_stride;
     T* o = out + static_cast<long long>(r0) * ff;
-    const bool fast = sizeof(T) == 2 && glu.kind == PCS_GLU_SILU;
     for (int i = (blockIdx.y * blockDim.x + threadIdx.x) * N; i < ff; i += gridDim.y * blockDim.x * N) {
       float a[kSiluRows][N], u[kSiluRows][N];
 #pragma unroll
@@ -409,13 +407,8 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ gu,
 #pragma unroll
       for (int r = 0; r < kSiluRows; ++r)
         if (r0 + r < n_rows) {
-          if (fast) {
 #pragma unroll
-            for (int e = 0; e < N; ++e) a[r][e] = a[r][e] * sigmoid16_(a[r][e]) * u[r][e];
-          } else {
-#pragma unroll
-            for (int e = 0; e < N; ++e) a[r][e] = glu(a[r][e], gated ? u[r][e] : 0.f);
-          }
+          for (int e = 0; e < N; ++e) a[r][e] = glu(a[r][e], gated ? u[r][e] : 0.f);
           st16(o + static_cast<long long>(r) * ff + i, a[r]);
         }
     }

@@ -1,4 +1,4 @@
-"""The output gate of the matrix-memory recurrence in every form: sigmoid with all bits, down to gates whose sigmoid is below the smallest normal number."""
+"""The output gate of the matrix-memory recurrence in every form, down to gates whose sigmoid is below the smallest normal number."""
 import pytest
 import torch
 
