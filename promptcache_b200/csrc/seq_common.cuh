@@ -122,6 +122,17 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 }
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + expf(-z)); }
+// The same without the divide's branch, which keeps the sigmoids of a loop from overlapping: the reciprocal's approximation and one step of the Newton-Raphson iteration r <- r + r (1 - x r),
+// with x scaled by a power of two where the result would be below the numbers that step is exact for.  The same bits wherever the result is a normal number (2^27 arguments and all of bfloat16),
+// within 2^-149 of them below.
+__device__ __forceinline__ float sigmoid_nr_(float z) {
+  const float x = 1.f + expf(-z);
+  const bool large = !(x < 0x1p120f), inf = x == INFINITY;
+  const float s = inf ? 0.f : large ? 0x1p-32f : 1.f, y = inf ? 1.f : large ? x * 0x1p-32f : x;
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return fmaf(r, fmaf(-y, r, 1.f), r) * s;
+}
 __device__ __forceinline__ float softplusf_(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 __device__ __forceinline__ float logsigmoidf_(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 

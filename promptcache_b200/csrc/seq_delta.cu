@@ -1950,7 +1950,7 @@ __global__ void __launch_bounds__(kDoMaxWarps * 32) delta_chunk_out_kernel(const
       const uint2 gv = *reinterpret_cast<const uint2*>(gs + r * 32);
       const float gf[4] = {__uint_as_float(gv.x << 16), __uint_as_float(gv.x & 0xffff0000u), __uint_as_float(gv.y << 16), __uint_as_float(gv.y & 0xffff0000u)};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) x[q] = x[q] * f * wv[q] * sigmoidf_(gf[q]) * (o.silu ? gf[q] : 1.f);
+      for (int q = 0; q < 4; ++q) x[q] = x[q] * f * wv[q] * sigmoid_nr_(gf[q]) * (o.silu ? gf[q] : 1.f);
       __nv_bfloat16* d = out + static_cast<long long>(i) * o.out_stride;
       if (vec) *reinterpret_cast<uint2*>(d) = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
       else {

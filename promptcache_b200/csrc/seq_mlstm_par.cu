@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(kOutWarps * 32, 1) mlstm_par_out_kernel(const 
     uint32_t y[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      y[k] = pack_bf16(x[2 * k] * f * w[2 * k] * sigmoidf_(__uint_as_float(g[k] << 16)), x[2 * k + 1] * f * w[2 * k + 1] * sigmoidf_(__uint_as_float(g[k] & 0xffff0000u)));
+      y[k] = pack_bf16(x[2 * k] * f * w[2 * k] * sigmoid_nr_(__uint_as_float(g[k] << 16)), x[2 * k + 1] * f * w[2 * k + 1] * sigmoid_nr_(__uint_as_float(g[k] & 0xffff0000u)));
     __nv_bfloat16* o = out + r * os;
     if (o16) *reinterpret_cast<uint4*>(o) = make_uint4(y[0], y[1], y[2], y[3]);
     else {
