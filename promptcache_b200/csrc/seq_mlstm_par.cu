@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(kST) mlstm_par_state_kernel(const pcs_mlstm_pa
   auto left_n = [&](int j) { return sc.left_n + (left0 + static_cast<long long>(j) * H) * D + d0; };
   auto factor = [&](int j) {   // of segment j
     float f = 1.f;
+#pragma unroll 4
     for (int i = 0; i < per; ++i) f *= sc.ce[entry0 + static_cast<long long>(j * per + i) * H];
     return f;
   };
@@ -254,16 +255,33 @@ __global__ void __launch_bounds__(kST) mlstm_par_state_kernel(const pcs_mlstm_pa
       for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(left(segs - 1) + j * 512) = make_float4(s[j][0], s[j][1], s[j][2], s[j][3]);
     }
   } else if (!from_pool) {
-    for (int i = 0; i == 0 || i < seg; ++i) {
-      const float f = i ? factor(i) : 0.f;
+    // (the next segment's numbers are under way while those before it are added)
+    float4 x[8];
+    auto fetch = [&](int i) {
       const float* l = left(seg ? i : segs - 1);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 x = *reinterpret_cast<const float4*>(l + j * 512);
-        s[j][0] = fmaf(s[j][0], f, x.x);
-        s[j][1] = fmaf(s[j][1], f, x.y);
-        s[j][2] = fmaf(s[j][2], f, x.z);
-        s[j][3] = fmaf(s[j][3], f, x.w);
+      for (int j = 0; j < 8; ++j) x[j] = *reinterpret_cast<const float4*>(l + j * 512);
+    };
+    fetch(0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { s[j][0] = x[j].x; s[j][1] = x[j].y; s[j][2] = x[j].z; s[j][3] = x[j].w; }
+    if (seg > 1) {
+      float f = factor(1);
+      fetch(1);
+#pragma unroll 1
+      for (int i = 1; i < seg; ++i) {
+        const float now = f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          s[j][0] = fmaf(s[j][0], now, x[j].x);
+          s[j][1] = fmaf(s[j][1], now, x[j].y);
+          s[j][2] = fmaf(s[j][2], now, x[j].z);
+          s[j][3] = fmaf(s[j][3], now, x[j].w);
+        }
+        if (i + 1 < seg) {
+          fetch(i + 1);
+          f = factor(i + 1);
+        }
       }
     }
   }
@@ -646,11 +664,20 @@ __global__ void __launch_bounds__(kOutWarps * 32, 1) mlstm_par_out_kernel(const 
   }
 }
 
-// Segments of a walk over `chunks`, each of at least three.  A step takes 0.75 us, the launch before costs about five (one head pair of 128 x 128 over 44 chunks: 67 us as
-// one walk, 43 in 14 segments; 3052 tokens of 4 heads 83 and 57).
+// Segments of a walk over `chunks`.  us, fitted: one walk 1.9 and 0.955 a chunk; two launches 5.3, 1.35 a chunk of a segment and 0.38 a segment (the later ones add up those before them).  Tiles x chunks,
+// as one walk / in so many segments: 4 x 7 8.5 / 8.6 in 4, 4 x 10 11.3 / 9.9 in 5, 8 x 13 13.9 / 9.9 in 7, 32 x 11 12.4 / 11.1 in 4, 32 x 16 17.0 / 13.2 in 4, 4 x 47 45.1 / 15.6 in 12.
 static int state_segments(long long tiles, int chunks) {
-  const int segs = static_cast<int>(kMaxTiles / tiles < chunks / 3 ? kMaxTiles / tiles : chunks / 3);
-  return segs > 1 && 2 * ((chunks + segs - 1) / segs) + 5 < chunks ? segs : 1;
+  int best = 1;
+  double least = 0.98 * (1.9 + 0.955 * chunks);
+  for (int per = 2; per < chunks; ++per) {
+    const int segs = (chunks + per - 1) / per;
+    const double us = 5.3 + 1.35 * per + 0.38 * segs;
+    if (us < least && segs * tiles <= kMaxTiles) {
+      least = us;
+      best = segs;
+    }
+  }
+  return best;
 }
 
 template <int MT>

@@ -14,6 +14,8 @@ DEV, BF16, F64 = torch.device("cuda:0"), torch.bfloat16, torch.float64
     (2, 80, 72, 2, [(961,), (1100,)]),               # tiles that reach past rows and columns; gates on 4 bytes
     (1, 256, 512, 2, [(449,)]),
     (1, 128, 256, 2, [(200,)]),
+    (2, 64, 128, 0, [(577, 129, 65), (64, 641, 1)]),  # five segments of two chunks: entries that fill the first, or part of it
+    (4, 128, 128, 0, [(705, 400)]),                  # as many segments as there are SMs for
 ])
 def test_long_walks_of_few_heads(H, D, V, gap, steps):
     from promptcache_b200 import _native_seq as nsq
