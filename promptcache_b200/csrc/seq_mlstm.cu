@@ -398,7 +398,7 @@ namespace pcs {
 int launch_mlstm_chunk(const pcs_mlstm_params& p, float* nm_new, cudaStream_t st);
 int launch_mlstm_par(const pcs_mlstm_params& p, cudaStream_t st, bool* handled);
 bool mlstm_par_serves(const pcs_mlstm_params& p);
-long long mlstm_par_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim);
+long long mlstm_par_wanted(const pcs_mlstm_params& p);
 constexpr int kChunkMinLen = 24;  // shorter steps (decoding, tails of a prompt) go token by token
 // rows in 16-byte pieces
 static bool mlstm_aligned(const pcs_mlstm_params& p) {
@@ -414,7 +414,7 @@ static bool mlstm_in_chunks(const pcs_mlstm_params& p) {
 
 PCS_API int64_t pcs_mlstm_scratch_wanted(const pcs_mlstm_params* p) {
   if (!p || p->n_seqs <= 0 || p->n_tokens <= 0 || p->heads <= 0 || p->dim <= 0 || p->vdim <= 0 || !pcs::mlstm_in_chunks(*p) || !pcs::mlstm_par_serves(*p)) return 0;
-  return pcs::mlstm_par_floats(p->n_tokens, p->n_seqs, p->heads, p->dim, p->vdim);
+  return pcs::mlstm_par_wanted(*p);
 }
 
 PCS_API int pcs_mlstm_gates(const void* h, int64_t h_stride, const void* w_i, const void* w_f, const float* b_i, const float* b_f,

@@ -22,20 +22,25 @@ constexpr int CL = 64;      // tokens per chunk
 constexpr int PROW = CL + 8;
 
 // The scratch of one launch.  An entry's chunks are consecutive slots behind those of the entries before it (whatever the order of their rows); there are at
-// most n_tokens / 64 + n_seqs of them.
+// most n_tokens / 64 + n_seqs of them.  A walk in segments has more behind these: what the segments add up to.
 struct Scratch {
-  float *left, *u, *n, *tok, *ce, *left_n;   // [entry][segment][head][tile][64 * 64], [slot][head][dim * vdim], [slot][head][dim], [slot][head][5][64], [slot][head],
+  float *u, *n, *tok, *ce, *left, *left_n;   // [slot][head][dim * vdim], [slot][head][dim], [slot][head][5][64], [slot][head], [entry][segment][head][tile][64 * 64],
                                              // [entry][segment][head][dim]
   int* first;                                // [entry] its first slot
   static constexpr int kLeft = 148 * 64 * 64, kLeftN = 148 * 64;   // (at most 148 tiles of all segments, each of which has at most 64 rows)
-  __host__ __device__ Scratch(float* base, long long slots, int H, int D, int V) {
-    left = base;
-    u = left + kLeft;
+  // floats up to `left`, which begins on 16 bytes as the scratch does
+  static __host__ __device__ long long whole(long long slots, int n_seqs, int H, int D, int V) {
+    return (slots * H * (static_cast<long long>(D) * V + D + 5 * CL + 1) + n_seqs + 3) / 4 * 4;
+  }
+  __host__ __device__ Scratch(float* base, long long slots, const pcs_mlstm_params& p) {
+    const int H = p.heads, D = p.dim, V = p.vdim;
+    u = base;
     n = u + slots * H * D * V;
     tok = n + slots * H * D;
     ce = tok + slots * H * 5 * CL;
-    left_n = ce + slots * H;
-    first = reinterpret_cast<int*>(left_n + kLeftN);
+    first = reinterpret_cast<int*>(ce + slots * H);
+    left = base + whole(slots, p.n_seqs, H, D, V);
+    left_n = left + kLeft;
   }
 };
 
@@ -68,7 +73,7 @@ struct ChunkGates {
 
 __global__ void __launch_bounds__(512) mlstm_par_gates_kernel(const pcs_mlstm_params p, float* scratch, long long slots) {
   extern __shared__ float sm[];   // per chunk: its last b, its largest a (then the stabiliser it starts from)
-  const Scratch sc(scratch, slots, p.heads, p.dim, p.vdim);
+  const Scratch sc(scratch, slots, p);
   const int b = blockIdx.x, head = blockIdx.y, H = p.heads, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int len = p.seq_len[b], off = p.seq_off[b];
   if (len <= 0) return;
@@ -142,7 +147,7 @@ __global__ void __launch_bounds__(kST) mlstm_par_state_kernel(const pcs_mlstm_pa
   const int D = p.dim, V = p.vdim, H = p.heads, b = blockIdx.z / segs, seg = blockIdx.z % segs, head = blockIdx.y, vtiles = (V + 63) / 64;
   const int d0 = static_cast<int>(blockIdx.x) / vtiles * 64, v0 = static_cast<int>(blockIdx.x) % vtiles * 64;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = lane >> 2, qd = lane & 3;
-  const Scratch sc(scratch, slots, H, D, V);
+  const Scratch sc(scratch, slots, p);
   const int all = p.seq_len[b];
   if (all <= 0) return;
   const int per = ((all + CL - 1) / CL + segs - 1) / segs, c_lo = seg * per, len = min(all - c_lo * CL, per * CL);   // this segment's chunks and tokens
@@ -402,7 +407,7 @@ __global__ void __launch_bounds__(kOutWarps * 32, 1) mlstm_par_out_kernel(const 
   float* nq = psum + 4 * CL;                                        // [64] q . n of the state
   float* inv = nq + CL;                                             // [64] 1 / rms
   float* ss = inv + CL;                                             // [columns' warps][64] sums of squares
-  const Scratch sc(scratch, slots, H, D, V);
+  const Scratch sc(scratch, slots, p);
   const int c = blockIdx.x, b = blockIdx.y / H, head = blockIdx.y - b * H;
   const int len = p.seq_len[b], i0 = c * CL;
   if (i0 >= len) return;
@@ -691,11 +696,16 @@ int launch_out(const pcs_mlstm_params& p, float* scratch, long long slots, dim3 
   return PCS_OK;
 }
 
+static long long tiles_of(int n_seqs, int heads, int dim, int vdim) { return static_cast<long long>((dim + 63) / 64) * ((vdim + 63) / 64) * heads * n_seqs; }
+
+static long long floats(int n_tokens, int n_seqs, int heads, int dim, int vdim, bool cut) {
+  return Scratch::whole(n_tokens / CL + n_seqs, n_seqs, heads, dim, vdim) + (cut ? Scratch::kLeft + Scratch::kLeftN : 0);
+}
+
 }  // namespace
 
-long long mlstm_par_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim) {
-  const long long slots = n_tokens / CL + n_seqs;
-  return slots * heads * (static_cast<long long>(dim) * vdim + dim + 5 * CL + 1) + Scratch::kLeft + Scratch::kLeftN + n_seqs;
+long long mlstm_par_wanted(const pcs_mlstm_params& p) {
+  return floats(p.n_tokens, p.n_seqs, p.heads, p.dim, p.vdim, state_segments(tiles_of(p.n_seqs, p.heads, p.dim, p.vdim), (p.max_len + CL - 1) / CL) > 1);
 }
 
 // The caller has checked type, alignment and dim (a multiple of 16, at most 256).  Four launches against one walk and two: fewer than four chunks (eight where
@@ -710,7 +720,7 @@ bool mlstm_par_serves(const pcs_mlstm_params& p) {
 int launch_mlstm_par(const pcs_mlstm_params& p, cudaStream_t st, bool* handled) {
   *handled = false;
   if (!p.chunk_scratch || !mlstm_par_serves(p) || (reinterpret_cast<uintptr_t>(p.chunk_scratch) & 15) != 0 ||
-      p.chunk_floats < mlstm_par_floats(p.n_tokens, p.n_seqs, p.heads, p.dim, p.vdim))
+      p.chunk_floats < floats(p.n_tokens, p.n_seqs, p.heads, p.dim, p.vdim, false))
     return PCS_OK;
   const long long slots = p.n_tokens / CL + p.n_seqs;
   const int chunks = (p.max_len + CL - 1) / CL;
@@ -724,7 +734,8 @@ int launch_mlstm_par(const pcs_mlstm_params& p, cudaStream_t st, bool* handled) 
     PCS_CHECK_CUDA(cudaFuncSetAttribute(mlstm_par_state_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(state_smem())));
     configured = true;
   }
-  const int tiles = ((p.dim + 63) / 64) * ((p.vdim + 63) / 64), segs = state_segments(tiles * p.heads * p.n_seqs, chunks);
+  const int tiles = ((p.dim + 63) / 64) * ((p.vdim + 63) / 64);
+  const int segs = p.chunk_floats < floats(p.n_tokens, p.n_seqs, p.heads, p.dim, p.vdim, true) ? 1 : state_segments(tiles_of(p.n_seqs, p.heads, p.dim, p.vdim), chunks);
   if (segs > 1) {
     mlstm_par_state_kernel<true><<<dim3(tiles, p.heads, p.n_seqs * segs), kST, state_smem(), st>>>(p, s, slots, segs);
     PCS_CHECK_CUDA(cudaGetLastError());
@@ -740,7 +751,11 @@ int launch_mlstm_par(const pcs_mlstm_params& p, cudaStream_t st, bool* handled) 
 
 }  // namespace pcs
 
+// What any call of these sizes may want: its longest entry, which decides on segments, has up to n_tokens
 PCS_API int64_t pcs_mlstm_scratch_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim) {
   if (n_tokens <= 0 || n_seqs <= 0 || heads <= 0 || dim <= 0 || vdim <= 0) return 0;
-  return pcs::mlstm_par_floats(n_tokens, n_seqs, heads, dim, vdim);
+  const long long tiles = pcs::tiles_of(n_seqs, heads, dim, vdim);
+  bool cut = false;
+  for (int c = 2; !cut && 2 * tiles <= pcs::kMaxTiles && c <= (n_tokens + pcs::CL - 1) / pcs::CL; ++c) cut = pcs::state_segments(tiles, c) > 1;
+  return pcs::floats(n_tokens, n_seqs, heads, dim, vdim, cut);
 }
