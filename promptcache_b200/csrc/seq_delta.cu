@@ -2108,6 +2108,9 @@ PCS_API int pcs_delta_chunk_prep(const pcs_delta_chunk_params* p, void* stream) 
   PCS_REQUIRE(p->qk && p->v && p->b && p->chunk_first && p->chunk_len && p->qd && p->kd && p->w && p->g && p->u && p->a, "pcs_delta_chunk_prep: null tensor");
   PCS_REQUIRE(p->heads > 0 && p->heads <= 65535 && p->kv_heads > 0 && p->heads % p->kv_heads == 0 && p->dim > 0 && p->dim <= 256 && p->vdim > 0,
               "pcs_delta_chunk_prep: bad sizes (dim %d of at most 256)", p->dim);
+  auto off = [](const void* q, int bytes) { return (reinterpret_cast<uintptr_t>(q) & (bytes - 1)) != 0; };
+  PCS_REQUIRE(!off(p->w, 16) && (p->dtype != PCS_BF16 || (!off(p->kd, 16) && (p->vdim % 4 != 0 || off(p->v, 8) || !off(p->u, 16)))),
+              "pcs_delta_chunk_prep: w, and in bfloat16 runs kd and u, must be 16-byte aligned");
   const int D4 = (p->dim + 3) & ~3;
   const size_t smem = (static_cast<size_t>(2) * pcs::kC * (D4 + 4) + static_cast<size_t>(pcs::kC) * (D4 + 4 > pcs::kTi ? D4 + 4 : pcs::kTi) + 4 * D4 + pcs::kC * pcs::kC + pcs::kC) * sizeof(float);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -2132,6 +2135,8 @@ PCS_API int pcs_delta_chunk_scan(const pcs_delta_chunk_params* p, void* stream) 
   PCS_REQUIRE(p->kd && p->w && p->g && p->u && p->s && p->s_pool && p->seq_slot && p->seq_pos0 && p->seq_chunk0 && p->seq_chunks, "pcs_delta_chunk_scan: null tensor");
   PCS_REQUIRE(p->heads > 0 && p->heads <= 65535 && p->n_seqs <= 65535 && p->dim > 0 && p->dim <= 256 && p->vdim > 0, "pcs_delta_chunk_scan: bad sizes");
   PCS_REQUIRE(((reinterpret_cast<uintptr_t>(p->kd) | reinterpret_cast<uintptr_t>(p->w)) & 15) == 0, "pcs_delta_chunk_scan: kd and w must be 16-byte aligned");
+  PCS_REQUIRE(p->dtype != PCS_BF16 || p->vdim % 2 != 0 || ((reinterpret_cast<uintptr_t>(p->u) | reinterpret_cast<uintptr_t>(p->s) | reinterpret_cast<uintptr_t>(p->s_pool)) & 7) == 0,
+              "pcs_delta_chunk_scan: u, s and s_pool must be 8-byte aligned");
   const int L = (p->dim + 63) & ~63;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (p->dtype == PCS_BF16) return p->dim <= 128 ? pcs::launch_delta_chunk_scan_tc<1>(*p, st) : pcs::launch_delta_chunk_scan_tc<2>(*p, st);
@@ -2156,6 +2161,7 @@ PCS_API int pcs_delta_chunk_out(const pcs_delta_chunk_params* p, const pcs_headn
   PCS_REQUIRE(p->dtype == PCS_BF16 && p->heads > 0 && p->heads <= 65535 && p->dim > 0 && p->dim <= 256 && p->vdim > 0 && p->vdim <= 32 * pcs::kDoMaxWarps,
               "pcs_delta_chunk_out: serves bfloat16, dim up to 256 and vdim up to %d", 32 * pcs::kDoMaxWarps);
   PCS_REQUIRE(((reinterpret_cast<uintptr_t>(p->qd) | reinterpret_cast<uintptr_t>(p->a)) & 15) == 0, "pcs_delta_chunk_out: qd and a must be 16-byte aligned");
+  PCS_REQUIRE(p->vdim % 4 != 0 || ((reinterpret_cast<uintptr_t>(p->s) | reinterpret_cast<uintptr_t>(p->u)) & 15) == 0, "pcs_delta_chunk_out: s and u must be 16-byte aligned");
   PCS_REQUIRE(p->parts == 0 || p->parts == 2 || p->parts == 3, "pcs_delta_chunk_out: operands enter in two parts or in three");
   const int warps = (p->vdim + 31) / 32 < 2 ? 2 : (p->vdim + 31) / 32, D16 = (p->dim + 15) & ~15;
   auto launch = [&](auto kernel, int parts, int tokens) -> int {
