@@ -1,39 +1,8 @@
 // What the attention kernels over the slot pool share: the keys a query sees, and where its result goes.
 #pragma once
-#include <atomic>
-#include <mutex>
-
 #include "seq_common.cuh"
 
 namespace pcs {
-
-// What a launch needs to know of its kernel, found out (and the kernel's shared memory raised) once on every device: attributes are a device's own.
-template <typename Info>
-class PerDevice {
- public:
-  // setup(Info&) -> cudaError_t; a failed one is tried again by the next launch
-  template <typename Setup>
-  int get(const Info** info, Setup setup) {
-    int d = 0;
-    PCS_CHECK_CUDA(cudaGetDevice(&d));
-    PCS_REQUIRE(d >= 0 && d < kDevices, "device %d: the attention kernels serve devices 0 to %d", d, kDevices - 1);
-    if (!ready_[d].load(std::memory_order_acquire)) {
-      std::lock_guard<std::mutex> hold(lock_);
-      if (!ready_[d].load(std::memory_order_relaxed)) {
-        PCS_CHECK_CUDA(setup(info_[d]));
-        ready_[d].store(true, std::memory_order_release);
-      }
-    }
-    *info = &info_[d];
-    return PCS_OK;
-  }
-
- private:
-  static constexpr int kDevices = 64;
-  std::mutex lock_;
-  std::atomic<bool> ready_[kDevices] = {};
-  Info info_[kDevices] = {};
-};
 
 // (slot, K/V head) planes of a pool for its tensor maps: they end where the pool ends, if the caller says where that is
 inline unsigned long long pool_planes(const pcs_attn_params& p) {

@@ -179,11 +179,8 @@ __global__ void __launch_bounds__(LB_THREADS) attn_latent_kernel(const pcs_attn_
 
 template <int NT>
 int launch_nt(const pcs_attn_params& p, cudaStream_t st, int DKP, int splits, size_t smem) {
-  static bool configured = false;
-  if (!configured) {
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(attn_latent_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    configured = true;
-  }
+  static PerDevice<NoInfo> set_up;
+  if (int rc = set_up.once([&] { return cudaFuncSetAttribute(attn_latent_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); })) return rc;
   dim3 grid(p.n_tokens, (p.n_heads + LB_HEADS - 1) / LB_HEADS, splits);
   attn_latent_kernel<NT><<<grid, LB_THREADS, smem, st>>>(p, DKP);
   PCS_CHECK_CUDA(cudaGetLastError());

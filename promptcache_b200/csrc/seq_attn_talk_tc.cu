@@ -272,11 +272,8 @@ __global__ void __launch_bounds__(NW * 32, MINB) attn_talk_tc_kernel(const pcs_a
 
 template <int WP, int HPW, int BN, int NW, int MINB>
 int launch_one(const pcs_attn_params& p, cudaStream_t st, size_t smem) {
-  static bool configured = false;
-  if (!configured) {
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(attn_talk_tc_kernel<WP, HPW, BN, NW, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    configured = true;
-  }
+  static PerDevice<NoInfo> set_up;
+  if (int rc = set_up.once([&] { return cudaFuncSetAttribute(attn_talk_tc_kernel<WP, HPW, BN, NW, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); })) return rc;
   const int n_qtiles = (p.max_len + TT_BM - 1) / TT_BM;
   attn_talk_tc_kernel<WP, HPW, BN, NW, MINB><<<p.n_seqs * n_qtiles, NW * 32, smem, st>>>(p);
   PCS_CHECK_CUDA(cudaGetLastError());

@@ -294,11 +294,8 @@ template <int DP, int VP>
 int launch(const pcs_attn_params& p, cudaStream_t st) {
   const size_t smem = (static_cast<size_t>(BM + 2 * BN) * (DP + PAD) + static_cast<size_t>(BN) * (VP + PAD)) * sizeof(__nv_bfloat16) +
                       272 * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(attn_tc_kernel<DP, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    configured = true;
-  }
+  static PerDevice<NoInfo> set_up;
+  if (int rc = set_up.once([&] { return cudaFuncSetAttribute(attn_tc_kernel<DP, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); })) return rc;
   dim3 grid(static_cast<unsigned>((p.max_len + BM - 1) / BM) * p.n_seqs * p.n_heads);
   attn_tc_kernel<DP, VP><<<grid, TC_THREADS, smem, st>>>(p);
   PCS_CHECK_CUDA(cudaGetLastError());

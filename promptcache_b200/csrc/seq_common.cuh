@@ -6,6 +6,9 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "../../include/promptcache_b200_seq.h"
 
 #define PCS_API extern "C" __attribute__((visibility("default")))
@@ -26,6 +29,41 @@ void count_launch(int n = 1);
   do {                                                                 \
     if (!(cond)) return pcs::set_error(PCS_ERR_INVALID, __VA_ARGS__);  \
   } while (0)
+
+// What a launch needs to know of its kernel, found out (and the kernel's shared memory raised) once on every device: attributes are a device's own.
+template <typename Info>
+class PerDevice {
+ public:
+  // setup(Info&) -> cudaError_t; a failed one is tried again by the next launch
+  template <typename Setup>
+  int get(const Info** info, Setup setup) {
+    int d = 0;
+    PCS_CHECK_CUDA(cudaGetDevice(&d));
+    PCS_REQUIRE(d >= 0 && d < kDevices, "device %d: the kernels serve devices 0 to %d", d, kDevices - 1);
+    if (!ready_[d].load(std::memory_order_acquire)) {
+      std::lock_guard<std::mutex> hold(lock_);
+      if (!ready_[d].load(std::memory_order_relaxed)) {
+        PCS_CHECK_CUDA(setup(info_[d]));
+        ready_[d].store(true, std::memory_order_release);
+      }
+    }
+    *info = &info_[d];
+    return PCS_OK;
+  }
+  template <typename Setup>   // setup() -> cudaError_t, of kernels of which nothing else needs to be known
+  int once(Setup setup) {
+    const Info* info;
+    return get(&info, [&](Info&) { return setup(); });
+  }
+
+ private:
+  static constexpr int kDevices = 64;
+  std::mutex lock_;
+  std::atomic<bool> ready_[kDevices] = {};
+  Info info_[kDevices] = {};
+};
+
+struct NoInfo {};
 
 // dispatch a templated launch on the run-time type code
 #define PCS_DISPATCH(dtype, ...)                                                    \

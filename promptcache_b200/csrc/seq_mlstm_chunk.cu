@@ -343,12 +343,12 @@ size_t mlstm_chunk_smem(int dim, int cvs) {
 }
 
 int launch_mlstm_chunk(const pcs_mlstm_params& p, float* nm_new, cudaStream_t st) {
-  static bool configured = false;
-  if (!configured) {
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(mlstm_chunk_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(mlstm_chunk_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    configured = true;
-  }
+  static PerDevice<NoInfo> set_up;
+  if (int rc = set_up.once([&] {
+        const cudaError_t err = cudaFuncSetAttribute(mlstm_chunk_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        return err != cudaSuccess ? err : cudaFuncSetAttribute(mlstm_chunk_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      }))
+    return rc;
   // 32 columns per block unless that leaves the GPU mostly empty (one long prompt): narrower slices recompute the q . k
   // scores in more blocks but halve everything else a block does per chunk
   const long long blocks32 = static_cast<long long>(p.n_seqs) * p.heads * ((p.vdim + 31) / 32);

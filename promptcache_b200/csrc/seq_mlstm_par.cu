@@ -685,11 +685,8 @@ static int state_segments(long long tiles, int chunks) {
 
 template <int MT>
 int launch_out(const pcs_mlstm_params& p, float* scratch, long long slots, dim3 grid, cudaStream_t st) {
-  static bool configured = false;
-  if (!configured) {
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(mlstm_par_out_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_smem(256, kOutWarps, MT)));
-    configured = true;
-  }
+  static PerDevice<NoInfo> set_up;
+  if (int rc = set_up.once([&] { return cudaFuncSetAttribute(mlstm_par_out_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_smem(256, kOutWarps, MT)); })) return rc;
   const int warps = (p.vdim + 31) / 32 * (4 / MT);
   mlstm_par_out_kernel<MT><<<grid, warps * 32, out_smem(p.dim, warps, MT), st>>>(p, scratch, slots);
   PCS_CHECK_CUDA(cudaGetLastError());
@@ -728,12 +725,12 @@ int launch_mlstm_par(const pcs_mlstm_params& p, cudaStream_t st, bool* handled) 
   float* s = p.chunk_scratch;
   mlstm_par_gates_kernel<<<dim3(p.n_seqs, p.heads), 512, 2 * chunks * sizeof(float), st>>>(p, s, slots);
   PCS_CHECK_CUDA(cudaGetLastError());
-  static bool configured = false;
-  if (!configured) {
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(mlstm_par_state_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(state_smem())));
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(mlstm_par_state_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(state_smem())));
-    configured = true;
-  }
+  static PerDevice<NoInfo> set_up;
+  if (int rc = set_up.once([&] {
+        const cudaError_t err = cudaFuncSetAttribute(mlstm_par_state_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(state_smem()));
+        return err != cudaSuccess ? err : cudaFuncSetAttribute(mlstm_par_state_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(state_smem()));
+      }))
+    return rc;
   const int tiles = ((p.dim + 63) / 64) * ((p.vdim + 63) / 64);
   const int segs = p.chunk_floats < floats(p.n_tokens, p.n_seqs, p.heads, p.dim, p.vdim, true) ? 1 : state_segments(tiles_of(p.n_seqs, p.heads, p.dim, p.vdim), chunks);
   if (segs > 1) {

@@ -303,12 +303,12 @@ PCS_API int pcs_moe_gemm(int stage, const void* a, int64_t a_stride, const void*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int per_block = stage == 0 ? pcs::GN / 2 : pcs::GN;  // output features of one block
   dim3 grid(pcs::plan_max_tiles(n_pairs, n_experts), ((stage == 0 ? ff : width) + per_block - 1) / per_block);
-  static bool configured = false;
-  if (!configured) {
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(pcs::moe_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pcs::G_SMEM)));
-    PCS_CHECK_CUDA(cudaFuncSetAttribute(pcs::moe_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pcs::G_SMEM)));
-    configured = true;
-  }
+  static pcs::PerDevice<pcs::NoInfo> set_up;
+  if (int rc = set_up.once([&] {
+        const cudaError_t err = cudaFuncSetAttribute(pcs::moe_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pcs::G_SMEM));
+        return err != cudaSuccess ? err : cudaFuncSetAttribute(pcs::moe_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pcs::G_SMEM));
+      }))
+    return rc;
   PCS_REQUIRE(grid.y <= 65535, "pcs_moe_gemm: too many output features");
   const pcs::GluAct act(glu);
   if (!act.gated()) return pcs::set_error(PCS_ERR_UNSUPPORTED, "pcs_moe_gemm: experts without a gate branch (activation %d) take the row kernels or the library's grouped product", act.kind);
