@@ -1001,11 +1001,11 @@ def _gla_chunk_plan(batch: Batch, chunk: int):
 
 
 def _gla_states_in_one(chunks: int, most: int, heads: int, dim: int, vdim: int) -> bool:
-    """Whether one walk over the chunks (`pcs_gla_chunk_states`) is expected to be faster than their own sums and a scan over them.  In us on B200, fitted to 40 drawn calls: a step of the
-    longest walk takes 1.08 and a step of all walks 1.33 of an SM; the sums and the scan move the states three times.  4 heads of 256 x 512, 1500 and 548 tokens: 42 against 68; of
-    128 x 128, 1950 tokens: 37 against 12."""
+    """Whether one walk over the chunks (`pcs_gla_chunk_states`) is expected to be faster than their own sums and a scan over them.  In us on B200, fitted to 146 calls of one to six entries: a
+    step of the longest walk takes 1.25 and a step of all walks 1.33 of an SM; the sums and the scan move the states three times.  Of those calls six then take a form that is slower by more than
+    3 % (at most 15).  4 heads of 256 x 512, 1500 and 548 tokens: 41 against 67; 8 heads of 128 x 256, 1024 tokens: 23 against 17; of 128 x 128, 1950 tokens: 37 against 12."""
     tiles = -(-dim // 64) * -(-vdim // 64)
-    return 1.5 + max(1.08 * most, 1.33 / 148 * chunks * heads * tiles) < 0.9 * (6.0 + 0.95e-6 * 4 * chunks * heads * dim * vdim)
+    return 2.7 + max(1.25 * most, 1.33 / 148 * chunks * heads * tiles) < 7.2 + 0.85e-6 * 4 * chunks * heads * dim * vdim
 
 
 def gla_scan_chunked(proj: torch.Tensor, offs, ld: torch.Tensor, norm_w: torch.Tensor, out: torch.Tensor, s_pool: torch.Tensor, eps: float, batch: Batch,
