@@ -1,4 +1,4 @@
-"""A chunk's preparation for the delta rule (bfloat16 runs, decays per channel) against float64: the sums over pairs, the solved values and the solved keys, at the edges of its tiles
+"""A chunk's preparation for the delta rule (bfloat16 runs, decays per channel or per head) against float64: the sums over pairs, the solved values and keys, the outgoing keys, at the edges of its tiles
 (four channels, eight, sixteen tokens, 32 columns), with strong decays, none at all, and values whose rows start off eight bytes."""
 import ctypes as C
 
@@ -13,7 +13,8 @@ DEV, BF16, F32, F64 = torch.device("cuda:0"), torch.bfloat16, torch.float32, tor
     (1, 1, 4, 4, (1, 64), 1.0), (1, 2, 20, 33, (15, 17), 0.1), (2, 1, 36, 40, (64, 33), 20.0), (1, 1, 100, 7, (63, 16, 49), 0.0), (2, 2, 128, 128, (64, 31), 1.0), (1, 2, 256, 512, (64, 50), 0.5),
     (1, 1, 7, 65, (40,), 1.0),
 ])
-def test_prep(KV, G, D, V, lens, rate):
+@pytest.mark.parametrize("per_head", [False, True])
+def test_prep(KV, G, D, V, lens, rate, per_head):
     from promptcache_b200 import _native_seq as nsq
     g = torch.Generator().manual_seed(D * 3 + V)
     H, T, nc = KV * G, sum(lens), len(lens)
@@ -24,11 +25,17 @@ def test_prep(KV, G, D, V, lens, rate):
     v = torch.randn(T, H * V, generator=g).to(BF16)
     ld = -rate * torch.rand(T, H, D, generator=g) * torch.rand(T, H, D, generator=g)
     b = torch.randn(T, H, generator=g).to(BF16)
+    dec_a, bias, rates = torch.randn(T, H, generator=g).to(BF16), torch.randn(H, generator=g) * 0.5, rate * (0.2 + torch.rand(H, generator=g))
+    if per_head:
+        ld = (-rates.to(F64) * torch.nn.functional.softplus(dec_a.to(F64) + bias.to(F64)))[:, :, None].expand(T, H, D)
+        rate = float(ld.abs().max())
     D8, L = (D + 7) // 8 * 8, (D + 63) // 64 * 64
-    dev = {n: t.to(DEV).contiguous() for n, t in dict(qk=qk, v=v, ld=ld, b=b, first=torch.tensor(first, dtype=torch.int32), lens=torch.tensor(lens, dtype=torch.int32)).items()}
+    dev = {n: t.to(DEV).contiguous() for n, t in dict(qk=qk, v=v, ld=ld.float(), b=b, dec_a=dec_a, bias=bias, rates=rates, first=torch.tensor(first, dtype=torch.int32), lens=torch.tensor(lens, dtype=torch.int32)).items()}
     o = {n: torch.full(s, 7.0, device=DEV) for n, s in dict(qd=(nc * H, 64, D), kd=(nc * H, 64 * L), w=(nc * H, D8 * 64), g=(nc * H, D), u=(nc * H, 64, V), a=(nc * H, 64, 64)).items()}
     p = nsq.pcs_delta_chunk_params()
     p.qk, p.v, p.ld, p.b, p.b_stride = (dev["qk"].data_ptr(), dev["v"].data_ptr(), dev["ld"].data_ptr(), dev["b"].data_ptr(), H)
+    if per_head:
+        p.ld, p.dec_a, p.dec_stride, p.dt_bias, p.rate = None, dev["dec_a"].data_ptr(), H, dev["bias"].data_ptr(), dev["rates"].data_ptr()
     p.heads, p.kv_heads, p.dim, p.vdim, p.n_chunks, p.n_tokens, p.dtype, p.n_seqs = H, KV, D, V, nc, T, nsq.PCS_BF16, 1
     p.chunk_first, p.chunk_len = dev["first"].data_ptr(), dev["lens"].data_ptr()
     p.qd, p.kd, p.w, p.g, p.u, p.a = (o[n].data_ptr() for n in ("qd", "kd", "w", "g", "u", "a"))
@@ -41,6 +48,8 @@ def test_prep(KV, G, D, V, lens, rate):
         for t in range(4):
             c = t + 4 * x
             w[:, :, c::8] = f[:, :, :, :, t, x, :].permute(0, 2, 4, 3, 1).reshape(nc * H, 64, D8 // 8)
+    # kd's tile of 16 channels and 8 tokens: a lane holds channels g, g + 8 of tokens t, t + 4
+    kd = got["kd"].view(nc * H, L // 16, 8, 8, 4, 2, 2).permute(0, 2, 5, 4, 1, 6, 3).reshape(nc * H, 64, L)
     # 2^-22 of an exponential, 2^-24 of each of the up to 64 numbers a running sum holds (64 rate each) and of the up to 256 terms of a sum; the solve adds 64 terms three times over
     eps = 2.0 ** -22 * (1 + 64 * rate) + 2.0 ** -23 * (16 + D ** 0.5)
     for c in range(nc):
@@ -62,3 +71,5 @@ def test_prep(KV, G, D, V, lens, rate):
             assert float((w[j, :n, :D] - wk).abs().max()) <= 4 * eps * size
             assert float((got["qd"][j, :n] - qf * torch.exp(B)).abs().max()) <= eps
             assert float((got["g"][j] - torch.exp(B[-1])).abs().max()) <= eps
+            assert float((kd[j, :n, :D] - kf * torch.exp(B[-1] - B)).abs().max()) <= eps
+            assert bool((kd[j, n:] == 0).all()) and bool((kd[j, :, D:] == 0).all())

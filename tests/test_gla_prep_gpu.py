@@ -27,6 +27,7 @@ def _prep(nsq, plan, batch, proj, shift, offs, ld, H, D, V, values=True):
 
 @pytest.mark.parametrize("H,D,V,lens,rate", [
     (2, 4, 8, (1, 64), 1.0), (1, 20, 36, (15, 16, 17), 0.1), (2, 48, 64, (65, 33), 30.0), (3, 132, 72, (130, 7), 0.0), (1, 256, 512, (200, 49), 1.0), (2, 128, 128, (63, 48), 5.0),
+    (1, 20, 36, (64, 61), 0.05), (2, 132, 72, (64,), 0.02), (1, 256, 512, (128, 50), 0.1),     # factors between blocks well away from 0 and 1
 ])
 def test_blocks_of_sixteen(H, D, V, lens, rate):
     from promptcache_b200 import _native_seq as nsq
@@ -51,6 +52,18 @@ def test_blocks_of_sixteen(H, D, V, lens, rate):
     size = float(proj[:, :H * D].float().abs().max() * proj[:, H * D:2 * H * D].float().abs().max()) * D ** 0.5
     assert float((new["a"] - old["a"]).abs().max()) <= (rel + D * 2.0 ** -24) * size
     assert bool((new["a"].triu(1) == 0).all())
+    # Every pair against float64: a factor is a product of up to four exponentials (2^-22 and a rounding each) of sums of up to sixteen numbers <= rate (sixteen roundings of numbers of up to
+    # 16 rate, three such sums at most), a sum of D products loses less than D roundings of what its terms add up to in size
+    rel = 2.0 ** -19 + 2.0 ** -24 * (3 * 16 * 16 * rate + D)
+    first, lens_of = plan["first"].tolist(), plan["len"].tolist()
+    for c in range(plan["n_chunks"]):
+        sl = slice(first[c], first[c] + lens_of[c])
+        for h in range(H):
+            B = ld[sl, h].double().cumsum(0)
+            q, k = (proj[sl, o + h * D:o + (h + 1) * D].double() for o in offs[:2])
+            E = torch.exp((B[:, None] - B[None]).clamp(max=0))
+            want, size = (torch.einsum("id,sd,isd->is", x * D ** -0.5, y, E).tril() for x, y in ((q, k), (q.abs(), k.abs())))
+            assert bool(((new["a"][c * H + h, :lens_of[c], :lens_of[c]].double() - want).abs() <= rel * size + 1e-30).all()), (c, h)
 
 
 @pytest.mark.parametrize("H,D,V,lens", [(2, 16, 8, (65, 1)), (1, 48, 136, (64, 33, 31)), (2, 256, 512, (130,)), (3, 64, 40, (17, 95))])
