@@ -507,8 +507,9 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: 
             raise NativeError("attention: the distance-bias numbers must be float32 [H]")
     p = pcs_attn_params()
     p.q, p.k_pool, p.v_pool, p.out = q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr()
-    p.n_heads, p.n_kv_heads, p.dim, p.cap, p.n_slots = n_heads, k_pool.shape[1], k_pool.shape[3], k_pool.shape[2], min(k_pool.shape[0], v_pool.shape[0])
-    p.vdim = out.shape[1] // n_heads if v_row_stride else v_pool.shape[3]
+    k_shape, v_shape = k_pool.shape, v_pool.shape
+    p.n_heads, p.n_kv_heads, p.dim, p.cap, p.n_slots = n_heads, k_shape[1], k_shape[3], k_shape[2], min(k_shape[0], v_shape[0])
+    p.vdim = out.shape[1] // n_heads if v_row_stride else v_shape[3]
     p.v_row_stride, p.sink_logit, p.pool_slot, p.talk = int(v_row_stride), _ptr(sink_logit), _ptr(pool_slot), _ptr(talk)
     if out_gate is not None:
         _cuda(out_gate)

@@ -1696,8 +1696,7 @@ static int launch_delta_chunk_scan(const pcs_delta_chunk_params& p, size_t smem,
 // part), six products per step of sixteen terms, the smallest first, and the steps' sums join in rounded additions (the tensor core's running sum cuts
 // bits off).  That takes registers for half of the tokens at most.
 // Bound by the legacy tensor path: 32 chunks of 4 heads of 256 x 512 are 48 products per warp and step, 17 us with two parts and 28 with three.
-// They take 40 and 69 us a launch (42 and 71 with operands that came straight from memory a step ahead and a straight-line end with IEEE divides); 25 drawn calls of the
-// delta rule are 1.05 times as fast, 25 of gated linear attention 1.03.
+// They take 40 and 69 us a launch (42 and 71 with operands that came straight from memory a step ahead and a straight-line end); their pipe is busy for 40 and 42 % of the time.
 constexpr int kDoMaxWarps = 16, kDoVRow = 40, kDoRow = 36, kDoStage = 16 * kDoRow, kDoStages = 3;
 
 template <int PARTS, int MT>   // MT: tiles of 16 tokens

@@ -509,6 +509,8 @@ __global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep_kernel(const pcs_
 // Running sums are kept inside the blocks (Bs), with the blocks' sums beside them.  Figures: 132 blocks of 64 x 256, 55 us above,
 // 26 here: 41 by the blocks, 29 once a row's pieces are requested together and nobody wants the copies of the values, 26 with two by two pairs inside the blocks
 // (one at a time read four rows per pair, and shared memory was what they waited for).
+// Error against float64 (rms, decays of logsigmoid(z + 1) / 16), exact exponentials / here: pairs of different blocks 2.34e-7 / 2.20e-7 at 256 channels, 1.60e-7 / 1.36e-7 at 64, inside 2.06e-7 / 0.95e-7
+// (shorter running sums); with decays fifty times weaker a product of several rounded factors shows, 2.07e-7 / 2.22e-7 across, 1.96e-7 / 0.93e-7 inside.
 constexpr int kP64 = 64, kP64Block = 16;
 __global__ void __launch_bounds__(kPrepThreads) gla_chunk_prep64_kernel(const pcs_gla_chunk_params p) {
   extern __shared__ __align__(16) float sm[];
@@ -789,7 +791,7 @@ __global__ void __launch_bounds__(kSumsThreads, 2) gla_chunk_sums_kernel(const p
 // The sums and the scan in one kernel: block = 64 state rows x 64 columns of one (entry, head), the chunks in order.  Per chunk the state it starts from goes to u,
 // S <- g S + kd^T v for the tile, the product as in gla_chunk_sums_kernel; the chunks' own sums never pass through memory, kd and v are read again by every tile (24 KB a chunk, from L2).
 // Four warps, one per scheduler, hold 16 rows x 64 columns each in registers, so that every number of kd is taken apart once per block; four others keep the loads three chunks ahead.
-// 33 chunks of 4 heads of 256 x 512: 42 us (sums 38, scan 30); the wrapper's rule says for which walks (a step takes 1.1 us whatever the number of blocks, so few tiles over long walks
+// 33 chunks of 4 heads of 256 x 512: 41 us (sums 38, scan 30); the wrapper's rule says for which walks (a step takes 1.25 to 1.33 us whatever the number of blocks, so few tiles over long walks
 // stay with the sums of all chunks side by side).
 constexpr int kStMul = 128, kStThreads = 2 * kStMul, kStStages = 4, kStKRow = 68, kStVRow = 72;
 constexpr int kStStage = kSumsChunk * (kStKRow * 4 + kStVRow * 2) + 64 * 4;   // bytes: kd, v, the rows' decays
