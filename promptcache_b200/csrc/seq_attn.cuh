@@ -11,7 +11,7 @@ inline unsigned long long pool_planes(const pcs_attn_params& p) {
 
 // A launch over a step's own dense K/V (`pool_slot`) with rows of 96 and 64 numbers once ended with an illegal memory access.  What raised it is not known: the sizes, strides and slots it
 // got are in range, and so is every index that the kernel forms from them.  Such pools with rows that a tensor map's boxes of 64 columns do not divide are served by the mma.sync kernel, which
-// reads by plain loads, until it is known.
+// reads by plain loads, until it is known (and which forms a row again whose result is not finite there, as the tcgen05 kernels do).
 inline bool dense_rows_off_boxes(const pcs_attn_params& p) { return p.pool_slot && (p.dim % 64 != 0 || p.vdim % 64 != 0); }
 
 // the launch chooses the kernel (1 and 2 name one)

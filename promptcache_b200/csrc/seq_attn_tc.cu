@@ -12,7 +12,7 @@
 //                         hi = bf16(P), lo = bf16(P - hi), so that the product keeps ~16 bits of every weight instead of 8
 // Key / value widths are padded in shared memory to 64, 128 or 256 (zero fill); every width that is a multiple of 8 up to
 // 256 is served.  Other types and shapes fall to the plain kernel (seq_attn.cu).
-#include "seq_common.cuh"
+#include "seq_attn.cuh"
 #include "seq_mma.cuh"
 
 namespace pcs {
@@ -49,8 +49,9 @@ __device__ __forceinline__ void load_tile_async(__nv_bfloat16* dst, const __nv_b
   }
 }
 
-template <int DP, int VP>
-__global__ void __launch_bounds__(TC_THREADS, (DP <= 128 && VP <= 128) ? 3 : 1) attn_tc_kernel(const pcs_attn_params p) {
+// AGAIN: hidden rows that are not finite do not reach a query, as in the tcgen05 kernels (an entry's dense rows, which those served before: dense_rows_off_boxes)
+template <int DP, int VP, bool AGAIN>
+__global__ void __launch_bounds__(TC_THREADS, (DP <= 128 && VP <= 128) ? 3 : 1) attn_tc_kernel(const __grid_constant__ pcs_attn_params p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_raw);
   __nv_bfloat16* Kbuf = Qs + BM * (DP + PAD);       // two stages of K, then one of V
@@ -278,9 +279,14 @@ __global__ void __launch_bounds__(TC_THREADS, (DP <= 128 && VP <= 128) ? 3 : 1) 
   }
   const long long os = p.out_stride > 0 ? p.out_stride : static_cast<long long>(p.n_heads) * V;
   __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(off) * os + h * V;
+  float zero_a = 0.f, zero_b = 0.f;   // stay 0 over finite numbers
 #pragma unroll
   for (int vn = 0; vn < VP / 8; ++vn) {
     const int c = vn * 8 + qd * 2;
+    if (AGAIN) {
+      zero_a = fmaf(o[vn][0] * inv_a, 0.f, fmaf(o[vn][1] * inv_a, 0.f, zero_a));
+      zero_b = fmaf(o[vn][2] * inv_b, 0.f, fmaf(o[vn][3] * inv_b, 0.f, zero_b));
+    }
     if (c < V) {
       if (q0 + row_a < len)
         *reinterpret_cast<uint32_t*>(out + static_cast<long long>(q0 + row_a) * os + c) = pack_bf16(o[vn][0] * inv_a, o[vn][1] * inv_a);
@@ -288,26 +294,43 @@ __global__ void __launch_bounds__(TC_THREADS, (DP <= 128 && VP <= 128) ? 3 : 1) 
         *reinterpret_cast<uint32_t*>(out + static_cast<long long>(q0 + row_b) * os + c) = pack_bf16(o[vn][2] * inv_b, o[vn][3] * inv_b);
     }
   }
+  // The products multiply hidden values of a tile by 0, and 0 * inf is not 0: rows whose result is not finite, from the keys they see alone
+#pragma unroll 1
+  for (int x = 0; AGAIN && x < 2; ++x) {
+    __syncwarp();
+    for (uint32_t w = __ballot_sync(0xffffffffu, (x ? zero_b : zero_a) != 0.f && q0 + (x ? row_b : row_a) < len); w;) {
+      const int r = (__ffs(w) - 1) >> 2, row = q0 + warp * 16 + 8 * x + r;   // (four lanes hold a row)
+      w &= ~(0xfu << (4 * r));
+      for (int c0 = 0; c0 < V; c0 += 128) attn_row_again_call<__nv_bfloat16>(p, b, h, off + row, pos0 + row, c0, min(128, V - c0));
+    }
+  }
 }
 
-template <int DP, int VP>
+template <int DP, int VP, bool AGAIN>
 int launch(const pcs_attn_params& p, cudaStream_t st) {
   const size_t smem = (static_cast<size_t>(BM + 2 * BN) * (DP + PAD) + static_cast<size_t>(BN) * (VP + PAD)) * sizeof(__nv_bfloat16) +
                       272 * sizeof(float);
   static PerDevice<NoInfo> set_up;
-  if (int rc = set_up.once([&] { return cudaFuncSetAttribute(attn_tc_kernel<DP, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); })) return rc;
+  if (int rc = set_up.once([&] { return cudaFuncSetAttribute(attn_tc_kernel<DP, VP, AGAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); })) return rc;
   dim3 grid(static_cast<unsigned>((p.max_len + BM - 1) / BM) * p.n_seqs * p.n_heads);
-  attn_tc_kernel<DP, VP><<<grid, TC_THREADS, smem, st>>>(p);
+  attn_tc_kernel<DP, VP, AGAIN><<<grid, TC_THREADS, smem, st>>>(p);
   PCS_CHECK_CUDA(cudaGetLastError());
   count_launch();
   return PCS_OK;
 }
 
-template <int DP>
+template <int DP, bool AGAIN>
 int launch_v(const pcs_attn_params& p, cudaStream_t st) {
-  if (p.vdim <= 64) return launch<DP, 64>(p, st);
-  if (p.vdim <= 128) return launch<DP, 128>(p, st);
-  return launch<DP, 256>(p, st);
+  if (p.vdim <= 64) return launch<DP, 64, AGAIN>(p, st);
+  if (p.vdim <= 128) return launch<DP, 128, AGAIN>(p, st);
+  return launch<DP, 256, AGAIN>(p, st);
+}
+
+template <bool AGAIN>
+int launch_d(const pcs_attn_params& p, cudaStream_t st) {
+  if (p.dim <= 64) return launch_v<64, AGAIN>(p, st);
+  if (p.dim <= 128) return launch_v<128, AGAIN>(p, st);
+  return launch_v<256, AGAIN>(p, st);
 }
 
 }  // namespace
@@ -319,9 +342,7 @@ int launch_attn_tc(const pcs_attn_params& p, cudaStream_t st, bool* handled) {
   if (p.out_stride % 2 != 0 || (reinterpret_cast<uintptr_t>(p.out) & 3) != 0) return PCS_OK;
   if (static_cast<long long>((p.max_len + BM - 1) / BM) * p.n_seqs * p.n_heads > 0x7fffffffLL) return PCS_OK;
   *handled = true;
-  if (p.dim <= 64) return launch_v<64>(p, st);
-  if (p.dim <= 128) return launch_v<128>(p, st);
-  return launch_v<256>(p, st);
+  return dense_rows_off_boxes(p) ? launch_d<true>(p, st) : launch_d<false>(p, st);
 }
 
 }  // namespace pcs

@@ -52,3 +52,28 @@ def test_dense_rows_off_the_boxes(H, G, D, V, n, stored, window):
         got = out[:, h * V:(h + 1) * V].to(F64)
         # the result is rounded to bfloat16 (2^-9 of it), the weights keep 16 bits and the scores 22
         assert bool(((got - want).abs() <= want.abs() * 2.0 ** -8 + vv.abs().max() * 2.0 ** -13).all()), h
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,G,D,V,limits", [(2, 2, 96, 64, {}), (2, 1, 96, 64, dict(window=30)), (4, 2, 72, 136, dict(softcap=20.0)), (2, 2, 200, 40, dict(chunk=70))])
+def test_hidden_rows_that_are_not_finite(H, G, D, V, limits):
+    """A value of NaN or infinity reaches the queries that see its key and no others of their tile."""
+    from promptcache_b200 import _native_seq as nsq
+    n, stored, key = 150, 9, 100
+    g = torch.Generator(device=DEV).manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV).to(BF16)
+    q, k, v, batch = rnd(n, H * D), rnd(1, G, 192, D), rnd(1, G, 192, V), nsq.Batch([1], [stored], [n], torch.device(DEV))
+    outs = []
+    for value in (None, torch.nan, torch.inf):
+        if value is not None:
+            v[0, :, key] = value
+        out = torch.full((n, H * V), 7.0, device=DEV, dtype=BF16)
+        nsq.attention(q, k, v, out, H, D ** -0.5, None, None, False, batch, pool_slot=torch.zeros(1, dtype=torch.int32, device=DEV), **limits)
+        outs.append(out)
+    i = torch.arange(stored, stored + n, device=DEV)
+    sees = (i >= key) & (i - key < limits.get("window", n)) & (i // limits.get("chunk", 10 ** 6) == key // limits.get("chunk", 10 ** 6))
+    assert 0 < int(sees.sum()) < n
+    for out in outs[1:]:
+        # the same numbers summed in another order, rounded to bfloat16
+        assert bool(((out[~sees].double() - outs[0][~sees].double()).abs() <= outs[0][~sees].double().abs() * 2.0 ** -7 + 2.0 ** -10).all())
+        assert not bool(out[sees].isfinite().any())
