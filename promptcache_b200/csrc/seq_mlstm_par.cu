@@ -126,24 +126,29 @@ __global__ void __launch_bounds__(512) mlstm_par_gates_kernel(const pcs_mlstm_pa
 // Four warps, one per scheduler, hold 16 columns x 64 rows each and form U transposed, (v w)^T k: a lane's numbers are then pairs of neighbouring
 // rows at one column, which, rounded, are the operand fragments of q S.  The states lie in the scratch as those fragments: [dim / 16][vdim / 8][lane] 16 bytes, rows 2t, 2t + 1 and
 // 2t + 8, 2t + 9 of column g as hi, then as lo, so that a fragment is written and read by one 16-byte access a lane.  The values are weighed and split in registers, by the only warp that uses them.
-// Four other warps keep the loads ahead and sum the normaliser; one barrier per chunk.
+// Four other warps keep the loads four chunks ahead, and CHAIN of them sum the normaliser, token by token: a warp takes 64 / CHAIN tokens of a chunk and goes on from where the warp before it
+// ended, a step earlier, so the last one is CHAIN - 1 chunks behind.  One barrier per chunk.  us a call with chains of 1 / 2 / 4: 32 chunks of 4 heads of 256 x 512 80.0 / 77.7 / 76.6, 20 of 4 of 128 x 256
+// in segments 36.9 / 36.1 / 36.7, 7 of 4 of 128 x 128 24.5 / 23.8 / 24.3: four from 24 chunks in one walk on, two elsewhere.  (Four sums of sixteen tokens added at the end: 0 to 2 % faster, other bits.)
 // 32 chunks of 4 heads of 256 x 512: 46 us as sums of the chunks and an element-wise scan over them, 32 in this form; the products alone take 9.  What a step waits for is the
 // one warp per scheduler: with eight warps that multiply (each weighing for itself) it took 38 us, with the values weighed by the helpers 34 to 40.
-constexpr int kSTHalf = 128, kST = 2 * kSTHalf, kSStages = 5, kSRow = 72, kSTile = CL * kSRow;
+constexpr int kSTHalf = 128, kST = 2 * kSTHalf, kSAhead = 4, kSRow = 72, kSTile = CL * kSRow;
 
 // Few tiles leave most of the GPU idle over a long walk: it is then cut into `segs` segments side by side.  A first launch (SUMS) walks all but the last without
 // writing states and leaves what they add up to; in the second a segment starts from those before it.  Twice the products, 1 / segs of the steps.
 constexpr int kMaxTiles = 148, kTileFloats = 64 * 64;   // segments of all tiles are at most one per SM
 
-static size_t state_smem() { return static_cast<size_t>(kSStages) * (2 * kSTile * 2 + CL * 4) + 2 * 4 * 64 * 4; }
+template <int CHAIN>
+constexpr int kStateSmem = (kSAhead + CHAIN) * (2 * kSTile * 2 + CL * 4) + (CHAIN - 1) * 2 * 64 * 4;
 
-template <bool SUMS>
+template <bool SUMS, int CHAIN>
 __global__ void __launch_bounds__(kST) mlstm_par_state_kernel(const pcs_mlstm_params p, float* scratch, long long slots, int segs) {
+  constexpr int kSStages = kSAhead + CHAIN;
+  static_assert(CL % CHAIN == 0 && CHAIN <= 4, "equal parts of a chunk's tokens");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __nv_bfloat16* Ks = reinterpret_cast<__nv_bfloat16*>(smem_raw);   // [stages][64][72]
   __nv_bfloat16* Vs = Ks + kSStages * kSTile;
   float* we = reinterpret_cast<float*>(Vs + kSStages * kSTile);     // [stages][64]
-  float* red = we + kSStages * CL;                                  // [2][4][64] sums of k over sixteen tokens
+  float* carry = we + kSStages * CL;                                // [chain - 1][2][64] sums of k over the first tokens of a chunk
   const int D = p.dim, V = p.vdim, H = p.heads, b = blockIdx.z / segs, seg = blockIdx.z % segs, head = blockIdx.y, vtiles = (V + 63) / 64;
   const int d0 = static_cast<int>(blockIdx.x) / vtiles * 64, v0 = static_cast<int>(blockIdx.x) % vtiles * 64;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = lane >> 2, qd = lane & 3;
@@ -204,44 +209,61 @@ __global__ void __launch_bounds__(kST) mlstm_par_state_kernel(const pcs_mlstm_pa
       cp_async_commit();
     };
 #pragma unroll 1
-    for (int c = 0; c < kSStages - 1; ++c) load();
-    const bool of_n = sums && ht < 64 && d0 + ht < D;
-    float ns = of_n && from_pool && !fresh ? p.n_pool[pool * D + d0 + ht] : 0.f, fc = sums ? sc.ce[at0] : 0.f;
-    if (SUMS) {
-      if (of_n && seg == 0) left_n(segs - 1)[ht] = ns;
-    } else if (of_n && !from_pool) {
-      ns = seg == 0 ? left_n(segs - 1)[ht] : left_n(0)[ht];
-      for (int j = 1; j < seg; ++j) ns = fmaf(ns, factor(j), left_n(j)[ht]);
-    }
-    for (int c = 0, st = 0; c <= nc; ++c) {
-      // the step after the last chunk only adds up its sums
-      cp_async_wait<kSStages - 2>();
-      __syncthreads();   // chunk c has landed; what chunk c - 1 lay in is free
-      load();
-      if (sums) {
-        if (of_n && c > 0) {
-          const float* r = red + ((c - 1) & 1) * 4 * 64 + ht;
-          if (!SUMS) sc.n[(at0 + static_cast<long long>(c - 1) * H) * D + d0 + ht] = ns;
-          ns = fmaf(ns, fc, (r[0] + r[64]) + (r[128] + r[192]));
-          if (c < nc) fc = sc.ce[at0 + static_cast<long long>(c) * H];
-        }
-        if (c < nc) {   // this warp's sixteen tokens, two rows of the state per lane
-          const __nv_bfloat16* k = Ks + st * kSTile + hw * 16 * kSRow + 2 * lane;
-          const float* w = we + st * CL + hw * 16;
-          float x = 0.f, y = 0.f;
-#pragma unroll
-          for (int t = 0; t < 16; ++t) {
-            const uint32_t kk = *reinterpret_cast<const uint32_t*>(k + t * kSRow);
-            x = fmaf(w[t], __uint_as_float(kk << 16), x);
-            y = fmaf(w[t], __uint_as_float(kk & 0xffff0000u), y);
-          }
-          *reinterpret_cast<float2*>(red + ((c & 1) * 4 + hw) * 64 + 2 * lane) = make_float2(x, y);
+    for (int c = 0; c < kSAhead; ++c) load();
+    const int row = 2 * lane;   // and the next
+    const bool of_n = sums && hw == CHAIN - 1 && d0 + row < D;
+    float ns[2] = {0.f, 0.f}, fc = sums ? sc.ce[at0] : 0.f;
+    if (of_n) {
+      if (from_pool && !fresh) {
+        ns[0] = p.n_pool[pool * D + d0 + row];
+        ns[1] = p.n_pool[pool * D + d0 + row + 1];
+      }
+      if (SUMS) {
+        if (seg == 0) *reinterpret_cast<float2*>(left_n(segs - 1) + row) = make_float2(ns[0], ns[1]);
+      } else if (!from_pool) {
+        for (int j = 0; j == 0 || j < seg; ++j) {
+          const float f = j ? factor(j) : 0.f;
+          const float2 x = *reinterpret_cast<const float2*>(left_n(seg ? j : segs - 1) + row);
+          ns[0] = fmaf(ns[0], f, x.x);
+          ns[1] = fmaf(ns[1], f, x.y);
         }
       }
-      st = st + 1 == kSStages ? 0 : st + 1;
     }
-    if (of_n && SUMS) left_n(seg)[ht] = ns;
-    if (of_n && !SUMS && last) p.n_pool[pool * D + d0 + ht] = ns;
+    const int steps = sums ? nc + CHAIN - 1 : nc;
+    for (int c = 0; c < steps; ++c) {
+      if (c < nc) {
+        cp_async_wait<kSAhead - 1>();
+        __syncthreads();   // chunk c has landed; what the chunk before the last one that is summed lay in is free
+        load();
+      } else {
+        asm volatile("bar.sync 1, 128;" ::: "memory");   // (these warps alone)
+      }
+      const int ch = c - hw, st = ch % kSStages;
+      if (!sums || hw >= CHAIN || ch < 0 || ch >= nc) continue;
+      float2 x = make_float2(0.f, 0.f);
+      if (hw) x = *reinterpret_cast<const float2*>(carry + ((hw - 1) * 2 + ((c - 1) & 1)) * 64 + row);
+      const __nv_bfloat16* k = Ks + st * kSTile + hw * (CL / CHAIN) * kSRow + row;
+      const float* w = we + st * CL + hw * (CL / CHAIN);
+#pragma unroll
+      for (int t = 0; t < CL / CHAIN; ++t) {
+        const uint32_t kk = *reinterpret_cast<const uint32_t*>(k + t * kSRow);
+        x.x = fmaf(w[t], __uint_as_float(kk << 16), x.x);
+        x.y = fmaf(w[t], __uint_as_float(kk & 0xffff0000u), x.y);
+      }
+      if (hw < CHAIN - 1) {
+        *reinterpret_cast<float2*>(carry + (hw * 2 + (c & 1)) * 64 + row) = x;
+      } else {
+        if (of_n && !SUMS) *reinterpret_cast<float2*>(sc.n + (at0 + static_cast<long long>(ch) * H) * D + d0 + row) = make_float2(ns[0], ns[1]);
+        ns[0] = fmaf(ns[0], fc, x.x);
+        ns[1] = fmaf(ns[1], fc, x.y);
+        if (ch + 1 < nc) fc = sc.ce[at0 + static_cast<long long>(ch + 1) * H];
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      if (of_n && SUMS) left_n(seg)[row + x] = ns[x];
+      if (of_n && !SUMS && last) p.n_pool[pool * D + d0 + row + x] = ns[x];
+    }
     return;
   }
   // this lane's state: columns vr and vr + 8, rows d0 + 8 j + 2 qd and the next
@@ -361,7 +383,6 @@ __global__ void __launch_bounds__(kST) mlstm_par_state_kernel(const pcs_mlstm_pa
       for (int x = 0; x < 4; ++x) s[j][x] = fmaf(s[j][x], f, acc[j][x]);
     st = st + 1 == kSStages ? 0 : st + 1;
   }
-  __syncthreads();   // (the helpers' last step)
   if (SUMS) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(left(seg) + j * 512) = make_float4(s[j][0], s[j][1], s[j][2], s[j][3]);
@@ -389,7 +410,7 @@ __host__ __device__ __forceinline__ int out_tiles(int D, int warps, int MT) {
   const int a = (2 * CL * (D + 8) + 2 * CL * PROW) * 2 + warps * kWStages * kWStage, b = warps * MT * 16 * 192;
   return a > b ? a : b;
 }
-static int out_smem(int D, int warps, int MT) { return out_tiles(D, warps, MT) + (kOutFloats + kOutWarps * CL) * 4; }
+static int out_smem(int D, int warps, int MT) { return out_tiles(D, warps, MT) + kOutFloats * 4; }
 
 template <int MT>
 __global__ void __launch_bounds__(kOutWarps * 32, 1) mlstm_par_out_kernel(const pcs_mlstm_params p, float* scratch, long long slots) {
@@ -406,7 +427,6 @@ __global__ void __launch_bounds__(kOutWarps * 32, 1) mlstm_par_out_kernel(const 
   float* psum = tok + 4 * CL;                                       // [4][64] sums of the weights over 16 keys
   float* nq = psum + 4 * CL;                                        // [64] q . n of the state
   float* inv = nq + CL;                                             // [64] 1 / rms
-  float* ss = inv + CL;                                             // [columns' warps][64] sums of squares
   const Scratch sc(scratch, slots, p);
   const int c = blockIdx.x, b = blockIdx.y / H, head = blockIdx.y - b * H;
   const int len = p.seq_len[b], i0 = c * CL;
@@ -596,43 +616,59 @@ __global__ void __launch_bounds__(kOutWarps * 32, 1) mlstm_par_out_kernel(const 
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int r = 16 * (m0 + m) + grp + 8 * i;
-      float w = psum[r];
+      float w[4];
 #pragma unroll
-      for (int k = 1; k < 4; ++k)
-        if (k <= m0 + m) w += psum[k * CL + r];
-      const float den = 1.f / (fmaxf(fabsf(nq[r] + w), tok[3 * CL + r]) + 1e-6f);
-      float x = 0.f;
+      for (int k = 0; k < 4; ++k) w[k] = k <= m0 + m ? psum[k * CL + r] : 0.f;
+      const float den = 1.f / (fmaxf(fabsf(nq[r] + (w[0] + w[1]) + (w[2] + w[3])), tok[3 * CL + r]) + 1e-6f);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        float &y0 = acc[m][j][i * 2], &y1 = acc[m][j][i * 2 + 1];
-        y0 *= den;
-        y1 *= den;
-        x = fmaf(y0, y0, fmaf(y1, y1, x));
+        acc[m][j][i * 2] *= den;
+        acc[m][j][i * 2 + 1] *= den;
       }
-      x += __shfl_xor_sync(0xffffffffu, x, 1);
-      x += __shfl_xor_sync(0xffffffffu, x, 2);
-      if (qd == 0) ss[wc * CL + r] = x;
     }
-  __syncthreads();
-  for (int r = tid; r < CL; r += nthr) {
-    float x = 0.f;
-    for (int w = 0; w < ncol; ++w) x += ss[w * CL + r];
-    inv[r] = 1.f / sqrtf(x / static_cast<float>(V) + p.eps);
-  }
-  // The warp's results pass through shared memory (what lay there has been read), 16-byte pieces of a row exchanged by its number: a lane then has eight columns of a
+  __syncthreads();   // (what lies in shared memory up to here has been read)
+  // The warp's results pass through shared memory, 16-byte pieces of a row exchanged by its number: a lane then has eight columns of a
   // row, and the code is a short loop (a block runs it once: straight-line code is fetched more slowly than it runs, 17 000 cycles against 5 000).
-  float* mine = reinterpret_cast<float*>(smem_raw + warp * (MT * 16 * 192));
+  constexpr int kMine = MT * 16 * 48;   // floats of a warp: its results, then its gates
+  float* mine = reinterpret_cast<float*>(smem_raw) + warp * kMine;
   uint4* gates = reinterpret_cast<uint4*>(mine + MT * 16 * 32) + lane;
+  auto at_row = [&](int row, int j) { return row * 32 + (((2 * j + (qd >> 1)) ^ (2 * (grp & 3))) * 4 + (qd & 1) * 2); };   // columns 8 j + 2 qd and the next of row `row` = grp mod 8
 #pragma unroll
   for (int m = 0; m < MT; ++m)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float* o = mine + (16 * m + grp) * 32 + (((2 * j + (qd >> 1)) ^ (2 * (grp & 3))) * 4 + (qd & 1) * 2);
-      *reinterpret_cast<float2*>(o) = make_float2(acc[m][j][0], acc[m][j][1]);
-      *reinterpret_cast<float2*>(o + 8 * 32) = make_float2(acc[m][j][2], acc[m][j][3]);
+      *reinterpret_cast<float2*>(mine + at_row(16 * m + grp, j)) = make_float2(acc[m][j][0], acc[m][j][1]);
+      *reinterpret_cast<float2*>(mine + at_row(16 * m + grp + 8, j)) = make_float2(acc[m][j][2], acc[m][j][3]);
     }
 #pragma unroll
   for (int h = 0; h < 2 * MT; ++h) gates[32 * h] = gate[h];
+  __syncthreads();
+  // Sums of squares: a row's in sixteen chains, four lanes for each quarter of the (padded) columns, whatever the number of warps that hold them (each warp its own columns: other bits, and no
+  // faster; from register to register, warp after warp: 1.9 us more a launch)
+#pragma unroll 1
+  for (int r = warp * 8; r < CL; r += nw * 8) {
+    const int t0w = r / (16 * MT), row = r - t0w * (16 * MT) + grp;
+    float x[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    for (int u = 0; u < MT; ++u) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (q * MT + u >= ncol) continue;
+        const float* from = reinterpret_cast<const float*>(smem_raw) + (t0w * ncol + q * MT + u) * kMine;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 y = *reinterpret_cast<const float2*>(from + at_row(row, j));
+          x[q] = fmaf(y.x, y.x, fmaf(y.y, y.y, x[q]));
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      x[q] += __shfl_xor_sync(0xffffffffu, x[q], 1);
+      x[q] += __shfl_xor_sync(0xffffffffu, x[q], 2);
+    }
+    if (qd == 0) inv[r + grp] = 1.f / sqrtf((((x[0] + x[1]) + x[2]) + x[3]) / static_cast<float>(V) + p.eps);
+  }
   __syncthreads();
   if (col >= V) return;   // (vdim is a multiple of 8)
   float w[8];
@@ -683,6 +719,15 @@ static int state_segments(long long tiles, int chunks) {
   return best;
 }
 
+template <bool SUMS, int CHAIN>
+int launch_state(const pcs_mlstm_params& p, float* scratch, long long slots, dim3 grid, int segs, cudaStream_t st) {
+  static PerDevice<NoInfo> set_up;
+  if (int rc = set_up.once([&] { return cudaFuncSetAttribute(mlstm_par_state_kernel<SUMS, CHAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStateSmem<CHAIN>); })) return rc;
+  mlstm_par_state_kernel<SUMS, CHAIN><<<grid, kST, kStateSmem<CHAIN>, st>>>(p, scratch, slots, segs);
+  PCS_CHECK_CUDA(cudaGetLastError());
+  return PCS_OK;
+}
+
 template <int MT>
 int launch_out(const pcs_mlstm_params& p, float* scratch, long long slots, dim3 grid, cudaStream_t st) {
   static PerDevice<NoInfo> set_up;
@@ -725,20 +770,12 @@ int launch_mlstm_par(const pcs_mlstm_params& p, cudaStream_t st, bool* handled) 
   float* s = p.chunk_scratch;
   mlstm_par_gates_kernel<<<dim3(p.n_seqs, p.heads), 512, 2 * chunks * sizeof(float), st>>>(p, s, slots);
   PCS_CHECK_CUDA(cudaGetLastError());
-  static PerDevice<NoInfo> set_up;
-  if (int rc = set_up.once([&] {
-        const cudaError_t err = cudaFuncSetAttribute(mlstm_par_state_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(state_smem()));
-        return err != cudaSuccess ? err : cudaFuncSetAttribute(mlstm_par_state_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(state_smem()));
-      }))
-    return rc;
   const int tiles = ((p.dim + 63) / 64) * ((p.vdim + 63) / 64);
   const int segs = p.chunk_floats < floats(p.n_tokens, p.n_seqs, p.heads, p.dim, p.vdim, true) ? 1 : state_segments(tiles_of(p.n_seqs, p.heads, p.dim, p.vdim), chunks);
-  if (segs > 1) {
-    mlstm_par_state_kernel<true><<<dim3(tiles, p.heads, p.n_seqs * segs), kST, state_smem(), st>>>(p, s, slots, segs);
-    PCS_CHECK_CUDA(cudaGetLastError());
-  }
-  mlstm_par_state_kernel<false><<<dim3(tiles, p.heads, p.n_seqs * segs), kST, state_smem(), st>>>(p, s, slots, segs);
-  PCS_CHECK_CUDA(cudaGetLastError());
+  const dim3 walks(tiles, p.heads, p.n_seqs * segs);
+  if (segs > 1)
+    if (int rc = launch_state<true, 2>(p, s, slots, walks, segs, st)) return rc;
+  if (int rc = segs == 1 && chunks >= 24 ? launch_state<false, 4>(p, s, slots, walks, 1, st) : launch_state<false, 2>(p, s, slots, walks, segs, st)) return rc;
   const dim3 grid(chunks, p.n_seqs * p.heads);
   const int rc = p.vdim <= 128 ? launch_out<1>(p, s, slots, grid, st) : p.vdim <= 256 ? launch_out<2>(p, s, slots, grid, st) : launch_out<4>(p, s, slots, grid, st);
   if (rc) return rc;

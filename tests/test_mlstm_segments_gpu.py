@@ -45,3 +45,26 @@ def test_long_walks_of_few_heads(H, D, V, gap, steps):
                 assert float((have - ref).abs().max()) <= 3e-5 * float(ref.abs().max()) + 1e-6
             pos[b] += ln
             o += ln
+
+
+@pytest.mark.parametrize("H,D,V,lens", [(4, 128, 128, (500, 64, 1)), (16, 128, 256, (1601,)), (2, 80, 64, (449,))])
+def test_normaliser_token_by_token(H, D, V, lens):
+    """Walks in one piece add the normaliser's terms in the order of the tokens within a chunk and of the chunks, whichever warps do: with gates that weigh every token by 1 the sums can be
+    formed here, bit for bit."""
+    from promptcache_b200 import _native_seq as nsq
+    g = torch.Generator().manual_seed(D)
+    B, T = len(lens), sum(lens)
+    proj, ones = torch.randn(T, 2 * H * D + 2 * H * V, generator=g).to(BF16), torch.ones(H * V, dtype=BF16, device=DEV)
+    s, n, m = torch.zeros(B, H, D, V, device=DEV), torch.zeros(B, H, D, device=DEV), torch.zeros(B, H, device=DEV)
+    nsq.mlstm_scan(proj.to(DEV), (0, H * D, 2 * H * D, 2 * H * D + H * V), torch.zeros(T, H, device=DEV), torch.zeros(T, H, device=DEV), ones, torch.empty(T, H * V, dtype=BF16, device=DEV),
+                   s, n, m, 1e-5, nsq.Batch(range(B), [0] * B, lens, DEV))
+    k, o = proj[:, H * D:2 * H * D].float(), 0
+    for b, ln in enumerate(lens):
+        want = torch.zeros(H * D)
+        for c in range(0, ln, 64):
+            own = torch.zeros(H * D)
+            for t in range(c, min(c + 64, ln)):
+                own = own + k[o + t]
+            want = want + own
+        assert torch.equal(n[b].cpu().flatten(), want), b
+        o += ln
