@@ -10,7 +10,7 @@
 // (1450 cycles, 530 of them products) and by the traffic of the states in `out` (4 bytes an element, written and read once).
 //
 // 2048 tokens, 4 heads of 256 x 512 (B200): serial 317 us; 122 with the chunks' own sums, a scan over them and operand loads shared by a block (gates 6, sums 26, scan 20, out 63);
-// 76 in this form (gates 6, state 32, out 34).  40 drawn calls of 150 to 4100 tokens: none slower than with those sums and that scan, 1.16 times as fast in the mean.
+// 76 in this form (gates 6, state 32, out 34).  40 drawn calls of 150 to 4100 tokens: none more than 2 % slower than with those sums and that scan, 1.15 times as fast in the mean.
 #include "seq_common.cuh"
 #include "seq_mma.cuh"
 
